@@ -133,6 +133,7 @@ struct Operator {
   DevBuf<double> inv_out64;   // 1 / colsum, 0 where colsum == 0 (dangling)
   DevBuf<float> inv_out32;
   uint32_t n_dangling = 0;
+  uint64_t n_loops = 0;       // self-loops among the arcs
   std::map<uint32_t, std::unique_ptr<Partition>> parts;
   std::mutex mu;  // guards parts and relabel
   const DevCsr* trans = nullptr;  // adjacency whose row lengths are this operator's column counts
@@ -189,8 +190,10 @@ struct GraphHandleImpl {
   };
   std::map<std::pair<int, int>, std::unique_ptr<WeightSlot>> wslots;  // guarded by mu
   WeightSlot& weight_slot(int which, double loop_factor, cudaStream_t s);
-  // Arc values, column sums and their inverses of o from d_w.
-  void fill_weights(Operator& o, const double* d_w, double loop_factor, cudaStream_t s);
+  // Arc values of o from d_w; with `sums` also the column sums and their
+  // inverses.
+  void fill_weights(Operator& o, const double* d_w, double loop_factor, bool sums,
+                    cudaStream_t s);
 };
 
 // Merge-path tile coordinates and split rows of a row-compressed matrix.

@@ -365,55 +365,160 @@ const DevCsr& GraphHandleImpl::undirected_rows(cudaStream_t s) {
 }
 
 // ======================================================================= operators
-// Arc values: weight (or 1) times the diagonal factor on self-loops
-// (eigenvector.rs:512-547); FP32 copies and whether they are exact.
-__global__ void op_values(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
-                          const double* __restrict__ w, uint32_t n, double lf,
-                          double* __restrict__ v64, float* __restrict__ v32,
-                          unsigned int* __restrict__ inexact) {
+// Set-up passes over an adjacency. A hub row of an R-MAT graph holds 10^5 or
+// more arcs, so a pass that gives each row to one thread waits for that
+// thread (R-MAT 24: 60 ms for the arc values, 29 ms for the row sums, where
+// streaming the arcs takes about 1 ms). Per-arc work therefore runs flat over
+// the arcs, the self-loops of a row are found by binary search (rows are
+// sorted by target), and row sums give long rows to whole CTAs.
+
+// First arc of row r whose target is at least r: its self-loops, if any, are
+// the run of arcs with target r from there.
+__device__ __forceinline__ uint32_t first_loop(const uint32_t* __restrict__ off,
+                                               const uint32_t* __restrict__ tgt, uint32_t r) {
+  uint32_t lo = off[r], hi = off[r + 1];
+  while (lo < hi) {
+    const uint32_t mid = lo + ((hi - lo) >> 1);
+    if (tgt[mid] < r) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// Arc values: weight (or 1), through the arc's edge index when `edge` is
+// given; FP32 copies and how many of them are inexact. Bound by the streams
+// (12 bytes read or 8 and 12 written per arc; with `edge` also one gathered
+// weight). R-MAT 20 with weights per edge (16.8M arcs, three fills a gradient
+// step): 9.7 ms a fill with a thread per row, 0.12 ms flat. R-MAT 24 without
+// edge index: 60 -> 0.93 ms.
+__global__ void arc_values(const uint32_t* __restrict__ edge, const double* __restrict__ w,
+                           uint64_t nnz, double* __restrict__ v64, float* __restrict__ v32,
+                           unsigned int* __restrict__ inexact) {
+  unsigned int bad = 0;
+  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < nnz;
+       k += (uint64_t)gridDim.x * blockDim.x) {
+    const double x = w ? w[edge ? edge[k] : k] : 1.0;
+    const float f = (float)x;
+    v64[k] = x;
+    v32[k] = f;
+    bad += (double)f != x;
+  }
+  bad = warp_sum(bad);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(inexact, bad);
+}
+
+// Self-loops times their diagonal factor (eigenvector.rs:512-547), after
+// arc_values; the count of inexact FP32 copies follows.
+__global__ void scale_loops(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
+                            uint32_t n, double lf, double* __restrict__ v64,
+                            float* __restrict__ v32, unsigned int* __restrict__ inexact) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    bool bad = false;
-    for (uint32_t k = off[r]; k < off[r + 1]; ++k) {
-      double x = w ? w[k] : 1.0;
-      if (tgt[k] == r) x *= lf;
-      v64[k] = x;
-      float f = (float)x;
+    const uint32_t end = off[r + 1];
+    for (uint32_t k = first_loop(off, tgt, r); k < end && tgt[k] == r; ++k) {
+      const double x = v64[k], y = x * lf;
+      const float f = (float)y;
+      const int was = (double)v32[k] != x, is = (double)f != y;
+      v64[k] = y;
       v32[k] = f;
-      if ((double)f != x) bad = true;
+      if (was != is) atomicAdd(inexact, (unsigned int)(is - was));
     }
-    if (bad) atomicOr(inexact, 1u);
   }
 }
 
 __global__ void count_loops(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
                             uint32_t n, unsigned long long* __restrict__ loops) {
   unsigned long long c = 0;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
-    for (uint32_t k = off[r]; k < off[r + 1]; ++k) c += tgt[k] == r;
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const uint32_t end = off[r + 1];
+    for (uint32_t k = first_loop(off, tgt, r); k < end && tgt[k] == r; ++k) ++c;
+  }
   c = warp_sum(c);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(loops, c);
 }
 
-// Row sums in CSR order, one thread per row: for PageRank's pull operator
-// the sums over the out-adjacency are the column sums of the in-adjacency
-// operator in the reference's accumulation order (spectral.rs:240-246).
-__global__ void row_sums_seq(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
-                             const double* __restrict__ w, uint32_t n, double lf,
-                             double* __restrict__ sum, double* __restrict__ inv64,
-                             float* __restrict__ inv32, unsigned int* __restrict__ dangling) {
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (uint32_t k = off[r]; k < off[r + 1]; ++k) {
-      double x = w ? w[k] : 1.0;
-      if (tgt[k] == r) x *= lf;
-      s += x;
-    }
-    sum[r] = s;
-    double inv = s > 0.0 ? 1.0 / s : 0.0;
-    inv64[r] = inv;
-    inv32[r] = (float)inv;
-    if (!(s > 0.0)) atomicAdd(dangling, 1u);
+// Row sums: for PageRank's pull operator the sums over the out-adjacency are
+// the column sums of the in-adjacency operator (spectral.rs:240-246). Rows of
+// at most ROW_SEQ arcs take one thread, which adds them in CSR order as the
+// reference does; longer rows go to a list whose rows take one CTA each (a
+// fixed association, whatever the list's order). `tgt` is null when no arc
+// needs the loop factor. Bound by the weights' stream: R-MAT 24 (263M arcs)
+// 28.9 ms with a thread per row, 1.03 ms in the two kernels.
+constexpr uint32_t ROW_SEQ = 64;
+constexpr int ROW_T = 128;
+
+struct RowTerms {
+  const uint32_t* off;
+  const uint32_t* tgt;   // null: no loop factor to apply
+  const uint32_t* edge;  // null: w holds one value per arc
+  const double* w;       // null: every arc counts 1
+  double lf;
+  __device__ __forceinline__ double operator()(uint32_t r, uint32_t k) const {
+    double x = w ? w[edge ? edge[k] : k] : 1.0;
+    if (tgt && tgt[k] == r) x *= lf;
+    return x;
   }
+};
+
+__device__ __forceinline__ bool row_sum_store(uint32_t r, double s, double* sum, double* inv64,
+                                              float* inv32) {
+  const double inv = s > 0.0 ? 1.0 / s : 0.0;
+  sum[r] = s;
+  inv64[r] = inv;
+  inv32[r] = (float)inv;
+  return !(s > 0.0);
+}
+
+__global__ void row_sums_short(RowTerms t, uint32_t n, double* __restrict__ sum,
+                               double* __restrict__ inv64, float* __restrict__ inv32,
+                               unsigned int* __restrict__ dangling, uint32_t* __restrict__ list,
+                               uint32_t* __restrict__ nlist) {
+  unsigned int empty = 0;
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const uint32_t b = t.off[r], e = t.off[r + 1];
+    if (e - b > ROW_SEQ) {
+      list[atomicAdd(nlist, 1u)] = r;
+      continue;
+    }
+    double s = 0.0;
+    for (uint32_t k = b; k < e; ++k) s += t(r, k);
+    empty += row_sum_store(r, s, sum, inv64, inv32);
+  }
+  empty = warp_sum(empty);
+  if ((threadIdx.x & 31) == 0 && empty) atomicAdd(dangling, empty);
+}
+
+__global__ void __launch_bounds__(ROW_T)
+row_sums_long(RowTerms t, const uint32_t* __restrict__ list, const uint32_t* __restrict__ nlist,
+              double* __restrict__ sum, double* __restrict__ inv64, float* __restrict__ inv32,
+              unsigned int* __restrict__ dangling) {
+  __shared__ double sh[ROW_T / 32];
+  const uint32_t count = *nlist;
+  for (uint32_t q = blockIdx.x; q < count; q += gridDim.x) {
+    const uint32_t r = list[q], e = t.off[r + 1];
+    double s = 0.0;
+#pragma unroll 4
+    for (uint32_t k = t.off[r] + threadIdx.x; k < e; k += ROW_T) s += t(r, k);
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0 && row_sum_store(r, s, sum, inv64, inv32)) atomicAdd(dangling, 1u);
+  }
+}
+
+// sum, 1 / sum (0 where the sum is not positive) and the count of such rows
+// (added to *dangling) over the rows of one adjacency.
+static void row_sums(const RowTerms& t, uint32_t n, uint64_t arcs, double* sum, double* inv64,
+                     float* inv32, unsigned int* dangling, cudaStream_t s) {
+  if (!n) return;
+  const uint64_t most = std::min<uint64_t>(n, arcs / (ROW_SEQ + 1));
+  DevBuf<uint32_t> list(most + 1);  // the count, then the rows
+  KNB_CUDA(cudaMemsetAsync(list.get(), 0, 4, s));
+  row_sums_short<<<grid_for(n, ROW_T), ROW_T, 0, s>>>(t, n, sum, inv64, inv32, dangling,
+                                                      list.get() + 1, list.get());
+  KNB_LAUNCH("row_sums_short");
+  if (most) {
+    row_sums_long<<<(unsigned)std::min<uint64_t>(most, 148 * 16), ROW_T, 0, s>>>(
+        t, list.get() + 1, list.get(), sum, inv64, inv32, dangling);
+    KNB_LAUNCH("row_sums_long");
+  }
+  KNB_CUDA(cudaStreamSynchronize(s));
 }
 
 // Merge-path coordinates of tile boundaries (diagonal t * TILE).
@@ -856,44 +961,18 @@ const SlicedOp& Operator::sliced(uint32_t lw, uint32_t pieces, cudaStream_t s) {
   return ref;
 }
 
-// Arc values from per-edge weights given by the caller (input edge order),
-// through each arc's edge index.
-__global__ void op_values_from_edges(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
-                                     const uint32_t* __restrict__ edge, const double* __restrict__ w,
-                                     uint32_t n, double lf, double* __restrict__ v64,
-                                     float* __restrict__ v32, unsigned int* __restrict__ inexact) {
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    bool bad = false;
-    for (uint32_t k = off[r]; k < off[r + 1]; ++k) {
-      double x = w[edge[k]];
-      if (tgt[k] == r) x *= lf;
-      v64[k] = x;
-      float f = (float)x;
-      v32[k] = f;
-      if ((double)f != x) bad = true;
-    }
-    if (bad) atomicOr(inexact, 1u);
-  }
-}
-
-__global__ void row_sums_from_edges(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
-                                    const uint32_t* __restrict__ edge, const double* __restrict__ w,
-                                    uint32_t n, double lf, double* __restrict__ sum,
-                                    double* __restrict__ inv64, float* __restrict__ inv32,
-                                    unsigned int* __restrict__ dangling) {
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (uint32_t k = off[r]; k < off[r + 1]; ++k) {
-      double x = w[edge[k]];
-      if (tgt[k] == r) x *= lf;
-      s += x;
-    }
-    sum[r] = s;
-    double inv = s > 0.0 ? 1.0 / s : 0.0;
-    inv64[r] = inv;
-    inv32[r] = (float)inv;
-    if (!(s > 0.0)) atomicAdd(dangling, 1u);
-  }
+// Self-loops among the arcs of an adjacency.
+static uint64_t loop_count(const DevCsr& rows, cudaStream_t s) {
+  if (!rows.n) return 0;
+  DevBuf<unsigned long long> loops(1);
+  KNB_CUDA(cudaMemsetAsync(loops.get(), 0, 8, s));
+  count_loops<<<grid_for(rows.n, 256), 256, 0, s>>>(rows.off.get(), rows.tgt.get(), rows.n,
+                                                    loops.get());
+  KNB_LAUNCH("count_loops");
+  unsigned long long h = 0;
+  KNB_CUDA(cudaMemcpyAsync(&h, loops.get(), 8, cudaMemcpyDeviceToHost, s));
+  KNB_CUDA(cudaStreamSynchronize(s));
+  return h;
 }
 
 // An operator over the chosen rows with value buffers allocated (not filled).
@@ -911,30 +990,34 @@ static std::unique_ptr<Operator> weights_skeleton(GraphHandleImpl& g, int which,
   o->colsum.alloc(std::max<uint32_t>(g.n, 1));
   o->inv_out64.alloc(std::max<uint32_t>(g.n, 1));
   o->inv_out32.alloc(std::max<uint32_t>(g.n, 1));
+  o->n_loops = loop_count(*rows, s);
   return o;
 }
 
-void GraphHandleImpl::fill_weights(Operator& o, const double* d_w, double lf, cudaStream_t s) {
+void GraphHandleImpl::fill_weights(Operator& o, const double* d_w, double lf, bool sums,
+                                   cudaStream_t s) {
   const DevCsr* rows = o.rows;
   const DevCsr* trans = o.trans;
   DevBuf<unsigned int> flags(2);
   KNB_CUDA(cudaMemsetAsync(flags.get(), 0, 8, s));
-  if (n) {
-    op_values_from_edges<<<grid_for(n, 256), 256, 0, s>>>(rows->off.get(), rows->tgt.get(),
-                                                          rows->edge.get(), d_w, n, lf,
-                                                          o.vals64.get(), o.vals32.get(),
-                                                          flags.get());
-    row_sums_from_edges<<<grid_for(n, 128), 128, 0, s>>>(trans->off.get(), trans->tgt.get(),
-                                                         trans->edge.get(), d_w, n, lf,
-                                                         o.colsum.get(), o.inv_out64.get(),
-                                                         o.inv_out32.get(), flags.get() + 1);
-    KNB_LAUNCH("weighted_op");
+  const bool loops = lf != 1.0 && o.n_loops > 0;
+  if (o.nnz) {
+    arc_values<<<grid_for(o.nnz, 256), 256, 0, s>>>(rows->edge.get(), d_w, o.nnz, o.vals64.get(),
+                                                    o.vals32.get(), flags.get());
+    if (loops)
+      scale_loops<<<grid_for(n, 256), 256, 0, s>>>(rows->off.get(), rows->tgt.get(), n, lf,
+                                                   o.vals64.get(), o.vals32.get(), flags.get());
+    KNB_LAUNCH("arc values");
   }
+  if (sums)
+    row_sums({trans->off.get(), loops ? trans->tgt.get() : nullptr, trans->edge.get(), d_w, lf}, n,
+             trans->arcs, o.colsum.get(), o.inv_out64.get(), o.inv_out32.get(), flags.get() + 1,
+             s);
   unsigned int hf[2] = {0, 0};
   KNB_CUDA(cudaMemcpyAsync(hf, flags.get(), 8, cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
   o.vals32_exact = hf[0] == 0;
-  o.n_dangling = hf[1];
+  if (sums) o.n_dangling = hf[1];
 }
 
 GraphHandleImpl::WeightSlot& GraphHandleImpl::weight_slot(int which, double lf, cudaStream_t s) {
@@ -963,34 +1046,27 @@ Operator& GraphHandleImpl::op(int which, bool wtd, double lf, cudaStream_t s) {
   o->nnz = rows->arcs;
   const double* wv = (wtd && weighted) ? rows->w.get() : nullptr;
   const double* wt = (wtd && weighted) ? trans->w.get() : nullptr;
-  DevBuf<unsigned long long> loops(1);
-  KNB_CUDA(cudaMemsetAsync(loops.get(), 0, 8, s));
-  if (n) {
-    count_loops<<<grid_for(n, 256), 256, 0, s>>>(rows->off.get(), rows->tgt.get(), n, loops.get());
-    KNB_LAUNCH("count_loops");
-  }
-  unsigned long long nloops = 0;
-  KNB_CUDA(cudaMemcpyAsync(&nloops, loops.get(), 8, cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaStreamSynchronize(s));
-  o->has_vals = wv != nullptr || (lf != 1.0 && nloops > 0);
+  o->n_loops = loop_count(*rows, s);
+  const bool scaled = lf != 1.0 && o->n_loops > 0;
+  o->has_vals = wv != nullptr || scaled;
   DevBuf<unsigned int> flags(2);
   KNB_CUDA(cudaMemsetAsync(flags.get(), 0, 8, s));
   if (o->has_vals && o->nnz) {
     o->vals64.alloc(o->nnz);
     o->vals32.alloc(o->nnz);
-    op_values<<<grid_for(n, 256), 256, 0, s>>>(rows->off.get(), rows->tgt.get(), wv, n, lf,
-                                               o->vals64.get(), o->vals32.get(), flags.get());
-    KNB_LAUNCH("op_values");
+    arc_values<<<grid_for(o->nnz, 256), 256, 0, s>>>(nullptr, wv, o->nnz, o->vals64.get(),
+                                                     o->vals32.get(), flags.get());
+    if (scaled)
+      scale_loops<<<grid_for(n, 256), 256, 0, s>>>(rows->off.get(), rows->tgt.get(), n, lf,
+                                                   o->vals64.get(), o->vals32.get(), flags.get());
+    KNB_LAUNCH("arc values");
   }
   o->colsum.alloc(std::max<uint32_t>(n, 1));
   o->inv_out64.alloc(std::max<uint32_t>(n, 1));
   o->inv_out32.alloc(std::max<uint32_t>(n, 1));
-  if (n) {
-    row_sums_seq<<<grid_for(n, 128), 128, 0, s>>>(trans->off.get(), trans->tgt.get(), wt, n, lf,
-                                                  o->colsum.get(), o->inv_out64.get(),
-                                                  o->inv_out32.get(), flags.get() + 1);
-    KNB_LAUNCH("row_sums_seq");
-  }
+  row_sums({trans->off.get(), scaled ? trans->tgt.get() : nullptr, nullptr, wt, lf}, n,
+           trans->arcs, o->colsum.get(), o->inv_out64.get(), o->inv_out32.get(),
+           flags.get() + 1, s);
   unsigned int hf[2] = {0, 0};
   KNB_CUDA(cudaMemcpyAsync(hf, flags.get(), 8, cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
