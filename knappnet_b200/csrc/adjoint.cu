@@ -8,9 +8,13 @@
 // matrix d (M + jump 1_D^T) is d times a column-stochastic matrix) and
 // g = dL/dx, the adjoint lambda solves A^T lambda = g, i.e.
 //     lambda = g + d M^T lambda + d 1_D (jump^T lambda),
-// a fixed-point iteration that contracts by d in the max norm. It pulls along
-// out-arcs: (M^T lambda)_j = sum over arcs (j -> i) of f_e w_e lambda_i / s_j,
-// so it runs on the merge-path sweep over the out-adjacency. Then, since
+// a fixed-point iteration lambda <- g + d G lambda that contracts by d in the
+// max norm. G is the walk itself (row-stochastic), so what each closed class
+// of nodes holds on average shrinks by no more than d per sweep, where
+// PageRank's own change dies out much faster; the span of the last sweeps
+// gives that part's limit (adj_extrapolate). The sweep pulls along out-arcs,
+// (M^T lambda)_j = sum over arcs (j -> i) of f_e w_e lambda_i / s_j, on the
+// merge-path sweep over the out-adjacency. Then, since
 // dM_kj/dw_e = f_e (delta_ki - M_kj) / s_j for e = (j -> i),
 //     dL/dw_e = d f_e (x_j / s_j) (lambda_i - (M^T lambda)_j),
 // the second term being the derivative of the row (out-strength)
@@ -26,8 +30,24 @@
 
 namespace knb {
 
+// One adjoint sweep: the update, its L1 change and jump^T lambda'. A solve
+// ends when the change meets the tolerance. Once an extrapolation has been
+// taken (st->ambiguous) it goes on to SETTLED times the tolerance, so that the
+// faster parts end about as small as the sweeps left out would have made
+// them, or to the sweep at which the plain iteration would have ended
+// (st->prev_inv_total), whichever is first.
+constexpr double SETTLED = 1e-2;
+__device__ __forceinline__ void adj_decide(IterState* st) {
+  const bool enough = st->ambiguous ? st->change <= SETTLED * st->tol ||
+                                          (st->change <= st->tol && st->iter >= st->prev_inv_total)
+                                    : st->change <= st->tol;
+  if (enough) st->converged = 1;
+  else if (st->iter >= st->max_iter) st->stopped = 1;
+}
+
 struct AdjointEpi {
   static constexpr int NACC = 2;
+  static constexpr bool SUMS = true;
   const double* g;
   const double* lam_old;
   double* lam_new;
@@ -36,7 +56,7 @@ struct AdjointEpi {
   double d, pu;
   double jdot = 0;
 
-  __device__ __forceinline__ void prepare(const IterState* st) { jdot = st ? st->dterm : 0.0; }
+  __device__ __forceinline__ void prepare(const IterState* st) { jdot = st->dterm; }
   static __device__ __forceinline__ void init(double* a) { a[0] = a[1] = 0.0; }
   static __device__ __forceinline__ double identity(int) { return 0.0; }
   static __device__ __forceinline__ double combine(int, double a, double b) { return a + b; }
@@ -52,8 +72,7 @@ struct AdjointEpi {
     st->change = tot[0];
     st->dterm = tot[1];
     st->iter += 1;
-    if (tot[0] <= st->tol) st->converged = 1;
-    else if (st->iter >= st->max_iter) st->stopped = 1;
+    adj_decide(st);
   }
 };
 
@@ -70,28 +89,109 @@ struct RowSumEpi {
   __device__ void finish(IterState*, const double*) const {}
 };
 
-__global__ void adj_init(const double* __restrict__ g, const double* __restrict__ jump, uint32_t n,
-                         double* __restrict__ lam, double* __restrict__ part, IterState* st) {
+// Sums of v and w over the CTAs of the grid (each CTA's value in thread 0),
+// in a fixed order; true in the last CTA, which gets them.
+__device__ __forceinline__ bool last_sums(double v, double w, double* part, unsigned int* ticket,
+                                          double* sh, double* t, double* u) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = v;
+    part[2 * blockIdx.x + 1] = w;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double x = 0, y = 0;
+  for (uint32_t q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
+    x += __ldcg(part + 2 * q);
+    y += __ldcg(part + 2 * q + 1);
+  }
+  *t = block_sum(x, sh);
+  *u = block_sum(y, sh);
+  return true;
+}
+
+// lambda = g; jump^T g; the tolerance, scaled by max(1, ||g||_1).
+__global__ void __launch_bounds__(256)
+adj_init(const double* __restrict__ g, const double* __restrict__ jump, uint32_t n, double tol,
+         double* __restrict__ lam, double* __restrict__ part, IterState* st) {
   __shared__ double sh[8];
-  double a = 0;
+  double a = 0, b = 0;
   const double pu = 1.0 / n;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    lam[i] = g[i];
-    a += (jump ? jump[i] : pu) * g[i];
+    const double v = g[i];
+    lam[i] = v;
+    a += (jump ? jump[i] : pu) * v;
+    b += fabs(v);
   }
   a = block_sum(a, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = a;
-  __threadfence();
+  b = block_sum(b, sh);
+  double t, u;
+  if (!last_sums(a, b, part, &st->ticket, sh, &t, &u) || threadIdx.x != 0) return;
+  st->dterm = t;
+  st->tol = tol * fmax(1.0, u);
+  st->ticket = 0;
+}
+
+// Extrapolation over the last SPAN sweeps. The part of lambda's error that G
+// keeps (the average over each closed class of nodes: G^SPAN leaves it as it
+// is, also where a class is a cycle of SPAN's divisors 2, 3 or 6) shrinks by
+// d^SPAN over SPAN sweeps, so E = b + c (b - a), c = d^SPAN / (1 - d^SPAN),
+// has none of it, where a is the iterate SPAN sweeps before b. Sweeping is
+// affine: had lambda been extrapolated one sweep earlier (from a0 and b0, the
+// iterates before a and b), this sweep would have turned it into E with the
+// change (1 + c) (b - b0) - c (a - a0). So E's place in the iteration, its
+// change and the same stopping rule come from one pass over four vectors, and
+// E is taken only where that change is below half of the plain one: a graph
+// whose error has no such part keeps the plain iteration.
+constexpr int SPAN = 6;
+constexpr int CYCLE = 24;  // an extrapolation is tried every CYCLE sweeps
+
+__global__ void __launch_bounds__(256)
+adj_extrapolate(const double* __restrict__ a0, const double* __restrict__ a,
+                const double* __restrict__ b0, const double* __restrict__ b, double c, double d,
+                const double* __restrict__ jump, uint32_t n, double* __restrict__ part,
+                IterState* st) {
+  if (iteration_done(st)) return;
+  __shared__ double sh[8];
+  double ch = 0, jd = 0;
+  const double pu = 1.0 / n;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double av = a[i], bv = b[i];
+    ch += fabs((1.0 + c) * (bv - b0[i]) - c * (av - a0[i]));
+    jd += (jump ? jump[i] : pu) * (bv + c * (bv - av));
+  }
+  ch = block_sum(ch, sh);
+  jd = block_sum(jd, sh);
+  double t, u;
+  if (!last_sums(ch, jd, part, &st->ticket, sh, &t, &u) || threadIdx.x != 0) return;
+  st->ticket = 0;
+  if (!(t < 0.5 * st->change)) return;
+  if (!st->ambiguous) {
+    st->ambiguous = 1;
+    st->prev_inv_total = st->iter + ceil(log(st->tol / st->change) / log(d));
+  }
+  st->top = 1.0;  // adj_take replaces b by E
+  st->change = t;
+  st->dterm = u;
+  adj_decide(st);
+}
+
+__global__ void adj_take(const double* __restrict__ a, double* __restrict__ b, double c,
+                         uint32_t n, IterState* st) {
+  if (st->top == 0.0) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    b[i] = b[i] + c * (b[i] - a[i]);
   __shared__ bool last;
+  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
   __syncthreads();
-  if (!last) return;
-  double t = 0;
-  for (uint32_t q = threadIdx.x; q < gridDim.x; q += blockDim.x) t += __ldcg(part + q);
-  t = block_sum(t, sh);
-  if (threadIdx.x == 0) {
-    st->dterm = t;
+  if (last && threadIdx.x == 0) {
+    st->top = 0.0;
     st->ticket = 0;
   }
 }
@@ -132,22 +232,36 @@ __global__ void adj_grad(const uint32_t* __restrict__ src, const uint32_t* __res
   }
 }
 
-static void normalized_jump(const double* d_pers, uint32_t n, DevBuf<double>& out,
-                            cudaStream_t s) {
-  std::vector<double> h(n);
-  KNB_CUDA(cudaMemcpyAsync(h.data(), d_pers, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaStreamSynchronize(s));
-  double t = 0;
-  for (double v : h) {
-    if (!std::isfinite(v) || v < 0.0)
-      throw Error("the personalization vector must hold finite, nonnegative values");
-    t += v;
+// Buffers, pinned state and events of adjoint solves, kept with the weight
+// slot of the forward operator (whose mutex a solve holds) between calls.
+struct AdjointWorkspace : Workspace {
+  DevBuf<double> lam[4], r, carry, head, part1, part2, part3, jump;
+  DevBuf<double2> terms;
+  DevBuf<IterState> st;
+  IterState* hst = nullptr;  // pinned, 2 slots
+  cudaEvent_t t0 = nullptr, t1 = nullptr, done[2] = {nullptr, nullptr};
+  ~AdjointWorkspace() override {
+    if (hst) cudaFreeHost(hst);
+    for (cudaEvent_t e : {t0, t1, done[0], done[1]})
+      if (e) cudaEventDestroy(e);
   }
-  if (!(t > 0.0)) throw Error("the personalization vector must have a positive sum");
-  for (double& v : h) v /= t;
-  out.alloc(n);
-  KNB_CUDA(cudaMemcpyAsync(out.get(), h.data(), (size_t)n * 8, cudaMemcpyHostToDevice, s));
-}
+  void ensure(uint32_t n, uint32_t ntiles) {
+    if (hst) return;  // a slot's sizes never change
+    for (auto& l : lam) l.alloc(n);
+    r.alloc(n);
+    terms.alloc(n);
+    carry.alloc(ntiles + 1);
+    head.alloc(ntiles + 1);
+    part1.alloc((size_t)ntiles * AdjointEpi::NACC + 4);
+    part2.alloc((size_t)SPLIT_CTAS * AdjointEpi::NACC + 4);
+    part3.alloc(2 * 1184 + 2);
+    st.alloc(1);
+    KNB_CUDA(cudaEventCreate(&t0));
+    KNB_CUDA(cudaEventCreate(&t1));
+    for (auto& e : done) KNB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    KNB_CUDA(cudaMallocHost(&hst, 2 * sizeof(IterState)));
+  }
+};
 
 void pagerank_weights(GraphHandleImpl& g, const double* d_w, const PagerankParams& prm,
                       double* d_out, PagerankInfo* info, cudaStream_t s) {
@@ -156,7 +270,7 @@ void pagerank_weights(GraphHandleImpl& g, const double* d_w, const PagerankParam
   const double lf = pagerank_loop_factor(which, prm.loops);
   GraphHandleImpl::WeightSlot& slot = g.weight_slot(which, lf, s);
   std::lock_guard<std::mutex> lock(slot.mu);
-  g.fill_weights(*slot.op, d_w, lf, true, s);
+  g.fill_weights(*slot.op, d_w, lf, true, true, s);
   PagerankParams p = prm;
   p.weighted = true;
   p.relabel = false;  // values change every call: no renumbered copy
@@ -180,100 +294,121 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
   Operator* fwd = fslot.op.get();
   Operator* tr = tslot.op.get();
   // the sweeps pull over tr's values; of fwd only the out-strengths are read
-  if (tr == fwd) {
-    g.fill_weights(*fwd, d_w, lf, true, s);
-  } else {
-    g.fill_weights(*tr, d_w, lf, false, s);
-    g.fill_weights(*fwd, d_w, lf, true, s);
+  g.fill_weights(*tr, d_w, lf, true, tr == fwd, s);
+  if (tr != fwd) g.fill_weights(*fwd, d_w, lf, false, true, s);
+  constexpr int IPT = 4, WPB = 16;
+  const Partition& P = tr->partition(32 * IPT, s);
+  if (!fslot.adj_ws) fslot.adj_ws = std::make_unique<AdjointWorkspace>();
+  AdjointWorkspace& W = *static_cast<AdjointWorkspace*>(fslot.adj_ws.get());
+  W.ensure(n, P.ntiles);
+  const double* jump = nullptr;
+  if (prm.personalization && prm.dangling == 0) {
+    if (!W.jump.p) W.jump.alloc(n);
+    KNB_CUDA(cudaMemcpyAsync(W.jump.get(), prm.personalization, (size_t)n * 8,
+                             cudaMemcpyDeviceToDevice, s));
+    normalize_personalization_device(W.jump.get(), n, s);
+    jump = W.jump.get();
   }
-  const Partition& P = tr->partition(128, s);
-  DevBuf<double> jump;
-  if (prm.personalization && prm.dangling == 0) normalized_jump(prm.personalization, n, jump, s);
-
-  // ||g||_1 scales the stopping rule
-  std::vector<double> hg(n);
-  KNB_CUDA(cudaMemcpyAsync(hg.data(), d_gx, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaStreamSynchronize(s));
-  double gnorm = 0;
-  for (double v : hg) gnorm += std::fabs(v);
-
-  DevBuf<double> lam[2] = {DevBuf<double>(n), DevBuf<double>(n)}, r(n), carry(P.ntiles + 1),
-                head(P.ntiles + 1), part1((size_t)P.ntiles * 2 + 2),
-                part2((size_t)SPLIT_CTAS * 2 + 2), part3(1184 + 2);
-  DevBuf<double2> terms(n);
-  DevBuf<IterState> st(1);
-  IterState is{};
-  is.tol = prm.tol * std::max(1.0, gnorm);
-  is.max_iter = (int32_t)std::min<int64_t>(prm.max_iter, INT32_MAX);
-  KNB_CUDA(cudaMemcpyAsync(st.get(), &is, sizeof(is), cudaMemcpyHostToDevice, s));
-  cudaEvent_t t0, t1;
-  KNB_CUDA(cudaEventCreate(&t0));
-  KNB_CUDA(cudaEventCreate(&t1));
-  KNB_CUDA(cudaEventRecord(t0, s));
+  IterState* st = W.st.get();
+  W.hst[0] = IterState{};
+  W.hst[0].max_iter = (int32_t)std::min<int64_t>(prm.max_iter, INT32_MAX);
+  KNB_CUDA(cudaMemcpyAsync(st, &W.hst[0], sizeof(IterState), cudaMemcpyHostToDevice, s));
+  KNB_CUDA(cudaEventRecord(W.t0, s));
   const unsigned gv = grid_for(n, 256, 1184);
-  adj_init<<<gv, 256, 0, s>>>(d_gx, jump.get(), n, lam[0].get(), part3.get(), st.get());
+  adj_init<<<gv, 256, 0, s>>>(d_gx, jump, n, prm.tol, W.lam[0].get(), W.part3.get(), st);
   KNB_LAUNCH("adj_init");
   int launches = 1;
-  constexpr int IPT = 4, WPB = 4;
+  // one CTA of 16 warps takes tiles until none is left; as many CTAs as fit
+  // at once (against one tile per warp and 4 warps per CTA: 104 -> 79 us a
+  // sweep on R-MAT 20)
   constexpr size_t smem = warp_smem_bytes<double, IPT, WPB>();
-  const unsigned grid = (P.ntiles + WPB - 1) / WPB;
+  const unsigned grid =
+      std::min((P.ntiles + WPB - 1) / WPB, 148u * (unsigned)warp_min_blocks<double, IPT, WPB>());
+  const uint32_t npart = std::min<uint32_t>(P.ntiles, grid * WPB);
   const OpView<double> v = tr->view64();
-  IterState h{};
-  int k = 0;
   fit_warp_carveout<double, double, AdjointEpi, IPT, WPB>();
   fit_warp_carveout<double, double, RowSumEpi, IPT, WPB>();
-  for (;;) {
-    for (int b = 0; b < 8; ++b, ++k) {
+  const double dspan = std::pow(prm.damping, SPAN), c = dspan / (1.0 - dspan);
+  // Sweep k turns iterate k into iterate k + 1. Iterates alternate between
+  // two buffers, but the two that an extrapolation looks back on (SPAN + 1
+  // and SPAN sweeps before the end of a cycle) have buffers of their own.
+  auto buffer = [&](int k) -> double* {
+    const int at = k == 0 ? 0 : (k - 1) % CYCLE + 1;  // place in its cycle, 1..CYCLE
+    return W.lam[at == CYCLE - SPAN - 1 ? 2 : at == CYCLE - SPAN ? 3 : k & 1].get();
+  };
+  int k = 0;
+  auto enqueue = [&](int slot) {
+    for (int q = 0; q < 8; ++q, ++k) {
       AdjointEpi e;
       e.g = d_gx;
-      e.lam_old = lam[k & 1].get();
-      e.lam_new = lam[1 - (k & 1)].get();
+      e.lam_old = buffer(k);
+      e.lam_new = buffer(k + 1);
       e.inv_out = fwd->inv_out64.get();
-      e.jump = jump.get();
+      e.jump = jump;
       e.d = prm.damping;
       e.pu = 1.0 / n;
       warp_spmv<double, double, AdjointEpi, IPT, WPB><<<grid, WPB * 32, smem, s>>>(
-          v, lam[k & 1].get(), e, P.coords.get(), P.ntiles, carry.get(), head.get(), part1.get(),
-          st.get(), 0xFFFFFFFFu);
+          v, buffer(k), e, P.coords.get(), P.ntiles, W.carry.get(), W.head.get(), W.part1.get(),
+          st, 0xFFFFFFFFu);
       split_rows<double, AdjointEpi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(
-          P.split.get(), P.nsplit, P.nshort, carry.get(), head.get(), e, part1.get(), P.ntiles,
-          part2.get(), st.get());
+          P.split.get(), P.nsplit, P.nshort, W.carry.get(), W.head.get(), e, W.part1.get(), npart,
+          W.part2.get(), st);
       launches += 2;
+      if ((k + 1) % CYCLE == 0) {
+        adj_extrapolate<<<gv, 256, 0, s>>>(W.lam[2].get(), W.lam[3].get(), buffer(k),
+                                           buffer(k + 1), c, prm.damping, jump, n, W.part3.get(),
+                                           st);
+        adj_take<<<gv, 256, 0, s>>>(W.lam[3].get(), buffer(k + 1), c, n, st);
+        launches += 2;
+      }
     }
     KNB_LAUNCH("adjoint sweep");
-    KNB_CUDA(cudaMemcpyAsync(&h, st.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
-    KNB_CUDA(cudaStreamSynchronize(s));
-    if (h.converged || h.stopped) break;
+    KNB_CUDA(cudaMemcpyAsync(&W.hst[slot], st, sizeof(IterState), cudaMemcpyDeviceToHost, s));
+    KNB_CUDA(cudaEventRecord(W.done[slot], s));
+  };
+  // one batch of sweeps in flight ahead of the state the host looks at;
+  // sweeps after the end exit at once
+  enqueue(0);
+  for (int slot = 0;; slot ^= 1) {
+    enqueue(slot ^ 1);
+    KNB_CUDA(cudaEventSynchronize(W.done[slot]));
+    if (W.hst[slot].converged || W.hst[slot].stopped) {
+      KNB_CUDA(cudaEventSynchronize(W.done[slot ^ 1]));
+      break;
+    }
   }
-  if (!h.converged)
+  const IterState h = W.hst[0].iter > W.hst[1].iter ? W.hst[0] : W.hst[1];
+  // The cap counts the sweeps of the plain iteration.
+  const bool within =
+      h.converged && (!h.ambiguous || h.prev_inv_total <= (double)prm.max_iter);
+  if (!within)
     throw Error("the PageRank adjoint did not converge within " + std::to_string(prm.max_iter) +
                 " iterations");
-  const double* lam_final = lam[h.iter & 1].get();
+  const double* lam_final = buffer(h.iter);
   // (M^T lambda)_j numerators with the final lambda, then the edge gradients
   {
-    RowSumEpi e{r.get()};
+    RowSumEpi e{W.r.get()};
     warp_spmv<double, double, RowSumEpi, IPT, WPB><<<grid, WPB * 32, smem, s>>>(
-        v, lam_final, e, P.coords.get(), P.ntiles, carry.get(), head.get(), part1.get(), nullptr,
-        0xFFFFFFFFu);
+        v, lam_final, e, P.coords.get(), P.ntiles, W.carry.get(), W.head.get(), W.part1.get(),
+        nullptr, 0xFFFFFFFFu);
     split_rows<double, RowSumEpi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(
-        P.split.get(), P.nsplit, P.nshort, carry.get(), head.get(), e, part1.get(), P.ntiles,
-        part2.get(), nullptr);
-    adj_node_terms<<<grid_for(n, 256), 256, 0, s>>>(d_x, fwd->inv_out64.get(), r.get(), n,
-                                                    prm.damping, terms.get());
+        P.split.get(), P.nsplit, P.nshort, W.carry.get(), W.head.get(), e, W.part1.get(), npart,
+        W.part2.get(), nullptr);
+    adj_node_terms<<<grid_for(n, 256), 256, 0, s>>>(d_x, fwd->inv_out64.get(), W.r.get(), n,
+                                                    prm.damping, W.terms.get());
     if (g.m)
-      adj_grad<<<grid_for(g.m, 256), 256, 0, s>>>(g.src.get(), g.tgt.get(), g.m, lf, terms.get(),
-                                                  lam_final, which != 1 ? 1 : 0, d_gw);
+      adj_grad<<<grid_for(g.m, 256), 256, 0, s>>>(g.src.get(), g.tgt.get(), g.m, lf,
+                                                  W.terms.get(), lam_final, which != 1 ? 1 : 0,
+                                                  d_gw);
     launches += 4;
     KNB_LAUNCH("adjoint gradient");
   }
   if (d_lambda)
     KNB_CUDA(cudaMemcpyAsync(d_lambda, lam_final, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
-  KNB_CUDA(cudaEventRecord(t1, s));
+  KNB_CUDA(cudaEventRecord(W.t1, s));
   KNB_CUDA(cudaStreamSynchronize(s));
   float ms = 0;
-  KNB_CUDA(cudaEventElapsedTime(&ms, t0, t1));
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
+  KNB_CUDA(cudaEventElapsedTime(&ms, W.t0, W.t1));
   if (info) {
     info->iterations = h.iter;
     info->change = h.change;

@@ -187,12 +187,13 @@ struct GraphHandleImpl {
   struct WeightSlot {
     std::mutex mu;
     std::unique_ptr<Operator> op;
+    std::unique_ptr<Workspace> adj_ws;  // adjoint solves' (adjoint.cu), created on first use
   };
   std::map<std::pair<int, int>, std::unique_ptr<WeightSlot>> wslots;  // guarded by mu
   WeightSlot& weight_slot(int which, double loop_factor, cudaStream_t s);
-  // Arc values of o from d_w; with `sums` also the column sums and their
-  // inverses.
-  void fill_weights(Operator& o, const double* d_w, double loop_factor, bool sums,
+  // From d_w, the arc values of o (`values`) and its column sums and their
+  // inverses (`sums`).
+  void fill_weights(Operator& o, const double* d_w, double loop_factor, bool values, bool sums,
                     cudaStream_t s);
 };
 

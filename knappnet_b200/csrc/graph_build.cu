@@ -994,14 +994,14 @@ static std::unique_ptr<Operator> weights_skeleton(GraphHandleImpl& g, int which,
   return o;
 }
 
-void GraphHandleImpl::fill_weights(Operator& o, const double* d_w, double lf, bool sums,
-                                   cudaStream_t s) {
+void GraphHandleImpl::fill_weights(Operator& o, const double* d_w, double lf, bool values,
+                                   bool sums, cudaStream_t s) {
   const DevCsr* rows = o.rows;
   const DevCsr* trans = o.trans;
   DevBuf<unsigned int> flags(2);
   KNB_CUDA(cudaMemsetAsync(flags.get(), 0, 8, s));
   const bool loops = lf != 1.0 && o.n_loops > 0;
-  if (o.nnz) {
+  if (values && o.nnz) {
     arc_values<<<grid_for(o.nnz, 256), 256, 0, s>>>(rows->edge.get(), d_w, o.nnz, o.vals64.get(),
                                                     o.vals32.get(), flags.get());
     if (loops)
@@ -1016,7 +1016,7 @@ void GraphHandleImpl::fill_weights(Operator& o, const double* d_w, double lf, bo
   unsigned int hf[2] = {0, 0};
   KNB_CUDA(cudaMemcpyAsync(hf, flags.get(), 8, cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
-  o.vals32_exact = hf[0] == 0;
+  if (values) o.vals32_exact = hf[0] == 0;
   if (sums) o.n_dangling = hf[1];
 }
 

@@ -117,3 +117,72 @@ def test_weights_forward_matches_graph_weights():
                                                  ctypes.c_void_p(out.data_ptr()),
                                                  ctypes.byref(info), err, K.ERR_LEN), err)
     assert np.abs(out.cpu().numpy() - a).sum() <= 1e-12
+
+
+def adjoint_vector(g, w, x, gx, tol=0.0, max_iter=0, pers=None, dangling=0):
+    """net_pagerank_grad_device with the adjoint vector: (grad, lambda, info)."""
+    import ctypes
+    grad = torch.empty(g.m, dtype=torch.float64, device="cuda")
+    lam = torch.empty(g.n, dtype=torch.float64, device="cuda")
+    info = K.NetSolveInfo()
+    err = ctypes.create_string_buffer(K.ERR_LEN)
+    p = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
+    torch.cuda.synchronize()
+    K._check(K.lib().net_pagerank_grad_device(g.h, p(w), p(x), p(gx), 0.85, int(g.directed),
+                                              p(pers), dangling, 0, tol, max_iter, p(grad), p(lam),
+                                              ctypes.byref(info), err, K.ERR_LEN), err)
+    return grad, lam, info
+
+
+@pytest.mark.parametrize("shape", ["mixing", "two closed halves", "cycle"])
+@pytest.mark.parametrize("personalized", [False, True])
+def test_adjoint_vector_solves_its_equation(shape, personalized):
+    """lambda = g + d G lambda, whether one closed class holds all that shrinks
+    slowly (mixing), two do (two closed halves), or no part of the change
+    shrinks faster than d (a cycle)."""
+    from knappnet_b200 import autograd as A
+    n = 400
+    rng = np.random.default_rng(11)
+    if shape == "cycle":
+        src, tgt = np.arange(n), (np.arange(n) + 1) % n
+    else:
+        src, tgt = rng.integers(0, n, 4000), rng.integers(0, n, 4000)
+        if shape == "two closed halves":
+            tgt = tgt % (n // 2) + np.where(src < n // 2, 0, n // 2)
+        else:  # dangling nodes
+            src = np.where(src >= n - 40, src - 40, src)
+    w = rng.lognormal(size=len(src))
+    g = K.Graph(n, src, tgt, w, True)
+    wt = torch.tensor(w, device="cuda")
+    pers = torch.rand(n, dtype=torch.float64, device="cuda") if personalized else None
+    x = A.pagerank(wt, g, personalization=pers, tol=1e-14).detach()
+    gx = torch.randn(n, dtype=torch.float64, device="cuda")
+    _, lam, info = adjoint_vector(g, wt, x, gx, pers=pers)
+    G = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    G.index_put_((torch.as_tensor(src, device="cuda"), torch.as_tensor(tgt, device="cuda")), wt,
+                 accumulate=True)
+    out = G.sum(1, keepdim=True)
+    jump = torch.full((n,), 1.0 / n, dtype=torch.float64, device="cuda")
+    if personalized:
+        jump = pers / pers.sum()
+    G = torch.where(out > 0, G / torch.where(out > 0, out, torch.ones_like(out)), jump)
+    ref = torch.linalg.solve(torch.eye(n, dtype=torch.float64, device="cuda") - 0.85 * G, gx)
+    # a change of at most tol max(1, ||g||_1) leaves an L1 error of at most
+    # n d / (1 - d) times it, and the dense solve one of its condition number
+    bound = n * 0.85 / 0.15 * 1e-12 * max(1.0, gx.abs().sum().item())
+    assert (lam - ref).abs().sum().item() <= bound + 1e-12 * ref.abs().sum().item()
+    if shape != "cycle":
+        assert info.iterations < 100  # 0.85^k alone would need 170
+
+
+def test_adjoint_iteration_cap_means_the_same_sweeps():
+    """The cap counts the sweeps the tolerance needs (the constant part shrinks
+    by d = 0.85: about ln(1e-12) / ln(0.85) = 170 here), though fewer run."""
+    g = K.generate_rmat(10, 16, seed=8, clean=True, lognormal=True, wseed=9)
+    w = torch.tensor(g.edges()[2], device="cuda")
+    x = torch.tensor(g.pagerank(weighted=True), device="cuda")
+    gx = torch.rand(g.n, dtype=torch.float64, device="cuda")
+    with pytest.raises(K.EngineError, match="did not converge within 100 iterations"):
+        adjoint_vector(g, w, x, gx, max_iter=100)
+    _, _, info = adjoint_vector(g, w, x, gx, max_iter=400)
+    assert info.iterations <= 400
