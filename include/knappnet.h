@@ -534,7 +534,9 @@ NET_API void net_shard_free(NetShard *shard);
 NET_API int32_t net_measure_gather(int32_t source, int64_t words, double *gathers_per_second,
                                    char *err, size_t err_len);
 
-/* Waits for the device; reports an asynchronous CUDA error if one occurred. */
+/* Waits for the device; reports an asynchronous CUDA error if one occurred.
+ * Also gives back to the driver the device memory the library keeps for its
+ * next allocations (at most 512 MiB per device between calls). */
 NET_API int32_t net_device_sync(char *err, size_t err_len);
 
 #ifdef __cplusplus

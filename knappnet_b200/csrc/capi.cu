@@ -1553,7 +1553,10 @@ int32_t net_shard_scores(const NetShard* shard, double* out, int32_t out_on_devi
 void net_shard_free(NetShard* shard) { delete shard; }
 
 int32_t net_device_sync(char* err, size_t err_len) {
-  return guard(err, err_len, [&] { KNB_CUDA(cudaDeviceSynchronize()); });
+  return guard(err, err_len, [&] {
+    KNB_CUDA(cudaDeviceSynchronize());
+    knb::device_pool_trim();
+  });
 }
 
 }  // extern "C"

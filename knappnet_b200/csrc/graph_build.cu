@@ -3,6 +3,8 @@
 // spectral measures.
 #include <algorithm>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "graph.cuh"
 
@@ -18,6 +20,94 @@ cudaStream_t thread_stream() {
     dev = cur;
   }
   return s;
+}
+
+// ======================================================================= device memory
+static thread_local int g_plain_memory = 0;
+PlainMemory::PlainMemory() { ++g_plain_memory; }
+PlainMemory::~PlainMemory() { --g_plain_memory; }
+
+// The pool of device `dev`, or null where the device has none.
+static cudaMemPool_t device_pool(int dev) {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = pools.find(dev);
+  if (it != pools.end()) return it->second;
+  cudaMemPool_t pool = nullptr;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  uint64_t keep = POOL_KEEP;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();
+    pool = nullptr;
+  }
+  pools[dev] = pool;
+  return pool;
+}
+
+DeviceBlock device_alloc(size_t bytes) {
+  DeviceBlock b;
+  KNB_CUDA(cudaGetDevice(&b.device));
+  cudaMemPool_t pool =
+      g_plain_memory || bytes > POOL_BLOCK ? nullptr : device_pool(b.device);
+  cudaError_t e;
+  if (pool) {
+    cudaStream_t s = thread_stream();
+    e = cudaMallocFromPoolAsync(&b.p, bytes, pool, s);
+    if (e != cudaSuccess) {  // once more with what other blocks still hold given back
+      cudaGetLastError();
+      cudaDeviceSynchronize();
+      cudaMemPoolTrimTo(pool, 0);
+      e = cudaMallocFromPoolAsync(&b.p, bytes, pool, s);
+    }
+    b.pooled = true;
+  } else {
+    e = cudaMalloc(&b.p, bytes);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      device_pool_trim();
+      e = cudaMalloc(&b.p, bytes);
+    }
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    throw Error("out of device memory allocating " + std::to_string(bytes) + " bytes");
+  }
+  return b;
+}
+
+void device_free(const DeviceBlock& b) noexcept {
+  if (!b.pooled) {
+    cudaFree(b.p);
+    return;
+  }
+  int cur = -1;
+  try {
+    if (cudaGetDevice(&cur) == cudaSuccess && cur == b.device &&
+        cudaFreeAsync(b.p, thread_stream()) == cudaSuccess)
+      return;
+  } catch (...) {
+  }
+  // another device is current: wait for the block's own, then free it there
+  cudaGetLastError();
+  if (cur >= 0 && cur != b.device && cudaSetDevice(b.device) == cudaSuccess) {
+    cudaDeviceSynchronize();
+    cudaFree(b.p);
+    cudaSetDevice(cur);
+  }
+}
+
+void device_pool_trim() {
+  int dev = 0;
+  KNB_CUDA(cudaGetDevice(&dev));
+  if (cudaMemPool_t pool = device_pool(dev)) {
+    KNB_CUDA(cudaDeviceSynchronize());
+    KNB_CUDA(cudaMemPoolTrimTo(pool, 0));
+  }
 }
 
 // ======================================================================= scan

@@ -229,6 +229,8 @@ std::unique_ptr<Shard> shard_new(Operator& op, double damping, const double* d_p
     if (bounds[k + 1] < bounds[k]) throw Error("shard bounds must not decrease");
     widest = std::max<size_t>(widest, (size_t)(bounds[k + 1] - bounds[k]));
   }
+  // a shard's calls run on the caller's streams
+  PlainMemory plain;
   auto sh = std::make_unique<Shard>();
   sh->op = &op;
   sh->n = op.n;
@@ -287,6 +289,7 @@ std::unique_ptr<Shard> shard_new(Operator& op, double damping, const double* d_p
 }
 
 void shard_sweep(Shard& sh, double* d_payload, cudaStream_t s) {
+  PlainMemory plain;
   const uint32_t rows = sh.r1 - sh.r0;
   if (rows > 0) {
     const Operator& op = *sh.op;
@@ -304,6 +307,7 @@ void shard_sweep(Shard& sh, double* d_payload, cudaStream_t s) {
 
 void shard_scores(Shard& sh, double* out, bool out_on_device, cudaStream_t s) {
   if (sh.n == 0) return;
+  PlainMemory plain;
   double* dst = out;
   if (!out_on_device) {
     if (!sh.scores.p) sh.scores.alloc(sh.n);
