@@ -13,6 +13,14 @@
 // sums are kept per lane, joined per CTA in warp order and per sweep in CTA
 // order, so the results do not change from run to run.
 //
+// A sweep costs what its width costs, and columns stop at very different sweeps
+// (most of 100 seed sets on R-MAT 20 after 17 to 43, one that reaches a closed
+// class after 125), so the columns still running are packed into a narrower
+// iterate whenever a quarter of the width has stopped; the others leave with
+// their result. On that batch only 23% of the column-sweeps of full-width
+// sweeps did anything (380 ms a solve at full width, 125 ms packed). Up to 16 columns a warp takes several rows at once (spmm_rows with
+// W < 32 lanes per row).
+//
 // Precision: FP64, or mixed (FP32 sweeps until every column's change is below
 // max(tol * switch_factor, switch_floor), then, on the same trajectories, one
 // FP64 anchor sweep and refinement sweeps gathering the FP32 correction (or
@@ -51,17 +59,23 @@ struct ColState {
   int32_t frozen;         // converged (or finished) columns keep their iterate
   int32_t iter;           // sweeps this column took
   int32_t converged;
-  int32_t pad;
+  int32_t buf;            // the buffer its last sweep wrote
 };
 
+// A sweep's columns: `B` of them, the iterate's row length. Column c of the
+// sweep is column cmap[c] of the `Bo` columns the batch began with, which the
+// teleport columns and the refinement's FP64 arrays keep; inv is the inverse
+// (NO_COL for a column that has stopped and left).
+constexpr uint32_t NO_COL = 0xFFFFFFFFu;
 struct BatchScalars {
   double d;
   double pu;    // 1 / n
-  uint32_t n, B;
+  uint32_t n, B, Bo;
   int jump_uniform;
   double tol;
   int32_t max_iter;
-  int32_t exact;
+  const uint32_t* cmap;
+  const uint32_t* inv;
 };
 
 // Arcs whose gathers one warp keeps in flight together (U): 1, 2 or 4,
@@ -160,8 +174,8 @@ __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int la
   for (int v = 0; v < VW; ++v) psp[v] = PT(0);
   if (!pv.dense) {
     for (uint32_t e = pv.rowptr[i]; e < pv.rowptr[i + 1]; ++e) {
-      const uint32_t c = pv.cols[e];
-      if ((c & 31u) != (uint32_t)lane) continue;
+      const uint32_t c = __ldg(bs.inv + pv.cols[e]);
+      if (c == NO_COL || (c & 31u) != (uint32_t)lane) continue;
       const PT x = (PT)pv.vals[e];
 #pragma unroll
       for (int v = 0; v < VW; ++v)
@@ -176,7 +190,7 @@ __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int la
       if (c >= bs.B || cs[c].frozen) continue;
       const VT it = (VT)cs[c].inv_total, dt = (VT)cs[c].dterm;
       const size_t q = (size_t)i * bs.B + c;
-      const VT pg = pv.dense ? (VT)pv.dense[q] : psp[v];
+      const VT pg = pv.dense ? (VT)pv.dense[(size_t)i * bs.Bo + __ldg(bs.cmap + c)] : psp[v];
       const VT jg = bs.jump_uniform ? (VT)bs.pu : pg;
       const VT u = (VT)bs.d * (s[v] * it + dt * jg) + (VT)(1.0 - bs.d) * pg;
       const VT xo = Yold[q] * it;
@@ -198,17 +212,18 @@ __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int la
       if (c >= bs.B || cs[c].frozen) continue;
       const double it = cs[c].inv_total, dt = cs[c].dterm;
       const size_t q = (size_t)i * bs.B + c;
+      const size_t r = (size_t)i * bs.Bo + __ldg(bs.cmap + c);
       double sum;
       if constexpr (MODE == EPI_ANCHOR) {
         sum = (double)s[v];
-        rb.sref[q] = sum;
+        rb.sref[r] = sum;
       } else {
-        sum = rb.sref[q] + (double)s[v];
+        sum = rb.sref[r] + (double)s[v];
       }
-      const double pg = pv.dense ? pv.dense[q] : psp[v];
+      const double pg = pv.dense ? pv.dense[r] : psp[v];
       const double jg = bs.jump_uniform ? bs.pu : pg;
       const double u = bs.d * (sum * it + dt * jg) + (1.0 - bs.d) * pg;
-      const double yr = rb.yref[q];
+      const double yr = rb.yref[r];
       const double yo = MODE == EPI_ANCHOR ? yr : yr + (double)rb.eold[q];
       const float en = (float)(u - yr);
       const double us = yr + (double)en;  // the iterate as stored
@@ -221,28 +236,46 @@ __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int la
   }
 }
 
-// Zeroes this warp's slice [3][B] of the per-warp column sums in smem.
-__device__ __forceinline__ double* warp_sums(double* smem, uint32_t B) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double* red = smem + (size_t)w * 3 * B;
-  for (uint32_t q = lane; q < 3 * B; q += 32) red[q] = 0.0;
+// Lanes per row: a whole warp for more than 16 columns (lane l holds columns
+// l, l + 32, ...); up to 16 columns W lanes, the power of two that holds them,
+// so a warp takes 32 / W rows at once.
+template <int W>
+struct Lanes {
+  static constexpr int G = 32 / W;  // rows a warp takes at once
+  int col, group;
+  __device__ __forceinline__ Lanes() {
+    const int lane = threadIdx.x & 31;
+    col = lane % W;
+    group = lane / W;
+  }
+};
+
+// Zeroes this group's slice [3][B] of the CTA's column sums in smem
+// ([BW][G][3][B]) and returns it.
+template <int W>
+__device__ __forceinline__ double* group_sums(double* smem, uint32_t B) {
+  const Lanes<W> l;
+  double* red = smem + (size_t)((threadIdx.x >> 5) * Lanes<W>::G + l.group) * 3 * B;
+  for (uint32_t q = l.col; q < 3 * B; q += W) red[q] = 0.0;
   __syncwarp();
   return red;
 }
 
-// Joins the warps' per-column sums of a CTA (smem [BW][3][B]) in warp order
-// into part[cta][3][B].
+// Joins the groups' column sums of a CTA in order into part[cta][3][B].
+template <int W>
 __device__ __forceinline__ void cta_column_sums(uint32_t B, double* __restrict__ part,
                                                 const double* smem) {
   __syncthreads();
   for (uint32_t q = threadIdx.x; q < 3 * B; q += BT) {
     double a = 0;
-    for (int ww = 0; ww < BW; ++ww) a += smem[(size_t)ww * 3 * B + q];
+    for (int g = 0; g < BW * Lanes<W>::G; ++g) a += smem[(size_t)g * 3 * B + q];
     part[(size_t)blockIdx.x * 3 * B + q] = a;
   }
 }
 
-template <class VT, class MT, int VW, int U, int MODE>
+// The rows of at most LONG_ROW arcs: their products and updates. Bound by the
+// gathers, one iterate row (B values) per arc.
+template <class VT, class MT, int W, int VW, int U, int MODE>
 __global__ void __launch_bounds__(BT)
 spmm_rows(OpView<MT> op, const VT* __restrict__ Z, const RowRange* __restrict__ ranges,
           uint32_t nranges, BatchScalars bs, const ColState* __restrict__ cs,
@@ -251,45 +284,46 @@ spmm_rows(OpView<MT> op, const VT* __restrict__ Z, const RowRange* __restrict__ 
           double* __restrict__ part, const int32_t* __restrict__ all_frozen) {
   if (*all_frozen) return;
   extern __shared__ double smem_b[];
-  const int lane = threadIdx.x & 31;
-  double* red = warp_sums(smem_b, bs.B);
+  const Lanes<W> l;
+  double* red = group_sums<W>(smem_b, bs.B);
   const uint32_t gw = blockIdx.x * BW + (threadIdx.x >> 5), nw = gridDim.x * BW;
   for (uint32_t r = gw; r < nranges; r += nw) {
     const RowRange rr = ranges[r];
-    for (uint32_t i = rr.lo; i < rr.hi; ++i) {
+    for (uint32_t i = rr.lo + l.group; i < rr.hi; i += Lanes<W>::G) {
       const uint32_t a0 = op.off[i], a1 = op.off[i + 1];
       if (a1 - a0 > LONG_ROW) continue;  // long rows: spmm_chunks / spmm_long
       VT acc[VW];
-      row_product<VT, MT, VW, U>(op, Z, bs.B, a0, a1, lane, acc);
-      row_update<VT, VW, MODE>(i, acc, lane, bs, cs, Yold, Ynew, Znew, inv_out, P, rb, red);
+      row_product<VT, MT, VW, U>(op, Z, bs.B, a0, a1, l.col, acc);
+      row_update<VT, VW, MODE>(i, acc, l.col, bs, cs, Yold, Ynew, Znew, inv_out, P, rb, red);
     }
   }
-  cta_column_sums(bs.B, part, smem_b);
+  cta_column_sums<W>(bs.B, part, smem_b);
 }
 
 // Partial products of the chunks of long rows.
-template <class VT, class MT, int VW, int U>
+template <class VT, class MT, int W, int VW, int U>
 __global__ void __launch_bounds__(BT)
 spmm_chunks(OpView<MT> op, const VT* __restrict__ Z, const Chunk* __restrict__ chunks,
             uint32_t nchunks, uint32_t B, VT* __restrict__ scratch,
             const int32_t* __restrict__ all_frozen) {
   if (*all_frozen) return;
-  const int lane = threadIdx.x & 31;
-  const uint32_t gw = blockIdx.x * BW + (threadIdx.x >> 5), nw = gridDim.x * BW;
+  const Lanes<W> l;
+  const uint32_t gw = (blockIdx.x * BW + (threadIdx.x >> 5)) * Lanes<W>::G + l.group;
+  const uint32_t nw = gridDim.x * BW * Lanes<W>::G;
   for (uint32_t q = gw; q < nchunks; q += nw) {
     const Chunk ch = chunks[q];
     VT acc[VW];
-    row_product<VT, MT, VW, U>(op, Z, B, ch.a0, ch.a1, lane, acc);
+    row_product<VT, MT, VW, U>(op, Z, B, ch.a0, ch.a1, l.col, acc);
 #pragma unroll
     for (int v = 0; v < VW; ++v) {
-      const uint32_t c = lane + 32 * v;
+      const uint32_t c = l.col + 32 * v;
       if (c < B) scratch[(size_t)q * B + c] = acc[v];
     }
   }
 }
 
 // Long rows: chunk partials added in chunk order, then the update.
-template <class VT, int VW, int MODE>
+template <class VT, int W, int VW, int MODE>
 __global__ void __launch_bounds__(BT)
 spmm_long(const uint32_t* __restrict__ lrow, const uint32_t* __restrict__ lfirst, uint32_t nlong,
           const VT* __restrict__ scratch, BatchScalars bs, const ColState* __restrict__ cs,
@@ -298,48 +332,86 @@ spmm_long(const uint32_t* __restrict__ lrow, const uint32_t* __restrict__ lfirst
           double* __restrict__ part, const int32_t* __restrict__ all_frozen) {
   if (*all_frozen) return;
   extern __shared__ double smem_b[];
-  const int lane = threadIdx.x & 31;
-  double* red = warp_sums(smem_b, bs.B);
-  const uint32_t gw = blockIdx.x * BW + (threadIdx.x >> 5), nw = gridDim.x * BW;
+  const Lanes<W> l;
+  double* red = group_sums<W>(smem_b, bs.B);
+  const uint32_t gw = (blockIdx.x * BW + (threadIdx.x >> 5)) * Lanes<W>::G + l.group;
+  const uint32_t nw = gridDim.x * BW * Lanes<W>::G;
   for (uint32_t q = gw; q < nlong; q += nw) {
     VT acc[VW];
 #pragma unroll
     for (int v = 0; v < VW; ++v) acc[v] = VT(0);
+#pragma unroll 4
     for (uint32_t k = lfirst[q]; k < lfirst[q + 1]; ++k)
 #pragma unroll
       for (int v = 0; v < VW; ++v) {
-        const uint32_t c = lane + 32 * v;
+        const uint32_t c = l.col + 32 * v;
         if (c < bs.B) acc[v] += scratch[(size_t)k * bs.B + c];
       }
-    row_update<VT, VW, MODE>(lrow[q], acc, lane, bs, cs, Yold, Ynew, Znew, inv_out, P, rb, red);
+    row_update<VT, VW, MODE>(lrow[q], acc, l.col, bs, cs, Yold, Ynew, Znew, inv_out, P, rb, red);
   }
-  cta_column_sums(bs.B, part, smem_b);
+  cta_column_sums<W>(bs.B, part, smem_b);
 }
 
-// Per column: sums over the CTAs in order, the stopping rule, the scalars of
-// the next sweep; then whether every column is frozen.
-__global__ void spmm_finish(const double* __restrict__ part, uint32_t nparts, BatchScalars bs,
-                            ColState* cs, int32_t* all_frozen, int32_t count_sweep) {
-  __shared__ int any_active;
-  if (threadIdx.x == 0) any_active = 0;
+// tot[q] = sum over p of part[p][q], q < count: CTA j takes 32 values, its
+// warps every 32nd partial in order, then the warps' sums in order. One CTA
+// for all of them (a thread per column, 1,184 partials one after the other)
+// took 0.9 ms a sweep, as long as half of the products (10 us since).
+constexpr int SP_T = 1024;
+__device__ __forceinline__ void sum_parts_tile(const double* __restrict__ part, uint32_t nparts,
+                                               uint32_t count, double* __restrict__ tot) {
+  __shared__ double sh[32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t q = blockIdx.x * 32 + lane;
+  double a = 0.0;
+  if (q < count) {
+#pragma unroll 4
+    for (uint32_t p = w; p < nparts; p += 32) a += part[(size_t)p * count + q];
+  }
+  sh[w][lane] = a;
   __syncthreads();
-  if (*all_frozen) return;
+  if (w == 0 && q < count) {
+    double t = 0.0;
+    for (int k = 0; k < 32; ++k) t += sh[k][lane];
+    tot[q] = t;
+  }
+}
+
+__global__ void __launch_bounds__(SP_T)
+sum_parts(const double* __restrict__ part, uint32_t nparts, uint32_t count,
+          double* __restrict__ tot) {
+  sum_parts_tile(part, nparts, count, tot);
+}
+
+// The sweep's column sums, then (last CTA) per column the stopping rule and
+// the scalars of the next sweep, and whether every column is frozen.
+// flags: 0 all frozen, 1 ticket.
+__global__ void __launch_bounds__(SP_T)
+spmm_finish(const double* __restrict__ part, uint32_t nparts, BatchScalars bs, ColState* cs,
+            double* __restrict__ tot, int32_t* flags, int32_t newbuf) {
+  __shared__ int any_active;
+  __shared__ bool last;
+  if (flags[0]) return;
+  sum_parts_tile(part, nparts, 3 * bs.B, tot);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    any_active = 0;
+    last = atomicAdd((unsigned int*)flags + 1, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   for (uint32_t c = threadIdx.x; c < bs.B; c += blockDim.x) {
     ColState s = cs[c];
     if (!s.frozen) {
-      double T = 0, D = 0, ch = 0;
-      for (uint32_t q = 0; q < nparts; ++q) {
-        const double* p = part + (size_t)q * 3 * bs.B;
-        T += p[c];
-        D += p[bs.B + c];
-        ch += p[2 * bs.B + c];
-      }
+      const double T = __ldcg(tot + c), D = __ldcg(tot + bs.B + c), ch = __ldcg(tot + 2 * bs.B + c);
       s.prev_inv_total = s.inv_total;
       s.total = T;
       s.inv_total = 1.0 / T;
       s.dterm = D / T;
       s.change = ch;
-      s.iter += count_sweep;
+      s.iter += 1;
+      s.buf = newbuf;
       if (ch <= bs.tol) {
         s.converged = 1;
         s.frozen = 1;
@@ -351,14 +423,16 @@ __global__ void spmm_finish(const double* __restrict__ part, uint32_t nparts, Ba
     if (!s.frozen) atomicOr(&any_active, 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0 && !any_active) *all_frozen = 1;
+  if (threadIdx.x == 0) {
+    flags[1] = 0;
+    if (!any_active) flags[0] = 1;
+  }
 }
 
-// Start: Y = 1/n, Z = Y / out, per-column dangling mass (fixed-order sums).
+// Start: Y = 1/n, Z = Y / out.
 template <class VT>
 __global__ void spmm_init(VT* __restrict__ Y, VT* __restrict__ Zb, const VT* __restrict__ inv_out,
-                          uint32_t n, uint32_t B, double* __restrict__ colD) {
-  // one CTA per column group of 256 threads: thread c sums column c's dangling mass
+                          uint32_t n, uint32_t B) {
   const VT x0 = (VT)(1.0 / (double)n);
   const uint64_t total = (uint64_t)n * B;
   for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < total;
@@ -367,11 +441,10 @@ __global__ void spmm_init(VT* __restrict__ Y, VT* __restrict__ Zb, const VT* __r
     Y[q] = x0;
     Zb[q] = x0 * inv_out[i];
   }
-  (void)colD;
 }
 
 // Dangling count (same for every column at the start): D0 = n_dangling / n.
-__global__ void spmm_set_state(ColState* cs, uint32_t B, double dterm0, int32_t max_iter) {
+__global__ void spmm_set_state(ColState* cs, uint32_t B, double dterm0) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < B; c += gridDim.x * blockDim.x) {
     ColState s{};
     s.inv_total = 1.0;
@@ -380,24 +453,39 @@ __global__ void spmm_set_state(ColState* cs, uint32_t B, double dterm0, int32_t 
     s.total = 1.0;
     cs[c] = s;
   }
-  (void)max_iter;
 }
 
-// FP32 -> FP64 hand-over: Y64 = Y32 / T per column, read from the buffer the
-// column's FP32 phase stopped in; Z64 = Y64 / out.
-__global__ void spmm_switch(const float* __restrict__ Y0, const float* __restrict__ Y1,
-                            const ColState* __restrict__ cs32, double* __restrict__ Y64,
-                            double* __restrict__ Z64, const double* __restrict__ inv_out,
-                            uint32_t n, uint32_t B) {
-  const uint64_t total = (uint64_t)n * B;
+// The columns sel[0, count) of a sweep's iterate (row length B), packed.
+template <class VT>
+__global__ void spmm_pack(const VT* __restrict__ Y, const VT* __restrict__ Z, uint32_t n,
+                          uint32_t B, const uint32_t* __restrict__ sel, uint32_t count,
+                          VT* __restrict__ Yp, VT* __restrict__ Zp) {
+  const uint64_t total = (uint64_t)n * count;
   for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < total;
        q += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = (uint32_t)(q / B), c = (uint32_t)(q % B);
-    const ColState s = cs32[c];
-    const float* Y = (s.iter & 1) ? Y1 : Y0;
-    const double y = (double)Y[q] * s.inv_total;
-    Y64[q] = y;
-    Z64[q] = y * inv_out[i];
+    const uint32_t i = (uint32_t)(q / count), c = sel[q % count];
+    Yp[q] = Y[(size_t)i * B + c];
+    Zp[q] = Z[(size_t)i * B + c];
+  }
+}
+
+// FP32 -> FP64 hand-over of the columns sel[0, count) of a sweep that have
+// stopped: Y64 = Y32 / T, read from the buffer the column stopped in; Z64 =
+// Y64 / out, in the batch's own column order.
+__global__ void spmm_switch(const float* __restrict__ Y0, const float* __restrict__ Y1,
+                            const ColState* __restrict__ cs32, const uint32_t* __restrict__ sel,
+                            uint32_t count, const uint32_t* __restrict__ cmap, uint32_t B,
+                            uint32_t Bo, double* __restrict__ Y64, double* __restrict__ Z64,
+                            const double* __restrict__ inv_out, uint32_t n) {
+  const uint64_t total = (uint64_t)n * count;
+  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < total;
+       q += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)(q / count), c = sel[q % count];
+    const float* Y = cs32[c].buf ? Y1 : Y0;
+    const double y = (double)Y[(size_t)i * B + c] * cs32[c].inv_total;
+    const size_t r = (size_t)i * Bo + cmap[c];
+    Y64[r] = y;
+    Z64[r] = y * inv_out[i];
   }
 }
 
@@ -418,45 +506,48 @@ __global__ void column_sums_part(const double* __restrict__ Y, const double* __r
   part[(size_t)blockIdx.x * 2 * B + B + c] = D;
 }
 
-__global__ void column_sums_finish(const double* __restrict__ part, uint32_t nparts, uint32_t B,
-                                   ColState* cs) {
+__global__ void column_sums_finish(const double* __restrict__ tot, uint32_t B, ColState* cs) {
   const uint32_t c = threadIdx.x;
   if (c >= B) return;
-  double T = 0, D = 0;
-  for (uint32_t q = 0; q < nparts; ++q) {
-    T += part[(size_t)q * 2 * B + c];
-    D += part[(size_t)q * 2 * B + B + c];
-  }
   ColState s{};
-  s.total = T;
-  s.inv_total = 1.0 / T;
+  s.total = tot[c];
+  s.inv_total = 1.0 / s.total;
   s.prev_inv_total = s.inv_total;
-  s.dterm = D / T;
+  s.dterm = tot[B + c] / s.total;
   cs[c] = s;
 }
 
-// Personalization: column-major input (p[c * n + i]) checked and rescaled per
-// column, stored node-major.
-__global__ void pers_columns(const double* __restrict__ pin, uint32_t n, uint32_t B,
-                             double* __restrict__ pnm, int32_t* __restrict__ bad,
-                             double* __restrict__ sums) {
-  // one warp per column: fixed-order sum
-  const int lane = threadIdx.x & 31;
-  for (uint32_t c = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); c < B;
-       c += gridDim.x * (blockDim.x / 32)) {
-    double a = 0;
-    int b = 0;
-    for (uint32_t i = lane; i < n; i += 32) {
-      double v = pin[(size_t)c * n + i];
-      if (!isfinite(v) || v < 0.0) b = 1;
-      else a += v;
-    }
-    a = warp_sum(a);
-    b = __any_sync(0xffffffffu, b);
-    if (lane == 0) {
-      sums[c] = a;
-      if (b || !(a > 0.0)) atomicOr(bad, b ? 1 : 2);
-    }
+// Personalization: column-major input (p[c * n + i]) checked, and its sum per
+// column in a fixed order: PERS_CTAS CTAs a column (one warp a column took
+// 3.8 ms for 100 columns of 2^20 values, 0.13 ms since), then one warp.
+constexpr uint32_t PERS_CTAS = 32;
+__global__ void __launch_bounds__(BT)
+pers_columns(const double* __restrict__ pin, uint32_t n, double* __restrict__ part,
+             int32_t* __restrict__ bad) {
+  __shared__ double sh[BT / 32];
+  const uint32_t c = blockIdx.y;
+  const double* p = pin + (size_t)c * n;
+  double a = 0;
+  int b = 0;
+  for (uint32_t i = blockIdx.x * BT + threadIdx.x; i < n; i += PERS_CTAS * BT) {
+    const double v = p[i];
+    if (!isfinite(v) || v < 0.0) b = 1;
+    else a += v;
+  }
+  a = block_sum(a, sh);
+  if (__syncthreads_or(b) && threadIdx.x == 0) atomicOr(bad, 1);
+  if (threadIdx.x == 0) part[c * PERS_CTAS + blockIdx.x] = a;
+}
+
+__global__ void pers_sums(const double* __restrict__ part, uint32_t B, double* __restrict__ sums,
+                          int32_t* __restrict__ bad) {
+  static_assert(PERS_CTAS == 32, "one lane per CTA's sum");
+  const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (c >= B) return;
+  const double a = warp_sum(part[c * PERS_CTAS + lane]);
+  if (lane == 0) {
+    sums[c] = a;
+    if (!(a > 0.0)) atomicOr(bad, 2);
   }
 }
 
@@ -497,35 +588,40 @@ __global__ void pers_row_fill(const double* __restrict__ pin, const double* __re
   }
 }
 
-// Output: column-major out[c * n + i] = Y_c[i] / T_c from the buffer the
-// column stopped in.
+// Scores of the columns sel[0, count) of a sweep that have stopped, into
+// column-major out (column cmap[c]): Y / T from the buffer the column stopped
+// in, or with Yref (row length Bo) (y_ref + e) / T. A CTA transposes tiles of
+// 32 rows by 32 columns through shared memory, so that both sides are read and
+// written in runs (100 columns of 2^20: 4.1 ms without, 1.1 ms in the four
+// calls of a solve).
 template <class VT>
-__global__ void spmm_output(const VT* __restrict__ Y0, const VT* __restrict__ Y1,
-                            const ColState* __restrict__ cs, uint32_t n, uint32_t B,
-                            double* __restrict__ out) {
-  const uint64_t total = (uint64_t)n * B;
-  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < total;
-       q += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = (uint32_t)(q % n), c = (uint32_t)(q / n);
-    const ColState s = cs[c];
-    const VT* Y = (s.iter & 1) ? Y1 : Y0;
-    out[q] = (double)Y[(size_t)i * B + c] / s.total;
-  }
-}
-
-// Output of a refined phase: (y_ref + e) / total per column, e read from the
-// buffer of the column's last sweep.
-__global__ void spmm_output_ref(const double* __restrict__ Yref, const float* __restrict__ E0,
-                                const float* __restrict__ E1, const ColState* __restrict__ cs,
-                                uint32_t n, uint32_t B, double* __restrict__ out) {
-  const uint64_t total = (uint64_t)n * B;
-  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < total;
-       q += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = (uint32_t)(q % n), c = (uint32_t)(q / n);
-    const ColState s = cs[c];
-    const float* E = (s.iter & 1) ? E1 : E0;
-    const size_t r = (size_t)i * B + c;
-    out[q] = (Yref[r] + (double)E[r]) / s.total;
+__global__ void __launch_bounds__(256)
+spmm_output(const VT* __restrict__ Y0, const VT* __restrict__ Y1, const double* __restrict__ Yref,
+            const ColState* __restrict__ cs, const uint32_t* __restrict__ sel, uint32_t count,
+            const uint32_t* __restrict__ cmap, uint32_t B, uint32_t Bo, uint32_t n,
+            double* __restrict__ out) {
+  __shared__ double tile[32][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const uint32_t k0 = blockIdx.y * 32;
+  const bool live = k0 + x < count;
+  const uint32_t c = live ? sel[k0 + x] : 0u, co = live ? cmap[c] : 0u;
+  const VT* Y = live && cs[c].buf ? Y1 : Y0;
+  const double total = live ? cs[c].total : 1.0;
+  const uint32_t nt = (n + 31) / 32;
+  for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
+    for (int r = y; r < 32; r += 8) {
+      const uint32_t i = t * 32 + r;
+      if (!live || i >= n) continue;
+      double v = (double)Y[(size_t)i * B + c];
+      if (Yref) v = Yref[(size_t)i * Bo + co] + v;
+      tile[r][x] = v / total;
+    }
+    __syncthreads();
+    for (int k = y; k < 32; k += 8) {
+      const uint32_t i = t * 32 + x;
+      if (k0 + k < count && i < n) out[(size_t)cmap[sel[k0 + k]] * n + i] = tile[x][k];
+    }
+    __syncthreads();
   }
 }
 
@@ -567,63 +663,90 @@ static void upload(DevBuf<T>& d, const std::vector<T>& h, cudaStream_t s) {
   if (!h.empty()) KNB_CUDA(cudaMemcpyAsync(d.get(), h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
 }
 
-// One sweep: the row products and updates, then (finish) the per-column
-// sums, stopping rule and next sweep's scalars. Without finish the sweep
-// only rewrites Ynew, Znew, the chunk scratch and the partials.
-template <class VT, class MT, int VW, int U, int MODE>
-static int batch_sweep(const OpView<MT>& op, const DevBuf<RowRange>& ranges, uint32_t nranges,
-                       const DevBuf<Chunk>& chunks, uint32_t nchunks, const DevBuf<uint32_t>& lrow,
-                       const DevBuf<uint32_t>& lfirst, uint32_t nlong, const BatchScalars& bs,
+// What the sweeps of one operator share: its row plan, and the scratch.
+struct SweepPlan {
+  const RowRange* ranges;
+  const Chunk* chunks;
+  const uint32_t *lrow, *lfirst;
+  uint32_t nranges, nchunks, nlong;
+  double* part;
+  double* tot;
+  int32_t* flags;  // all frozen, ticket
+};
+
+// One sweep from buffers (Yold, Zold) to (Ynew, Znew) = buffer newbuf: the
+// row products and updates, then (finish) the per-column sums, stopping rule
+// and next sweep's scalars. Without finish the sweep only rewrites Ynew, Znew,
+// the chunk scratch and the partials.
+template <class VT, class MT, int W, int VW, int U, int MODE>
+static int batch_sweep(const OpView<MT>& op, const SweepPlan& sp, const BatchScalars& bs,
                        ColState* cs, const VT* Yold, VT* Ynew, const VT* Zold, VT* Znew,
                        const VT* inv_out, const PersView& P, const RefineBufs& rb, VT* scratch,
-                       double* part, int32_t* all_frozen, unsigned grid, bool finish,
-                       cudaStream_t s) {
-  const size_t smem = (size_t)BW * 3 * bs.B * sizeof(double);
-  set_func_attr((const void*)spmm_rows<VT, MT, VW, U, MODE>,
-                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BW * 3 * 256 * sizeof(double)));
-  set_func_attr((const void*)spmm_long<VT, VW, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                (int)(BW * 3 * 256 * sizeof(double)));
-  int launches = 0;
-  if (nchunks) {
-    spmm_chunks<VT, MT, VW, U><<<grid, BT, 0, s>>>(op, Zold, chunks.get(), nchunks, bs.B, scratch,
-                                                    all_frozen);
+                       int newbuf, bool finish, cudaStream_t s) {
+  // 32 resident warps per SM with whole-warp rows (their sums take 3 B doubles
+  // of shared memory a warp), 64 with narrow ones
+  const unsigned grid = W == 32 ? 148 * 4 : 148 * 8;
+  const size_t smem = (size_t)BW * Lanes<W>::G * 3 * bs.B * sizeof(double);
+  if (W == 32) {
+    set_func_attr((const void*)spmm_rows<VT, MT, W, VW, U, MODE>,
+                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                  (int)(BW * 3 * 256 * sizeof(double)));
+    set_func_attr((const void*)spmm_long<VT, W, VW, MODE>,
+                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                  (int)(BW * 3 * 256 * sizeof(double)));
+  }
+  int launches = 1;
+  if (sp.nchunks) {
+    spmm_chunks<VT, MT, W, VW, U><<<grid, BT, 0, s>>>(op, Zold, sp.chunks, sp.nchunks, bs.B,
+                                                       scratch, sp.flags);
     ++launches;
   }
-  spmm_rows<VT, MT, VW, U, MODE><<<grid, BT, smem, s>>>(op, Zold, ranges.get(), nranges, bs, cs,
-                                                        Yold, Ynew, Znew, inv_out, P, rb, part,
-                                                        all_frozen);
-  spmm_long<VT, VW, MODE><<<grid, BT, smem, s>>>(lrow.get(), lfirst.get(), nlong, scratch, bs, cs,
-                                                 Yold, Ynew, Znew, inv_out, P, rb,
-                                                 part + (size_t)grid * 3 * bs.B, all_frozen);
-  if (finish) spmm_finish<<<1, 256, 0, s>>>(part, 2 * grid, bs, cs, all_frozen, 1);
+  spmm_rows<VT, MT, W, VW, U, MODE><<<grid, BT, smem, s>>>(op, Zold, sp.ranges, sp.nranges, bs,
+                                                           cs, Yold, Ynew, Znew, inv_out, P, rb,
+                                                           sp.part, sp.flags);
+  unsigned parts = grid;
+  if (sp.nlong) {
+    const unsigned gl = std::min(grid, (sp.nlong + BW - 1) / BW);
+    spmm_long<VT, W, VW, MODE><<<gl, BT, smem, s>>>(sp.lrow, sp.lfirst, sp.nlong, scratch, bs, cs,
+                                                    Yold, Ynew, Znew, inv_out, P, rb,
+                                                    sp.part + (size_t)grid * 3 * bs.B, sp.flags);
+    parts += gl;
+    ++launches;
+  }
+  if (finish) {
+    spmm_finish<<<(3 * bs.B + 31) / 32, SP_T, 0, s>>>(sp.part, parts, bs, cs, sp.tot, sp.flags,
+                                                      newbuf);
+    ++launches;
+  }
   KNB_LAUNCH("batch sweep");
-  return launches + (finish ? 3 : 2);
+  return launches;
 }
 
+// u: arcs in flight per warp of a whole-warp row (1, 2 or 4; narrow rows,
+// whose lanes hold one column, keep 8).
 template <class VT, class MT, int MODE = EPI_PLAIN>
-static int batch_sweep_vw(int vw, int u, const OpView<MT>& op, const DevBuf<RowRange>& ranges,
-                          uint32_t nranges, const DevBuf<Chunk>& chunks, uint32_t nchunks,
-                          const DevBuf<uint32_t>& lrow, const DevBuf<uint32_t>& lfirst,
-                          uint32_t nlong, const BatchScalars& bs, ColState* cs, const VT* Yold,
-                          VT* Ynew, const VT* Zold, VT* Znew, const VT* inv_out, const PersView& P,
-                          VT* scratch, double* part, int32_t* all_frozen, unsigned grid,
-                          cudaStream_t s, bool finish = true, const RefineBufs& rb = RefineBufs{}) {
-#define KNB_SW(V, UU)                                                                             \
-  return batch_sweep<VT, MT, V, UU, MODE>(op, ranges, nranges, chunks, nchunks, lrow, lfirst,     \
-                                          nlong, bs, cs, Yold, Ynew, Zold, Znew, inv_out, P, rb,  \
-                                          scratch, part, all_frozen, grid, finish, s)
-#define KNB_SWU(V)                   \
-  switch (u) {                       \
-    case 1: KNB_SW(V, 1);            \
-    case 2: KNB_SW(V, 2);            \
-    default: KNB_SW(V, 4);           \
+static int batch_sweep_vw(int u, const OpView<MT>& op, const SweepPlan& sp, const BatchScalars& bs,
+                          ColState* cs, const VT* Yold, VT* Ynew, const VT* Zold, VT* Znew,
+                          const VT* inv_out, const PersView& P, const RefineBufs& rb, VT* scratch,
+                          int newbuf, cudaStream_t s, bool finish = true) {
+#define KNB_SW(WW, V, UU)                                                                          \
+  return batch_sweep<VT, MT, WW, V, UU, MODE>(op, sp, bs, cs, Yold, Ynew, Zold, Znew, inv_out, P,  \
+                                              rb, scratch, newbuf, finish, s)
+#define KNB_SWU(V)                       \
+  switch (u) {                           \
+    case 1: KNB_SW(32, V, 1);            \
+    case 2: KNB_SW(32, V, 2);            \
+    default: KNB_SW(32, V, 4);           \
   }
-  switch (vw) {
-    case 1: KNB_SWU(1);
-    case 2: KNB_SWU(2);
-    case 4: KNB_SWU(4);
-    default: KNB_SWU(8);
-  }
+  if (bs.B <= 1) KNB_SW(1, 1, 8);
+  if (bs.B <= 2) KNB_SW(2, 1, 8);
+  if (bs.B <= 4) KNB_SW(4, 1, 8);
+  if (bs.B <= 8) KNB_SW(8, 1, 8);
+  if (bs.B <= 16) KNB_SW(16, 1, 8);
+  if (bs.B <= 32) KNB_SWU(1);
+  if (bs.B <= 64) KNB_SWU(2);
+  if (bs.B <= 128) KNB_SWU(4);
+  KNB_SWU(8);
 #undef KNB_SWU
 #undef KNB_SW
 }
@@ -632,13 +755,9 @@ static int batch_sweep_vw(int vw, int u, const OpView<MT>& op, const DevBuf<RowR
 // state (without the finish, so nothing but buffers the first real sweep
 // rewrites is touched) and returns the fastest.
 template <class VT, class MT>
-static int tune_arcs_in_flight(int vw, const OpView<MT>& op, const DevBuf<RowRange>& ranges,
-                               uint32_t nranges, const DevBuf<Chunk>& chunks, uint32_t nchunks,
-                               const DevBuf<uint32_t>& lrow, const DevBuf<uint32_t>& lfirst,
-                               uint32_t nlong, const BatchScalars& bs, ColState* cs,
-                               const VT* Yold, VT* Ynew, const VT* Zold, VT* Znew,
-                               const VT* inv_out, const PersView& P, VT* scratch, double* part,
-                               int32_t* all_frozen, unsigned grid, cudaStream_t s) {
+static int tune_arcs_in_flight(const OpView<MT>& op, const SweepPlan& sp, const BatchScalars& bs,
+                               ColState* cs, const VT* Yold, VT* Ynew, const VT* Zold, VT* Znew,
+                               const VT* inv_out, const PersView& P, VT* scratch, cudaStream_t s) {
   cudaEvent_t e0, e1;
   KNB_CUDA(cudaEventCreate(&e0));
   KNB_CUDA(cudaEventCreate(&e1));
@@ -646,9 +765,8 @@ static int tune_arcs_in_flight(int vw, const OpView<MT>& op, const DevBuf<RowRan
   float best_ms = 0;
   for (int u : U_CANDIDATES) {
     KNB_CUDA(cudaEventRecord(e0, s));
-    batch_sweep_vw<VT, MT>(vw, u, op, ranges, nranges, chunks, nchunks, lrow, lfirst, nlong, bs,
-                           cs, Yold, Ynew, Zold, Znew, inv_out, P, scratch, part, all_frozen, grid,
-                           s, false);
+    batch_sweep_vw<VT, MT>(u, op, sp, bs, cs, Yold, Ynew, Zold, Znew, inv_out, P, RefineBufs{},
+                           scratch, 1, s, false);
     KNB_CUDA(cudaEventRecord(e1, s));
     KNB_CUDA(cudaEventSynchronize(e1));
     float ms = 0;
@@ -686,6 +804,8 @@ struct BatchWorkspace : Workspace {
   DevBuf<float> Y32[2], Z32[2], sc32;
   DevBuf<ColState> cs;
   DevBuf<int32_t> flags, all_frozen;
+  DevBuf<double> tot, pparts;
+  DevBuf<uint32_t> maps;  // cmap, inv and the columns selected, 256 each
 };
 
 template <class T>
@@ -734,12 +854,7 @@ void pagerank_batch(GraphHandleImpl& g, const BatchParams& prm, const double* pe
     KNB_CUDA(cudaStreamSynchronize(s));
     ws.planned = true;
   }
-  const DevBuf<RowRange>& d_ranges = ws.d_ranges;
-  const DevBuf<Chunk>& d_chunks = ws.d_chunks;
-  const DevBuf<uint32_t>& d_lrow = ws.d_lrow;
-  const DevBuf<uint32_t>& d_lfirst = ws.d_lfirst;
-  const uint32_t nranges = ws.nranges, nchunks = ws.nchunks, nlong = ws.nlong;
-  const unsigned grid = 148 * 4;
+  const uint32_t nchunks = ws.nchunks;
 
   cudaEvent_t t0, t1, l0, l1;
   KNB_CUDA(cudaEventCreate(&t0));
@@ -772,7 +887,6 @@ void pagerank_batch(GraphHandleImpl& g, const BatchParams& prm, const double* pe
     outp = ws.dout.get();
   }
   std::vector<int32_t> col_iters(Btot, 0);
-  std::vector<uint8_t> col_conv(Btot, 0);
   // column groups of at most 256
   for (uint32_t c0 = 0; c0 < Btot; c0 += 256) {
     const uint32_t B = std::min<uint32_t>(256, Btot - c0);
@@ -787,8 +901,10 @@ void pagerank_batch(GraphHandleImpl& g, const BatchParams& prm, const double* pe
     grow(prow, (size_t)n + 1);
     grow(flags, 2);
     KNB_CUDA(cudaMemsetAsync(flags.get(), 0, 8, s));
-    pers_columns<<<grid_for(B, BW, 1184), BT, 0, s>>>(pin.get() + (size_t)c0 * n, n, B, nullptr,
-                                                      flags.get(), sums.get());
+    grow(ws.pparts, (size_t)PERS_CTAS * 256);
+    pers_columns<<<dim3(PERS_CTAS, B), BT, 0, s>>>(pin.get() + (size_t)c0 * n, n, ws.pparts.get(),
+                                                   flags.get());
+    pers_sums<<<(B + BW - 1) / BW, BT, 0, s>>>(ws.pparts.get(), B, sums.get(), flags.get());
     int32_t hf[2];
     KNB_CUDA(cudaMemcpyAsync(hf, flags.get(), 8, cudaMemcpyDeviceToHost, s));
     KNB_CUDA(cudaStreamSynchronize(s));
@@ -815,192 +931,226 @@ void pagerank_batch(GraphHandleImpl& g, const BatchParams& prm, const double* pe
     }
     KNB_LAUNCH("teleport columns");
     launches += 4;
-    BatchScalars bs{prm.damping, 1.0 / n, n, B, prm.dangling == 1 ? 1 : 0, 0.0, 0, 0};
-    DevBuf<ColState>& cs = ws.cs;
-    DevBuf<int32_t>& all_frozen = ws.all_frozen;
-    DevBuf<double>& part = ws.part;
-    grow(cs, B);
-    grow(all_frozen, 1);
-    grow(part, std::max<size_t>((size_t)2 * grid * 3 * B, (size_t)1184 * 2 * B));
+    constexpr unsigned MAX_PARTS = 2 * 148 * 8;  // two grids of narrow sweeps
+    grow(ws.cs, 256);
+    grow(ws.all_frozen, 2);
+    grow(ws.maps, 3 * 256);
+    grow(ws.tot, 3 * 256);
+    grow(ws.part, std::max<size_t>((size_t)MAX_PARTS * 3 * 16,
+                                   std::max<size_t>((size_t)MAX_PARTS / 2 * 3 * B,
+                                                    (size_t)1184 * 2 * B)));
+    uint32_t* const cmap = ws.maps.get();
+    uint32_t* const inv = cmap + 256;
+    uint32_t* const sel = inv + 256;
+    ColState* const cs = ws.cs.get();
+    double* const part = ws.part.get();
+    const SweepPlan sp{ws.d_ranges.get(), ws.d_chunks.get(), ws.d_lrow.get(), ws.d_lfirst.get(),
+                       ws.nranges, ws.nchunks, ws.nlong, part, ws.tot.get(), ws.all_frozen.get()};
+    BatchScalars bs{prm.damping, 1.0 / n, n, B, B, prm.dangling == 1 ? 1 : 0, 0.0,
+                    (int32_t)std::min<int64_t>(prm.max_iter, INT32_MAX), cmap, inv};
     const double dterm0 = (double)op.n_dangling / (double)n;
-    int64_t done32 = 0;
     const size_t nb = (size_t)n * B;
-    DevBuf<float>(&Y32)[2] = ws.Y32;
-    DevBuf<float>(&Z32)[2] = ws.Z32;
-    DevBuf<float>& sc32 = ws.sc32;
-    DevBuf<double>(&Y64)[2] = ws.Y64;
-    DevBuf<double>(&Z64)[2] = ws.Z64;
-    DevBuf<double>& sc64 = ws.sc64;
-    if (mixed) {
-      for (int k = 0; k < 2; ++k) {
-        grow(Y32[k], nb);
-        grow(Z32[k], nb);
+    float* Y32[2] = {nullptr, nullptr};
+    float* Z32[2] = {nullptr, nullptr};
+    double* Y64[2];
+    double* Z64[2];
+    for (int k = 0; k < 2; ++k) {
+      if (mixed) {
+        grow(ws.Y32[k], nb);
+        grow(ws.Z32[k], nb);
+        Y32[k] = ws.Y32[k].get();
+        Z32[k] = ws.Z32[k].get();
       }
-      grow(sc32, std::max<size_t>((size_t)nchunks * B, 1));
-      spmm_init<float><<<grid_for(nb, 256), 256, 0, s>>>(Y32[0].get(), Z32[0].get(),
-                                                          op.inv_out32.get(), n, B, nullptr);
-      spmm_set_state<<<1, 256, 0, s>>>(cs.get(), B, dterm0, 0);
-      KNB_CUDA(cudaMemsetAsync(all_frozen.get(), 0, 4, s));
+      grow(ws.Y64[k], nb);
+      grow(ws.Z64[k], nb);
+      Y64[k] = ws.Y64[k].get();
+      Z64[k] = ws.Z64[k].get();
+    }
+    grow(ws.sc64, std::max<size_t>((size_t)nchunks * B, 1));
+    if (mixed) grow(ws.sc32, std::max<size_t>((size_t)nchunks * B, 1));
+    float* const sc32 = ws.sc32.get();
+    double* const sc64 = ws.sc64.get();
+
+    // The sweep's columns, by their number in the batch; all of them at the
+    // start of a phase.
+    std::vector<uint32_t> cols;
+    auto set_columns = [&](std::vector<uint32_t> c) {
+      cols = std::move(c);
+      std::vector<uint32_t> m(512, NO_COL);
+      for (uint32_t k = 0; k < cols.size(); ++k) {
+        m[k] = cols[k];
+        m[256 + cols[k]] = k;
+      }
+      KNB_CUDA(cudaMemcpyAsync(cmap, m.data(), m.size() * 4, cudaMemcpyHostToDevice, s));
+      bs.B = (uint32_t)cols.size();
+    };
+    auto all_columns = [&] {
+      std::vector<uint32_t> c(B);
+      for (uint32_t k = 0; k < B; ++k) c[k] = k;
+      set_columns(std::move(c));
+    };
+    auto select = [&](const std::vector<uint32_t>& k) {
+      KNB_CUDA(cudaMemcpyAsync(sel, k.data(), k.size() * 4, cudaMemcpyHostToDevice, s));
+      return (uint32_t)k.size();
+    };
+    // Runs sweeps (from, to = buffer indices) until every column has stopped.
+    // Every 4 sweeps the host looks at the columns' states; once a quarter of
+    // the width has stopped, the stopped columns leave (leave(count): sel's
+    // columns, in their last buffers) and the others are packed, which costs
+    // about as much as half a sweep. Returns the sweeps run.
+    auto run = [&](int cur, int64_t k, auto sweep, auto leave, auto Y, auto Z) -> int64_t {
+      std::vector<ColState> h;
+      for (;;) {
+        sweep(cur, 1 - cur);
+        cur = 1 - cur;
+        ++k;
+        if (k % 4 != 0) continue;
+        h.resize(bs.B);
+        KNB_CUDA(cudaMemcpyAsync(h.data(), cs, bs.B * sizeof(ColState), cudaMemcpyDeviceToHost, s));
+        KNB_CUDA(cudaStreamSynchronize(s));
+        std::vector<uint32_t> gone, left, names;
+        for (uint32_t c = 0; c < bs.B; ++c) (h[c].frozen ? gone : left).push_back(c);
+        if (!left.empty() && left.size() * 4 > (size_t)bs.B * 3) continue;
+        for (uint32_t c : gone) {
+          if (!h[c].converged)
+            throw Error("PageRank did not converge to tolerance " + std::to_string(prm.tol) +
+                        " within " + std::to_string(prm.max_iter) + " iterations");
+          col_iters[c0 + cols[c]] += h[c].iter;
+        }
+        if (!gone.empty()) launches += leave(select(gone));
+        if (left.empty()) return k;
+        const uint32_t count = select(left);
+        spmm_pack<<<grid_for((uint64_t)n * count, 256), 256, 0, s>>>(
+            Y[cur], Z[cur], n, bs.B, sel, count, Y[1 - cur], Z[1 - cur]);
+        KNB_LAUNCH("spmm_pack");
+        ++launches;
+        cur = 1 - cur;
+        std::vector<ColState> hs;
+        for (uint32_t c : left) {
+          names.push_back(cols[c]);
+          hs.push_back(h[c]);
+        }
+        set_columns(std::move(names));
+        KNB_CUDA(cudaMemcpyAsync(cs, hs.data(), hs.size() * sizeof(ColState),
+                                 cudaMemcpyHostToDevice, s));
+      }
+    };
+    all_columns();
+    KNB_CUDA(cudaMemsetAsync(ws.all_frozen.get(), 0, 8, s));
+    int u32 = 4;
+    if (mixed) {
+      spmm_init<float><<<grid_for(nb, 256), 256, 0, s>>>(Y32[0], Z32[0], op.inv_out32.get(), n, B);
+      spmm_set_state<<<1, 256, 0, s>>>(cs, B, dterm0);
       bs.tol = std::max(prm.tol * prm.switch_factor, prm.switch_floor);
-      bs.max_iter = (int32_t)prm.max_iter;
       launches += 2;
-      int u32 = tuned_u(vw * 4 + 0);
-      if (!u32) {
-        u32 = tune_arcs_in_flight<float, float>(
-            vw, op.view32(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong, bs,
-            cs.get(), Y32[0].get(), Y32[1].get(), Z32[0].get(), Z32[1].get(), op.inv_out32.get(),
-            P, sc32.get(), part.get(), all_frozen.get(), grid, s);
+      if (B > 16 && !(u32 = tuned_u(vw * 4 + 0))) {
+        u32 = tune_arcs_in_flight<float, float>(op.view32(), sp, bs, cs, Y32[0], Y32[1], Z32[0],
+                                                Z32[1], op.inv_out32.get(), P, sc32, s);
         keep_u(vw * 4 + 0, u32);
       }
-      int k = 0;
       KNB_CUDA(cudaEventRecord(l0, s));
-      for (;;) {
-        const int b = k & 1;
-        launches += batch_sweep_vw<float, float>(
-            vw, u32, op.view32(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong,
-            bs, cs.get(), Y32[b].get(), Y32[1 - b].get(), Z32[b].get(), Z32[1 - b].get(),
-            op.inv_out32.get(), P, sc32.get(), part.get(), all_frozen.get(), grid, s);
-        ++k;
-        if (k % 4 == 0) {
-          int32_t af = 0;
-          KNB_CUDA(cudaMemcpyAsync(&af, all_frozen.get(), 4, cudaMemcpyDeviceToHost, s));
-          KNB_CUDA(cudaStreamSynchronize(s));
-          if (af) break;
-        }
-      }
+      sweeps32 += run(
+          0, 0,
+          [&](int a, int b) {
+            launches += batch_sweep_vw<float, float>(u32, op.view32(), sp, bs, cs, Y32[a], Y32[b],
+                                                     Z32[a], Z32[b], op.inv_out32.get(), P,
+                                                     RefineBufs{}, sc32, b, s);
+          },
+          [&](uint32_t count) {
+            spmm_switch<<<grid_for((uint64_t)n * count, 256), 256, 0, s>>>(
+                Y32[0], Y32[1], cs, sel, count, cmap, bs.B, B, Y64[0], Z64[0],
+                op.inv_out64.get(), n);
+            KNB_LAUNCH("batch hand-over");
+            return 1;
+          },
+          Y32, Z32);
       loop_end();
-      // every column's FP32 phase ended; hand over from its own buffer
-      std::vector<ColState> h(B);
-      KNB_CUDA(cudaMemcpyAsync(h.data(), cs.get(), B * sizeof(ColState), cudaMemcpyDeviceToHost, s));
-      KNB_CUDA(cudaStreamSynchronize(s));
-      for (uint32_t c = 0; c < B; ++c) {
-        if (!h[c].converged)
-          throw Error("PageRank did not converge to tolerance " + std::to_string(prm.tol) +
-                      " within " + std::to_string(prm.max_iter) + " iterations");
-        done32 = std::max<int64_t>(done32, h[c].iter);
-      }
-      sweeps32 += k;
-      // columns stopped at different sweeps: each is read from its own buffer
-      for (int kk = 0; kk < 2; ++kk) {
-        grow(Y64[kk], nb);
-        grow(Z64[kk], nb);
-      }
-      spmm_switch<<<grid_for(nb, 256), 256, 0, s>>>(Y32[0].get(), Y32[1].get(), cs.get(),
-                                                    Y64[0].get(), Z64[0].get(),
-                                                    op.inv_out64.get(), n, B);
-      column_sums_part<<<1184, 256, 0, s>>>(Y64[0].get(), op.inv_out64.get(), n, B, part.get());
-      column_sums_finish<<<1, 256, 0, s>>>(part.get(), 1184, B, cs.get());
+      for (uint32_t c = 0; c < B; ++c) colits32 += col_iters[c0 + c];
+      all_columns();
+      column_sums_part<<<1184, 256, 0, s>>>(Y64[0], op.inv_out64.get(), n, B, part);
+      sum_parts<<<(2 * B + 31) / 32, SP_T, 0, s>>>(part, 1184, 2 * B, ws.tot.get());
+      column_sums_finish<<<1, 256, 0, s>>>(ws.tot.get(), B, cs);
       KNB_LAUNCH("batch hand-over");
       launches += 3;
-      for (uint32_t c = 0; c < B; ++c) {
-        col_iters[c0 + c] = h[c].iter;
-        colits32 += h[c].iter;
-      }
     } else {
-      for (int kk = 0; kk < 2; ++kk) {
-        grow(Y64[kk], nb);
-        grow(Z64[kk], nb);
-      }
-      spmm_init<double><<<grid_for(nb, 256), 256, 0, s>>>(Y64[0].get(), Z64[0].get(),
-                                                           op.inv_out64.get(), n, B, nullptr);
-      spmm_set_state<<<1, 256, 0, s>>>(cs.get(), B, dterm0, 0);
+      spmm_init<double><<<grid_for(nb, 256), 256, 0, s>>>(Y64[0], Z64[0], op.inv_out64.get(), n,
+                                                           B);
+      spmm_set_state<<<1, 256, 0, s>>>(cs, B, dterm0);
       launches += 2;
     }
     // FP64 phase
-    KNB_CUDA(cudaMemsetAsync(all_frozen.get(), 0, 4, s));
+    KNB_CUDA(cudaMemsetAsync(ws.all_frozen.get(), 0, 8, s));
     bs.tol = prm.tol;
-    bs.max_iter = (int32_t)(prm.max_iter - (mixed ? 0 : 0));
-    grow(sc64, std::max<size_t>((size_t)nchunks * B, 1));
     const bool use32v = op.has_vals && op.vals32_exact;
     const int key64 = vw * 4 + (use32v ? 1 : 2);
-    int u64 = tuned_u(key64);
-    if (!u64) {
-      u64 = use32v
-                ? tune_arcs_in_flight<double, float>(
-                      vw, op.view32(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst,
-                      nlong, bs, cs.get(), Y64[0].get(), Y64[1].get(), Z64[0].get(), Z64[1].get(),
-                      op.inv_out64.get(), P, sc64.get(), part.get(), all_frozen.get(), grid, s)
-                : tune_arcs_in_flight<double, double>(
-                      vw, op.view64(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst,
-                      nlong, bs, cs.get(), Y64[0].get(), Y64[1].get(), Z64[0].get(), Z64[1].get(),
-                      op.inv_out64.get(), P, sc64.get(), part.get(), all_frozen.get(), grid, s);
+    int u64 = 4;
+    if (B > 16 && !(u64 = tuned_u(key64))) {
+      u64 = use32v ? tune_arcs_in_flight<double, float>(op.view32(), sp, bs, cs, Y64[0], Y64[1],
+                                                        Z64[0], Z64[1], op.inv_out64.get(), P,
+                                                        sc64, s)
+                   : tune_arcs_in_flight<double, double>(op.view64(), sp, bs, cs, Y64[0], Y64[1],
+                                                         Z64[0], Z64[1], op.inv_out64.get(), P,
+                                                         sc64, s);
       keep_u(key64, u64);
     }
-    int k = 0;
-    KNB_CUDA(cudaEventRecord(l0, s));
-    auto all_done = [&] {
-      int32_t af = 0;
-      KNB_CUDA(cudaMemcpyAsync(&af, all_frozen.get(), 4, cudaMemcpyDeviceToHost, s));
-      KNB_CUDA(cudaStreamSynchronize(s));
-      return af != 0;
+    auto out_grid = [&](uint32_t count) {
+      return dim3(std::min<uint32_t>((n + 31) / 32, 148 * 16), (count + 31) / 32);
     };
+    double* const outc = outp + (size_t)c0 * n;
+    KNB_CUDA(cudaEventRecord(l0, s));
     if (refine) {
       // the anchor sweep: FP64 gathers of z_ref = Y64[0] / out; s_ref into
       // Y64[1], the correction e and z_e into Y32[1] and Z32[1]
-      const RefineBufs rb0{Y64[0].get(), Y64[1].get(), nullptr, Y32[1].get(), Z32[1].get(),
-                           op.inv_out32.get()};
+      const RefineBufs rb0{Y64[0], Y64[1], nullptr, Y32[1], Z32[1], op.inv_out32.get()};
       if (use32v)
         launches += batch_sweep_vw<double, float, EPI_ANCHOR>(
-            vw, u64, op.view32(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong,
-            bs, cs.get(), Y64[0].get(), Y64[1].get(), Z64[0].get(), Z64[1].get(),
-            op.inv_out64.get(), P, sc64.get(), part.get(), all_frozen.get(), grid, s, true, rb0);
+            u64, op.view32(), sp, bs, cs, Y64[0], Y64[1], Z64[0], Z64[1], op.inv_out64.get(), P,
+            rb0, sc64, 1, s);
       else
         launches += batch_sweep_vw<double, double, EPI_ANCHOR>(
-            vw, u64, op.view64(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong,
-            bs, cs.get(), Y64[0].get(), Y64[1].get(), Z64[0].get(), Z64[1].get(),
-            op.inv_out64.get(), P, sc64.get(), part.get(), all_frozen.get(), grid, s, true, rb0);
-      k = 1;
+            u64, op.view64(), sp, bs, cs, Y64[0], Y64[1], Z64[0], Z64[1], op.inv_out64.get(), P,
+            rb0, sc64, 1, s);
       // refinement sweeps: FP32 gathers of z_e, FP32 arc values (the FP32
       // phase's arcs in flight)
-      int ur = tuned_u(vw * 4 + 0);
-      if (!ur) ur = 4;
-      for (;;) {
-        const int b = k & 1;
-        const RefineBufs rb{Y64[0].get(), Y64[1].get(), Y32[b].get(), Y32[1 - b].get(),
-                            Z32[1 - b].get(), op.inv_out32.get()};
-        launches += batch_sweep_vw<float, float, EPI_REFINE>(
-            vw, ur, op.view32(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong,
-            bs, cs.get(), Y32[b].get(), Y32[1 - b].get(), Z32[b].get(), Z32[1 - b].get(),
-            op.inv_out32.get(), P, sc32.get(), part.get(), all_frozen.get(), grid, s, true, rb);
-        ++k;
-        if (k % 4 == 0 && all_done()) break;
-      }
+      sweeps64 += run(
+          1, 1,
+          [&](int a, int b) {
+            const RefineBufs rb{Y64[0], Y64[1], Y32[a], Y32[b], Z32[b], op.inv_out32.get()};
+            launches += batch_sweep_vw<float, float, EPI_REFINE>(
+                u32, op.view32(), sp, bs, cs, Y32[a], Y32[b], Z32[a], Z32[b], op.inv_out32.get(),
+                P, rb, sc32, b, s);
+          },
+          [&](uint32_t count) {
+            spmm_output<float><<<out_grid(count), 256, 0, s>>>(Y32[0], Y32[1], Y64[0], cs, sel,
+                                                               count, cmap, bs.B, B, n, outc);
+            KNB_LAUNCH("spmm_output");
+            return 1;
+          },
+          Y32, Z32);
     } else {
-      for (;;) {
-        const int b = k & 1;
-        if (use32v)
-          launches += batch_sweep_vw<double, float>(
-              vw, u64, op.view32(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong,
-              bs, cs.get(), Y64[b].get(), Y64[1 - b].get(), Z64[b].get(), Z64[1 - b].get(),
-              op.inv_out64.get(), P, sc64.get(), part.get(), all_frozen.get(), grid, s);
-        else
-          launches += batch_sweep_vw<double, double>(
-              vw, u64, op.view64(), d_ranges, nranges, d_chunks, nchunks, d_lrow, d_lfirst, nlong,
-              bs, cs.get(), Y64[b].get(), Y64[1 - b].get(), Z64[b].get(), Z64[1 - b].get(),
-              op.inv_out64.get(), P, sc64.get(), part.get(), all_frozen.get(), grid, s);
-        ++k;
-        if (k % 4 == 0 && all_done()) break;
-      }
+      sweeps64 += run(
+          0, 0,
+          [&](int a, int b) {
+            if (use32v)
+              launches += batch_sweep_vw<double, float>(u64, op.view32(), sp, bs, cs, Y64[a],
+                                                        Y64[b], Z64[a], Z64[b],
+                                                        op.inv_out64.get(), P, RefineBufs{}, sc64,
+                                                        b, s);
+            else
+              launches += batch_sweep_vw<double, double>(u64, op.view64(), sp, bs, cs, Y64[a],
+                                                         Y64[b], Z64[a], Z64[b],
+                                                         op.inv_out64.get(), P, RefineBufs{},
+                                                         sc64, b, s);
+          },
+          [&](uint32_t count) {
+            spmm_output<double><<<out_grid(count), 256, 0, s>>>(Y64[0], Y64[1], nullptr, cs, sel,
+                                                                count, cmap, bs.B, B, n, outc);
+            KNB_LAUNCH("spmm_output");
+            return 1;
+          },
+          Y64, Z64);
     }
     loop_end();
-    sweeps64 += k;
-    std::vector<ColState> h(B);
-    KNB_CUDA(cudaMemcpyAsync(h.data(), cs.get(), B * sizeof(ColState), cudaMemcpyDeviceToHost, s));
-    KNB_CUDA(cudaStreamSynchronize(s));
-    for (uint32_t c = 0; c < B; ++c) {
-      if (!h[c].converged)
-        throw Error("PageRank did not converge to tolerance " + std::to_string(prm.tol) +
-                    " within " + std::to_string(prm.max_iter) + " iterations");
-      col_iters[c0 + c] += h[c].iter;
-      col_conv[c0 + c] = 1;
-    }
-    if (refine)
-      spmm_output_ref<<<grid_for(nb, 256), 256, 0, s>>>(Y64[0].get(), Y32[0].get(), Y32[1].get(),
-                                                        cs.get(), n, B, outp + (size_t)c0 * n);
-    else
-      spmm_output<double><<<grid_for(nb, 256), 256, 0, s>>>(Y64[0].get(), Y64[1].get(), cs.get(),
-                                                            n, B, outp + (size_t)c0 * n);
-    ++launches;
   }
   if (!prm.on_device)
     KNB_CUDA(cudaMemcpyAsync(out_colmajor, outp, (size_t)n * Btot * 8, cudaMemcpyDeviceToHost, s));
