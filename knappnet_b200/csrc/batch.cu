@@ -28,7 +28,9 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 #include <vector>
 
@@ -41,7 +43,12 @@ constexpr int BT = 256;          // threads per CTA
 constexpr int BW = BT / 32;      // warps per CTA
 constexpr int MAXVW = 8;         // columns per lane (B <= 256 per launch)
 constexpr uint32_t LONG_ROW = 512;
-constexpr uint32_t RANGE_ARCS = 256;
+// A warp's share of rows: an arc costs one gathered iterate row, a row about
+// ROW_COST of them (its iterates read and written, and a chain of waits). With
+// 256 per range and rows at 1 a third of the sweep's time went by with SMs
+// idle: ranges of empty rows took longest.
+constexpr uint32_t RANGE_ARCS = 128;
+constexpr uint32_t ROW_COST = 6;
 
 struct RowRange {
   uint32_t lo, hi;
@@ -93,23 +100,24 @@ struct PersView {
   const double* vals;
 };
 
-// Row sum of one row of A times Z for this lane's columns. U arcs at a
-// time: their indices, then all their gathers, then the products added in
-// arc order (so each column's sum keeps the order of a one-arc loop).
-template <class VT, class MT, int VW, int U>
+// Row sum of arcs [a0, a1) of A times Z for this lane's columns, taking every
+// P-th arc from a0. U arcs at a time: their indices, then all their gathers,
+// then the products added in arc order (so each sum keeps the order of a
+// one-arc loop).
+template <class VT, class MT, int VW, int U, int P>
 __device__ __forceinline__ void row_product(const OpView<MT>& op, const VT* __restrict__ Z,
                                             uint32_t B, uint32_t a0, uint32_t a1, int lane,
                                             VT (&acc)[VW]) {
 #pragma unroll
   for (int v = 0; v < VW; ++v) acc[v] = VT(0);
   uint32_t k = a0;
-  for (; k + U <= a1; k += U) {
+  for (; k + (U - 1) * P < a1; k += U * P) {
     uint32_t j[U];
     VT w[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      j[u] = __ldg(op.cols + k + u);
-      w[u] = op.vals ? (VT)__ldg(op.vals + k + u) : VT(1);
+      j[u] = __ldg(op.cols + k + u * P);
+      w[u] = op.vals ? (VT)__ldg(op.vals + k + u * P) : VT(1);
     }
     VT z[U][VW];
 #pragma unroll
@@ -127,7 +135,7 @@ __device__ __forceinline__ void row_product(const OpView<MT>& op, const VT* __re
       for (int v = 0; v < VW; ++v)
         if (lane + 32 * v < B) acc[v] += w[u] * z[u][v];
   }
-  for (; k < a1; ++k) {
+  for (; k < a1; k += P) {
     const uint32_t j = __ldg(op.cols + k);
     const VT w = op.vals ? (VT)__ldg(op.vals + k) : VT(1);
     const VT* zr = Z + (size_t)j * B;
@@ -157,61 +165,82 @@ struct RefineBufs {
   const float* io32;   // 1 / out in FP32 (0 for dangling nodes)
 };
 
+// What row i's update reads besides the product, loaded before the product so
+// that the waits overlap (the FP64 arrays of the refinement after it: with
+// them the sweep needs 80 registers, a CTA per SM less).
+template <class VT, int VW>
+struct RowIn {
+  VT yo[VW];         // plain: the old iterate; refinement: e of the old iterate
+  VT io;
+  uint32_t e0, e1;   // the row's sparse teleport entries
+};
+
+template <class VT, int VW, int MODE>
+__device__ __forceinline__ RowIn<VT, VW> row_fetch(uint32_t i, int lane,
+                                                         const BatchScalars& bs,
+                                                         const VT* __restrict__ Yold,
+                                                         const VT* __restrict__ inv_out,
+                                                         const PersView& pv,
+                                                         const RefineBufs& rb) {
+  RowIn<VT, VW> in;
+  in.e0 = in.e1 = 0;
+  if (!pv.dense) {
+    in.e0 = pv.rowptr[i];
+    in.e1 = pv.rowptr[i + 1];
+  }
+  in.io = MODE == EPI_PLAIN ? inv_out[i] : (VT)rb.io32[i];
+#pragma unroll
+  for (int v = 0; v < VW; ++v) {
+    const uint32_t c = lane + 32 * v;
+    in.yo[v] = VT(0);
+    if (c >= bs.B) continue;
+    if constexpr (MODE == EPI_PLAIN) in.yo[v] = Yold[(size_t)i * bs.B + c];
+    if constexpr (MODE == EPI_REFINE) in.yo[v] = (VT)rb.eold[(size_t)i * bs.B + c];
+  }
+  return in;
+}
+
 // The PageRank update of row i for this lane's columns, and its per-column
-// sums (mass, dangling mass, L1 change) into the warp's slice red[3][B] of
-// shared memory (column c belongs to lane c mod 32, so every slot has one
-// writer and takes its rows in order).
+// sums (mass, dangling mass, L1 change) into the group's slice red[3][B] of
+// shared memory (every slot has one writer, which takes its rows in order).
 template <class VT, int VW, int MODE>
 __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int lane,
                                            const BatchScalars& bs, const ColState* cs,
-                                           const VT* __restrict__ Yold, VT* __restrict__ Ynew,
-                                           VT* __restrict__ Znew, const VT* __restrict__ inv_out,
-                                           const PersView& pv, const RefineBufs& rb,
-                                           double* red) {
+                                           const RowIn<VT, VW>& in, VT* __restrict__ Ynew,
+                                           VT* __restrict__ Znew, const PersView& pv,
+                                           const RefineBufs& rb, double* red) {
   using PT = std::conditional_t<MODE == EPI_PLAIN, VT, double>;
   PT psp[VW];  // this lane's teleport values of row i (sparse teleport)
 #pragma unroll
   for (int v = 0; v < VW; ++v) psp[v] = PT(0);
-  if (!pv.dense) {
-    for (uint32_t e = pv.rowptr[i]; e < pv.rowptr[i + 1]; ++e) {
-      const uint32_t c = __ldg(bs.inv + pv.cols[e]);
-      if (c == NO_COL || (c & 31u) != (uint32_t)lane) continue;
-      const PT x = (PT)pv.vals[e];
+  for (uint32_t e = in.e0; e < in.e1; ++e) {
+    const uint32_t c = __ldg(bs.inv + pv.cols[e]);
+    if (c == NO_COL || (c & 31u) != (uint32_t)lane) continue;
+    const PT x = (PT)pv.vals[e];
 #pragma unroll
-      for (int v = 0; v < VW; ++v)
-        if ((c >> 5) == (uint32_t)v) psp[v] = x;
-    }
+    for (int v = 0; v < VW; ++v)
+      if ((c >> 5) == (uint32_t)v) psp[v] = x;
   }
-  if constexpr (MODE == EPI_PLAIN) {
-    const VT io = inv_out[i];
 #pragma unroll
-    for (int v = 0; v < VW; ++v) {
-      const uint32_t c = lane + 32 * v;
-      if (c >= bs.B || cs[c].frozen) continue;
+  for (int v = 0; v < VW; ++v) {
+    const uint32_t c = lane + 32 * v;
+    if (c >= bs.B || cs[c].frozen) continue;
+    const size_t q = (size_t)i * bs.B + c;
+    if constexpr (MODE == EPI_PLAIN) {
+      const VT io = in.io;
       const VT it = (VT)cs[c].inv_total, dt = (VT)cs[c].dterm;
-      const size_t q = (size_t)i * bs.B + c;
       const VT pg = pv.dense ? (VT)pv.dense[(size_t)i * bs.Bo + __ldg(bs.cmap + c)] : psp[v];
       const VT jg = bs.jump_uniform ? (VT)bs.pu : pg;
       const VT u = (VT)bs.d * (s[v] * it + dt * jg) + (VT)(1.0 - bs.d) * pg;
-      const VT xo = Yold[q] * it;
+      const VT xo = in.yo[v] * it;
       Ynew[q] = u;
       Znew[q] = u * io;
       red[c] += (double)u;
       if (io == VT(0)) red[bs.B + c] += (double)u;
       red[2 * bs.B + c] += fabs((double)u - (double)xo);
-    }
-  } else {
-    (void)Yold;
-    (void)Ynew;
-    (void)Znew;
-    (void)inv_out;
-    const float io = rb.io32[i];
-#pragma unroll
-    for (int v = 0; v < VW; ++v) {
-      const uint32_t c = lane + 32 * v;
-      if (c >= bs.B || cs[c].frozen) continue;
+    } else {
+      const float io = (float)in.io;
       const double it = cs[c].inv_total, dt = cs[c].dterm;
-      const size_t q = (size_t)i * bs.B + c;
       const size_t r = (size_t)i * bs.Bo + __ldg(bs.cmap + c);
       double sum;
       if constexpr (MODE == EPI_ANCHOR) {
@@ -224,7 +253,7 @@ __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int la
       const double jg = bs.jump_uniform ? bs.pu : pg;
       const double u = bs.d * (sum * it + dt * jg) + (1.0 - bs.d) * pg;
       const double yr = rb.yref[r];
-      const double yo = MODE == EPI_ANCHOR ? yr : yr + (double)rb.eold[q];
+      const double yo = MODE == EPI_ANCHOR ? yr : yr + (double)in.yo[v];
       const float en = (float)(u - yr);
       const double us = yr + (double)en;  // the iterate as stored
       rb.enew[q] = en;
@@ -236,17 +265,35 @@ __device__ __forceinline__ void row_update(uint32_t i, const VT (&s)[VW], int la
   }
 }
 
-// Lanes per row: a whole warp for more than 16 columns (lane l holds columns
-// l, l + 32, ...); up to 16 columns W lanes, the power of two that holds them,
-// so a warp takes 32 / W rows at once.
+// Lanes of a row: a whole warp for more than 16 columns (lane l holds columns
+// l, l + 32, ...). Up to 16 columns W lanes hold them, the power of two that
+// does, and a row takes S = max(W, 8) lanes, which share its arcs out by
+// S / W: a warp then has 32 / S rows under way, and a row of 512 arcs does not
+// hold up its neighbours (one column on R-MAT 20: 200 us a sweep with one lane
+// per row, 95 us with 8).
 template <int W>
 struct Lanes {
-  static constexpr int G = 32 / W;  // rows a warp takes at once
-  int col, group;
+  static constexpr int S = W < 8 ? 8 : W;
+  static constexpr int G = 32 / S;  // rows a warp takes at once
+  static constexpr int P = S / W;   // arcs of a row under way at once
+  int col, group, arc;
   __device__ __forceinline__ Lanes() {
     const int lane = threadIdx.x & 31;
     col = lane % W;
-    group = lane / W;
+    arc = lane % S / W;
+    group = lane / S;
+  }
+  // The sum over the lanes that share a row's arcs, in a fixed order, in
+  // every one of them.
+  template <class VT, int VW>
+  __device__ __forceinline__ void join(VT (&acc)[VW]) const {
+    if constexpr (P > 1) {
+      const unsigned mask = ((1u << S) - 1u) << (group * S);
+#pragma unroll
+      for (int o = W; o < S; o <<= 1)
+#pragma unroll
+        for (int v = 0; v < VW; ++v) acc[v] += __shfl_xor_sync(mask, acc[v], o);
+    }
   }
 };
 
@@ -256,7 +303,7 @@ template <int W>
 __device__ __forceinline__ double* group_sums(double* smem, uint32_t B) {
   const Lanes<W> l;
   double* red = smem + (size_t)((threadIdx.x >> 5) * Lanes<W>::G + l.group) * 3 * B;
-  for (uint32_t q = l.col; q < 3 * B; q += W) red[q] = 0.0;
+  for (uint32_t q = l.arc * W + l.col; q < 3 * B; q += Lanes<W>::S) red[q] = 0.0;
   __syncwarp();
   return red;
 }
@@ -274,9 +321,12 @@ __device__ __forceinline__ void cta_column_sums(uint32_t B, double* __restrict__
 }
 
 // The rows of at most LONG_ROW arcs: their products and updates. Bound by the
-// gathers, one iterate row (B values) per arc.
+// gathers, one iterate row (B values) per arc: 100 columns on R-MAT 20 (6.2 GB
+// of gathers a sweep) 2.35 ms with ranges by arcs, late loads and 4 CTAs per
+// SM whatever the kernel's registers, 1.00 ms since (refinement 3.05 and
+// 1.60).
 template <class VT, class MT, int W, int VW, int U, int MODE>
-__global__ void __launch_bounds__(BT)
+__global__ void __launch_bounds__(BT, VW * sizeof(VT) <= 16 ? 4 : 2)
 spmm_rows(OpView<MT> op, const VT* __restrict__ Z, const RowRange* __restrict__ ranges,
           uint32_t nranges, BatchScalars bs, const ColState* __restrict__ cs,
           const VT* __restrict__ Yold, VT* __restrict__ Ynew, VT* __restrict__ Znew,
@@ -292,32 +342,40 @@ spmm_rows(OpView<MT> op, const VT* __restrict__ Z, const RowRange* __restrict__ 
     for (uint32_t i = rr.lo + l.group; i < rr.hi; i += Lanes<W>::G) {
       const uint32_t a0 = op.off[i], a1 = op.off[i + 1];
       if (a1 - a0 > LONG_ROW) continue;  // long rows: spmm_chunks / spmm_long
+      const auto in = row_fetch<VT, VW, MODE>(i, l.col, bs, Yold, inv_out, P, rb);
       VT acc[VW];
-      row_product<VT, MT, VW, U>(op, Z, bs.B, a0, a1, l.col, acc);
-      row_update<VT, VW, MODE>(i, acc, l.col, bs, cs, Yold, Ynew, Znew, inv_out, P, rb, red);
+      row_product<VT, MT, VW, U, Lanes<W>::P>(op, Z, bs.B, a0 + l.arc, a1, l.col, acc);
+      l.join(acc);
+      if (l.arc == 0)
+        row_update<VT, VW, MODE>(i, acc, l.col, bs, cs, in, Ynew, Znew, P, rb, red);
     }
   }
   cta_column_sums<W>(bs.B, part, smem_b);
 }
 
-// Partial products of the chunks of long rows.
+// Partial products of the chunks of long rows: a warp per chunk, whose lanes
+// share its arcs out by 32 / W.
 template <class VT, class MT, int W, int VW, int U>
 __global__ void __launch_bounds__(BT)
 spmm_chunks(OpView<MT> op, const VT* __restrict__ Z, const Chunk* __restrict__ chunks,
             uint32_t nchunks, uint32_t B, VT* __restrict__ scratch,
             const int32_t* __restrict__ all_frozen) {
   if (*all_frozen) return;
-  const Lanes<W> l;
-  const uint32_t gw = (blockIdx.x * BW + (threadIdx.x >> 5)) * Lanes<W>::G + l.group;
-  const uint32_t nw = gridDim.x * BW * Lanes<W>::G;
+  constexpr int P = 32 / W;
+  const int lane = threadIdx.x & 31, col = lane % W, arc = lane / W;
+  const uint32_t gw = blockIdx.x * BW + (threadIdx.x >> 5), nw = gridDim.x * BW;
   for (uint32_t q = gw; q < nchunks; q += nw) {
     const Chunk ch = chunks[q];
     VT acc[VW];
-    row_product<VT, MT, VW, U>(op, Z, B, ch.a0, ch.a1, l.col, acc);
+    row_product<VT, MT, VW, U, P>(op, Z, B, ch.a0 + arc, ch.a1, col, acc);
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+      for (int v = 0; v < VW; ++v) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
 #pragma unroll
     for (int v = 0; v < VW; ++v) {
-      const uint32_t c = l.col + 32 * v;
-      if (c < B) scratch[(size_t)q * B + c] = acc[v];
+      const uint32_t c = col + 32 * v;
+      if (arc == 0 && c < B) scratch[(size_t)q * B + c] = acc[v];
     }
   }
 }
@@ -337,6 +395,7 @@ spmm_long(const uint32_t* __restrict__ lrow, const uint32_t* __restrict__ lfirst
   const uint32_t gw = (blockIdx.x * BW + (threadIdx.x >> 5)) * Lanes<W>::G + l.group;
   const uint32_t nw = gridDim.x * BW * Lanes<W>::G;
   for (uint32_t q = gw; q < nlong; q += nw) {
+    const auto in = row_fetch<VT, VW, MODE>(lrow[q], l.col, bs, Yold, inv_out, P, rb);
     VT acc[VW];
 #pragma unroll
     for (int v = 0; v < VW; ++v) acc[v] = VT(0);
@@ -347,7 +406,8 @@ spmm_long(const uint32_t* __restrict__ lrow, const uint32_t* __restrict__ lfirst
         const uint32_t c = l.col + 32 * v;
         if (c < bs.B) acc[v] += scratch[(size_t)k * bs.B + c];
       }
-    row_update<VT, VW, MODE>(lrow[q], acc, l.col, bs, cs, Yold, Ynew, Znew, inv_out, P, rb, red);
+    if (l.arc == 0)
+      row_update<VT, VW, MODE>(lrow[q], acc, l.col, bs, cs, in, Ynew, Znew, P, rb, red);
   }
   cta_column_sums<W>(bs.B, part, smem_b);
 }
@@ -644,7 +704,7 @@ static BatchPlan make_plan(const std::vector<uint32_t>& off, uint32_t n) {
       for (uint32_t a = off[i]; a < off[i + 1]; a += LONG_ROW)
         p.chunks.push_back({i, a, std::min(off[i + 1], a + LONG_ROW)});
     } else {
-      acc += deg + 1;
+      acc += deg + ROW_COST;
     }
     if (acc >= RANGE_ARCS) {
       p.ranges.push_back({lo, i + 1});
@@ -674,6 +734,24 @@ struct SweepPlan {
   int32_t* flags;  // all frozen, ticket
 };
 
+// CTAs of a sweep kernel that fit on the GPU at once, at most MAX_CTAS.
+constexpr unsigned MAX_CTAS = 148 * 8;
+static unsigned resident_ctas(const void* fn, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, size_t>, unsigned> known;
+  int dev = 0;
+  KNB_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  unsigned& g = known[{dev, fn, smem}];
+  if (!g) {
+    int per_sm = 0, sms = 0;
+    KNB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, BT, smem));
+    KNB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    g = std::min(MAX_CTAS, (unsigned)std::max(1, per_sm) * (unsigned)sms);
+  }
+  return g;
+}
+
 // One sweep from buffers (Yold, Zold) to (Ynew, Znew) = buffer newbuf: the
 // row products and updates, then (finish) the per-column sums, stopping rule
 // and next sweep's scalars. Without finish the sweep only rewrites Ynew, Znew,
@@ -683,9 +761,6 @@ static int batch_sweep(const OpView<MT>& op, const SweepPlan& sp, const BatchSca
                        ColState* cs, const VT* Yold, VT* Ynew, const VT* Zold, VT* Znew,
                        const VT* inv_out, const PersView& P, const RefineBufs& rb, VT* scratch,
                        int newbuf, bool finish, cudaStream_t s) {
-  // 32 resident warps per SM with whole-warp rows (their sums take 3 B doubles
-  // of shared memory a warp), 64 with narrow ones
-  const unsigned grid = W == 32 ? 148 * 4 : 148 * 8;
   const size_t smem = (size_t)BW * Lanes<W>::G * 3 * bs.B * sizeof(double);
   if (W == 32) {
     set_func_attr((const void*)spmm_rows<VT, MT, W, VW, U, MODE>,
@@ -695,9 +770,11 @@ static int batch_sweep(const OpView<MT>& op, const SweepPlan& sp, const BatchSca
                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                   (int)(BW * 3 * 256 * sizeof(double)));
   }
+  // the CTAs that fit at once, at most what the partials hold
+  const unsigned grid = resident_ctas((const void*)spmm_rows<VT, MT, W, VW, U, MODE>, smem);
   int launches = 1;
   if (sp.nchunks) {
-    spmm_chunks<VT, MT, W, VW, U><<<grid, BT, 0, s>>>(op, Zold, sp.chunks, sp.nchunks, bs.B,
+    spmm_chunks<VT, MT, W, VW, U><<<148 * 8, BT, 0, s>>>(op, Zold, sp.chunks, sp.nchunks, bs.B,
                                                        scratch, sp.flags);
     ++launches;
   }
@@ -722,8 +799,8 @@ static int batch_sweep(const OpView<MT>& op, const SweepPlan& sp, const BatchSca
   return launches;
 }
 
-// u: arcs in flight per warp of a whole-warp row (1, 2 or 4; narrow rows,
-// whose lanes hold one column, keep 8).
+// u: arcs in flight per lane of a whole-warp row (1, 2 or 4; lanes of narrow
+// rows, which hold one column, keep 4).
 template <class VT, class MT, int MODE = EPI_PLAIN>
 static int batch_sweep_vw(int u, const OpView<MT>& op, const SweepPlan& sp, const BatchScalars& bs,
                           ColState* cs, const VT* Yold, VT* Ynew, const VT* Zold, VT* Znew,
@@ -738,11 +815,11 @@ static int batch_sweep_vw(int u, const OpView<MT>& op, const SweepPlan& sp, cons
     case 2: KNB_SW(32, V, 2);            \
     default: KNB_SW(32, V, 4);           \
   }
-  if (bs.B <= 1) KNB_SW(1, 1, 8);
-  if (bs.B <= 2) KNB_SW(2, 1, 8);
-  if (bs.B <= 4) KNB_SW(4, 1, 8);
-  if (bs.B <= 8) KNB_SW(8, 1, 8);
-  if (bs.B <= 16) KNB_SW(16, 1, 8);
+  if (bs.B <= 1) KNB_SW(1, 1, 4);
+  if (bs.B <= 2) KNB_SW(2, 1, 4);
+  if (bs.B <= 4) KNB_SW(4, 1, 4);
+  if (bs.B <= 8) KNB_SW(8, 1, 4);
+  if (bs.B <= 16) KNB_SW(16, 1, 4);
   if (bs.B <= 32) KNB_SWU(1);
   if (bs.B <= 64) KNB_SWU(2);
   if (bs.B <= 128) KNB_SWU(4);
@@ -931,14 +1008,11 @@ void pagerank_batch(GraphHandleImpl& g, const BatchParams& prm, const double* pe
     }
     KNB_LAUNCH("teleport columns");
     launches += 4;
-    constexpr unsigned MAX_PARTS = 2 * 148 * 8;  // two grids of narrow sweeps
     grow(ws.cs, 256);
     grow(ws.all_frozen, 2);
     grow(ws.maps, 3 * 256);
     grow(ws.tot, 3 * 256);
-    grow(ws.part, std::max<size_t>((size_t)MAX_PARTS * 3 * 16,
-                                   std::max<size_t>((size_t)MAX_PARTS / 2 * 3 * B,
-                                                    (size_t)1184 * 2 * B)));
+    grow(ws.part, (size_t)2 * MAX_CTAS * 3 * std::max<uint32_t>(B, 16));  // rows, long rows
     uint32_t* const cmap = ws.maps.get();
     uint32_t* const inv = cmap + 256;
     uint32_t* const sel = inv + 256;
