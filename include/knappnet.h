@@ -431,7 +431,7 @@ NET_API void net_set_sweep_timing(int32_t on);
  * 15 = packed graphs: graphs of at least this many nodes are each split
  * over a thread-block cluster (0, default: the larger of 4096 and the node
  * count over the launch's CTAs); 16 = packed graphs: CTAs per cluster for
- * those graphs (0 tuned with key 6 per batch, 1 none, 4, 8); 17 = FP64
+ * those graphs (0 chosen with key 6 per batch, up to 16; 1 none, 4, 8); 17 = FP64
  * PageRank (teleport vector, if any, in host memory) on at most this many
  * edges runs as one
  * packed-graph launch (default 262,144; 0 never; NetSolveInfo.sweep_kernel is

@@ -4,24 +4,39 @@
 //
 // Graphs are taken off queues largest first (so the last graphs to start are
 // the small ones) and each runs the reference's iteration on its own
-// (crates/engine/src/metrics/spectral.rs:247-280): z = x / out with the
-// dangling mass `stuck`, y = A z, y = d (y + stuck jump) + (1 - d) p, the
-// division by the total and the L1 change, every sum in a fixed order. Each
-// graph therefore gets what a separate net_pagerank call on it returns, up to
+// (crates/engine/src/metrics/spectral.rs:247-280), every sum in a fixed order,
+// so each graph gets what a separate net_pagerank call on it returns, up to
 // the association of sums. A large graph would keep one CTA busy long after
 // the rest of the batch is done, so the launch runs in thread-block clusters:
-// each cluster first splits the large graphs' rows over its CTAs, which add
-// their sums through distributed shared memory, then every CTA takes small
-// graphs alone. The vectors of the graph being solved stay in L2 (a graph's
-// nodes are contiguous in the packed numbering). A single small graph's
-// solve runs here too, as a batch of one.
+// each cluster first splits the large graphs over its CTAs, then every CTA
+// takes small graphs alone. A single small graph's solve runs here too, as a
+// batch of one.
+//
+// What bounds an iteration of a graph this small is latency: the chain from a
+// row's offsets over its columns to the gathered values, the sums, and the
+// barriers. So a graph is brought into shared memory once (16-bit columns,
+// values, out-strengths, and z = x / out in two buffers of which an iteration
+// reads one and writes the other), and an iteration has one reduction and one
+// barrier: the division by the total is left to the next iteration's scalars,
+// as in the sweeps (pagerank.cu), with the exact L1 change computed only when
+// the fused one cannot decide. CTAs of a cluster each keep all of z and write
+// every value they compute into all of the copies. Graphs whose arcs do not
+// fit keep those in global memory, graphs whose vectors do not fit keep
+// everything there.
+// With the graph in global memory and two reductions an iteration of a graph
+// of 500 nodes took 8.0 us, now 1.8 us; 10,000 nodes and 100,000 arcs on a
+// cluster of 8 13.6 us, now 7.5 us; R-MAT graphs of 30,000 nodes, whose hub rows
+// each waited for one thread, 235 us and 25 us.
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <numeric>
+#include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -39,161 +54,312 @@ struct EgoParams {
   int32_t jump_uniform;  // dangling nodes jump uniformly (1) or by p (0)
 };
 
-// Fixed-order CTA sums of K values at once (warp butterflies, then the warps
-// in order): two CTA barriers for all K. sh holds 32 K doubles.
-template <int K>
-__device__ __forceinline__ void cta_sums(double (&v)[K], double* sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int j = 0; j < K; ++j) v[j] = warp_sum(v[j]);
-  __syncthreads();  // the previous sums' reads of sh are done
-  if (lane == 0) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) sh[32 * j + w] = v[j];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    double t = 0;
-    for (int k = 0; k < nw; ++k) t += sh[32 * j + k];  // same order in every thread
-    v[j] = t;
-  }
-}
-
-// Sums over the rows of one graph split across the CTAs of a cluster: each
-// CTA's fixed-order sums go to its slots, and every thread adds the slots in
-// rank order through distributed shared memory, so all CTAs hold the same
-// bits. The cluster barrier also publishes every global write made before
-// it to the whole cluster (the z a product gathers from other CTAs' rows).
-template <int C, int K>
-__device__ __forceinline__ void cluster_sums(double (&v)[K], double* sh, double* slot,
-                                             cg::cluster_group& cl) {
-  cta_sums<K>(v, sh);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) slot[j] = v[j];
-  }
-  cl.sync();
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    double s = 0;
-#pragma unroll
-    for (int r = 0; r < C; ++r) s += cl.map_shared_rank(slot, (unsigned)r)[j];
-    v[j] = s;
-  }
-}
-
-// Fixed-order sums of K values over the rows of a graph: one CTA (C == 1)
-// or a cluster. Slots (C > 1): two sets of 4 doubles of this CTA's shared
-// memory, taken by turns, so a slot is written again only after every CTA
-// has passed the next cluster barrier and so has read it.
-template <int C, int K>
-__device__ __forceinline__ void graph_sums(double (&v)[K], double* sh, double* slots, int turn) {
-  if constexpr (C == 1) {
-    (void)slots;
-    (void)turn;
-    cta_sums<K>(v, sh);
-  } else {
-    cg::cluster_group cl = cg::this_cluster();
-    cluster_sums<C, K>(v, sh, slots + 4 * (turn & 1), cl);
-  }
-}
-
-// One graph's iteration over rows [lo, hi) of nodes [g_lo, g_hi): the whole
-// graph when C is 1 (one CTA), this CTA's share of it otherwise. The
-// reference's steps (z = x / out with the dangling mass, y = A z, the
-// update, the division by the total, the L1 change) with the next z and
-// dangling mass formed in the same pass as the division and the change, so
-// an iteration has two reductions (each a cluster barrier when C > 1).
+// Fixed-order sums of three values over the threads of a graph's CTAs: warp
+// butterflies, the warps of each CTA, and with C > 1 the CTAs of the cluster
+// in rank order, each CTA writing its sums into all CTAs' slots, so that all
+// hold the same bits. The barrier in it (the CTA's, or the cluster's) also
+// publishes everything written before it. sh (2 x 3 x 32 doubles) and slots
+// (2 x C x 4) are taken by turns: whoever writes one again has passed the
+// next barrier, so everybody has read it.
 template <int C>
-__device__ void ego_solve(const OpView<double>& op, const double* __restrict__ outstr,
-                          uint32_t g_lo, uint32_t g_hi, uint32_t lo, uint32_t hi,
-                          const EgoParams& prm, const double* __restrict__ pers, double ps,
-                          double* __restrict__ xa, double* __restrict__ xb,
-                          double* __restrict__ zb, double* __restrict__ out, int32_t* it_out,
-                          int32_t* done_out, double* change_out, double* sh, double* slots) {
-  const uint32_t nk = g_hi - g_lo;
-  const double inv_n = 1.0 / (double)nk;
-  double* x = xa;
-  double* y = xb;
-  int turn = 0;
-  // x = 1 / n; z = x / out; stuck = dangling mass
-  double st[1] = {0.0};
-  for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    x[i] = inv_n;
-    const double o = outstr[i];
-    if (o > 0.0) {
-      zb[i] = inv_n / o;
+__device__ __forceinline__ void ego_sums(double (&v)[3], double* sh, double* slots, int turn) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double* s = sh + (turn & 1) * 96;
+  const double m = warp_sum_scatter<3>(v, lane);
+  if ((lane & 7) == 0 && lane < 24) s[(lane >> 3) * 32 + w] = m;
+  __syncthreads();
+  if (C == 1 || w == 0) {
+    double a[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = lane < nw ? s[k * 32 + lane] : 0.0;
+    const double t = warp_sum_scatter<3>(a, lane);
+    if constexpr (C == 1) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = __shfl_sync(0xffffffffu, t, 8 * k);
     } else {
-      zb[i] = 0.0;
-      st[0] += inv_n;
+      cg::cluster_group cl = cg::this_cluster();
+      const int k = lane >> 3;
+      if (k < 3)
+        for (int r = lane & 7; r < C; r += 8)
+          cl.map_shared_rank(slots, (unsigned)r)[((turn & 1) * C + cl.block_rank()) * 4 + k] = t;
     }
   }
-  graph_sums<C, 1>(st, sh, slots, turn++);  // includes the barrier before z is read
-  double stuck = st[0];
+  if constexpr (C > 1) {
+    cg::this_cluster().sync();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double t = 0;
+#pragma unroll
+      for (int r = 0; r < C; ++r) t += slots[((turn & 1) * C + r) * 4 + k];
+      v[k] = t;
+    }
+  }
+}
+
+// A graph and this CTA's rows of it.
+struct EgoGraph {
+  OpView<double> op;
+  const float* vals32;   // the values in FP32 where all are exact there, else null
+  const double* inv_out; // 1 / out-strength, 0 for dangling nodes
+  uint32_t g_lo, nk;     // its nodes [g_lo, g_lo + nk)
+  uint32_t lo, hi;       // this CTA's rows
+  uint32_t rmax;         // most rows of any CTA of the cluster
+  const double* pers;    // null: uniform
+  double ps;             // sum of the graph's pers
+  double *y, *z;         // global iterates, each in two buffers n apart
+  uint32_t n;
+  double* out;
+};
+
+// Rows of more arcs than this are summed by a whole warp, before the others
+// and spread over the warps (the hubs of a skewed graph tend to be neighbours).
+constexpr uint32_t EGO_LONG = 32;
+
+// Where a graph lives: everything in shared memory, all but its arcs, nothing.
+enum { EGO_SMEM = 1, EGO_ARCS_GLOBAL = 2, EGO_GLOBAL = 3 };
+
+__host__ __device__ constexpr size_t ego_vector_bytes(size_t nk, size_t rows, bool pers) {
+  return 16 * nk + rows * (16 + 8 + (pers ? 8 : 0)) + 4 * ((rows + 2) & ~size_t(1));
+}
+__host__ __device__ constexpr size_t ego_arc_bytes(size_t arcs, size_t value_bytes) {
+  return ((arcs * value_bytes + 7) & ~size_t(7)) + arcs * 2;
+}
+
+// One graph's iteration. y holds the unnormalised iterate (x = y / T), z =
+// y / out; a sweep forms u = d (s / T + (D / T) jump) + (1 - d) p with D the
+// dangling mass of y. MT: the arc values' type (void: every entry is 1).
+template <int C, int TIER, class MT>
+__device__ __forceinline__ void ego_iterate(const EgoGraph& g, const EgoParams& prm, double* sh,
+                                            double* slots, int32_t* it_out, int32_t* done_out,
+                                            double* change_out) {
+  extern __shared__ __align__(16) unsigned char ego_smem[];
+  constexpr bool VALS = !std::is_void<MT>::value;
+  using V = std::conditional_t<VALS, MT, double>;
+  const uint32_t R = g.hi - g.lo, first = g.lo - g.g_lo;
+  const uint32_t lane = threadIdx.x & 31, T = blockDim.x;
+  const double inv_n = 1.0 / (double)g.nk;
+  const uint32_t a0 = g.op.off[g.lo], na = g.op.off[g.hi] - a0;
+  // z and y in two buffers each: b zs, b ys apart
+  double* z;
+  double* y;
+  const double* io;
+  const double* p;
+  const uint32_t* off;
+  const V* vals = nullptr;
+  const uint16_t* c16 = nullptr;
+  uint32_t zs = g.n, ys = g.n, off0 = a0;  // off[r] - off0: position in the CTA's arcs
+  const uint32_t* c32 = g.op.cols + a0;
+  if constexpr (VALS) {
+    if constexpr (sizeof(V) == 4) vals = g.vals32 + a0;
+    else vals = g.op.vals + a0;
+  }
+  if constexpr (TIER != EGO_GLOBAL) {
+    z = reinterpret_cast<double*>(ego_smem);
+    zs = g.nk;
+    y = z + 2 * zs;
+    ys = g.rmax;
+    double* sio = y + 2 * ys;
+    double* sp = sio + g.rmax;
+    uint32_t* soff = reinterpret_cast<uint32_t*>(sp + (g.pers ? g.rmax : 0));
+    for (uint32_t r = threadIdx.x; r < R; r += T) {
+      sio[r] = g.inv_out[g.lo + r];
+      if (g.pers) sp[r] = g.pers[g.lo + r] / g.ps;
+    }
+    for (uint32_t r = threadIdx.x; r <= R; r += T) soff[r] = g.op.off[g.lo + r] - a0;
+    if constexpr (TIER == EGO_SMEM) {
+      V* sv = reinterpret_cast<V*>(soff + ((g.rmax + 2) & ~1u));
+      uint16_t* sc = reinterpret_cast<uint16_t*>(sv);
+      if constexpr (VALS) sc = reinterpret_cast<uint16_t*>(sv + (sizeof(V) == 4 ? (na + 1) & ~1u : na));
+      for (uint32_t k = threadIdx.x; k < na; k += T) {
+        sc[k] = (uint16_t)(c32[k] - g.g_lo);
+        if constexpr (VALS) sv[k] = vals[k];
+      }
+      c16 = sc;
+      if constexpr (VALS) vals = sv;
+    }
+    io = sio;
+    p = sp;
+    off = soff;
+    off0 = 0;
+    __syncthreads();
+  } else {
+    z = g.z + g.g_lo;
+    y = g.y + g.lo;
+    io = g.inv_out + g.lo;
+    p = g.pers + g.lo;
+    off = g.op.off + g.lo;
+  }
+  const bool pers = g.pers != nullptr;
+  // z value of row r into every copy of buffer b
+  auto put_z = [&](int b, uint32_t r, double v) {
+    if constexpr (C == 1 || TIER == EGO_GLOBAL) {
+      z[b * zs + first + r] = v;
+    } else {
+      cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+      for (int q = 0; q < C; ++q) cl.map_shared_rank(z, (unsigned)q)[b * zs + first + r] = v;
+    }
+  };
+  auto column = [&](uint32_t k) {
+    if constexpr (TIER == EGO_SMEM) return (uint32_t)c16[k];
+    else return c32[k] - g.g_lo;
+  };
+  auto value = [&](uint32_t k) {
+    if constexpr (VALS) return vals[k];
+    else return 1.0;
+  };
+  auto term = [&](V w, double zv) {
+    if constexpr (VALS) return (double)w * zv;
+    else return zv;
+  };
+  int turn = 0;
+  double v3[3] = {0.0, 0.0, 0.0};
+  bool any_long = false;
+  for (uint32_t r = threadIdx.x; r < R; r += T) {
+    any_long |= off[r + 1] - off[r] > EGO_LONG;
+    y[r] = inv_n;
+    const double i = io[r];
+    put_z(0, r, inv_n * i);
+    if (i == 0.0) v3[1] += inv_n;
+  }
+  any_long = __syncthreads_or(any_long);
+  ego_sums<C>(v3, sh, slots, turn++);
+  double c_it = 1.0, c_dt = v3[1], total = 1.0, change = 0.0;
   int32_t it = 0, done = 0;
-  double change = 0.0;
+  int b = 0;
   while (it < prm.max_iter) {
-    // y = d (A z + stuck jump) + (1 - d) p
-    double tot[1] = {0.0};
-    for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      // arcs in CSR order; four gathers in flight before their products
-      // are added in that order
-      double s = 0;
-      uint32_t k = op.off[i];
-      const uint32_t ke = op.off[i + 1];
-      for (; k + 4 <= ke; k += 4) {
-        double zk[4], wk[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          zk[u] = zb[op.cols[k + u]];
-          wk[u] = op.vals ? op.vals[k + u] : 1.0;
+    const double* zb = z + b * zs;
+    const double* yo = y + b * ys;
+    double* yn = y + (b ^ 1) * ys;
+    double acc[3] = {0.0, 0.0, 0.0};
+    if (any_long) {  // their sums, left in yn
+      const uint32_t w = threadIdx.x >> 5, nw = T >> 5;
+      for (uint32_t r0 = 0; r0 < R; r0 += T) {
+        const uint32_t r = r0 + lane * nw + w;
+        const uint32_t k = r < R ? off[r] - off0 : 0u, ke = r < R ? off[r + 1] - off0 : 0u;
+        for (uint32_t m = __ballot_sync(0xffffffffu, ke - k > EGO_LONG); m; m &= m - 1) {
+          const int src = __ffs(m) - 1;
+          const uint32_t kb = __shfl_sync(0xffffffffu, k, src);
+          const uint32_t kx = __shfl_sync(0xffffffffu, ke, src);
+          double t = 0.0;
+#pragma unroll 4
+          for (uint32_t q = kb + lane; q < kx; q += 32) t += term(value(q), zb[column(q)]);
+          t = warp_sum(t);
+          if ((int)lane == src) yn[r] = t;
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s += wk[u] * zk[u];
       }
-      for (; k < ke; ++k) {
-        const double w = op.vals ? op.vals[k] : 1.0;
-        s += w * zb[op.cols[k]];
-      }
-      const double p = pers ? pers[i] / ps : inv_n;
-      const double jmp = prm.jump_uniform ? inv_n : p;
-      const double v = prm.d * (s + stuck * jmp) + (1.0 - prm.d) * p;
-      y[i] = v;
-      tot[0] += v;
+      __syncthreads();
     }
-    graph_sums<C, 1>(tot, sh, slots, turn++);  // every product has read z
-    const double total = tot[0];
-    // the division, the change, and the next z and dangling mass
-    double cs[2] = {0.0, 0.0};
-    for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      const double v = y[i] / total;
-      y[i] = v;
-      cs[0] += fabs(v - x[i]);
-      const double o = outstr[i];
-      if (o > 0.0) {
-        zb[i] = v / o;
+    for (uint32_t r = threadIdx.x; r < R; r += T) {
+      uint32_t k = off[r] - off0;
+      const uint32_t ke = off[r + 1] - off0;
+      double s = 0.0;
+      // arcs in CSR order, four under way at a time
+      if (ke - k > EGO_LONG) {
+        s = yn[r];
       } else {
-        zb[i] = 0.0;
-        cs[1] += v;
+        for (; k < ke; k += 4) {
+          uint32_t c[4];
+          V w[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t q = min(k + u, ke - 1);
+            c[u] = column(q);
+            w[u] = value(q);
+          }
+          double t[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) t[u] = zb[c[u]];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (k + u < ke) s += term(w[u], t[u]);
+        }
       }
+      const double pr = !pers ? inv_n : TIER != EGO_GLOBAL ? p[r] : p[r] / g.ps;
+      const double u = prm.d * (s * c_it + c_dt * (prm.jump_uniform ? inv_n : pr)) +
+                       (1.0 - prm.d) * pr;
+      const double i = io[r];
+      yn[r] = u;
+      put_z(b ^ 1, r, u * i);
+      acc[0] += u;
+      if (i == 0.0) acc[1] += u;
+      acc[2] += fabs(u - yo[r] * c_it);
     }
-    graph_sums<C, 2>(cs, sh, slots, turn++);  // publishes the next z
-    change = cs[0];
-    stuck = cs[1];
-    double* t = x;
-    x = y;
-    y = t;
+    ego_sums<C>(acc, sh, slots, turn++);
+    // sum |u - x| differs from the change sum |u / T - x| by at most |1 - T|;
+    // where that could decide otherwise, the change itself
+    total = acc[0];
+    change = acc[2];
+    if (fabs(change - prm.tol) <=
+        2.0 * fabs(1.0 - total) + 64.0 * DBL_EPSILON * fmax(change, prm.tol)) {
+      double ex[3] = {0.0, 0.0, 0.0};
+      for (uint32_t r = threadIdx.x; r < R; r += T) ex[0] += fabs(yn[r] / total - yo[r] * c_it);
+      ego_sums<C>(ex, sh, slots, turn++);
+      change = ex[0];
+    }
+    c_it = 1.0 / total;
+    c_dt = acc[1] * c_it;
+    b ^= 1;
     ++it;
     if (change <= prm.tol) {  // the same bits in every CTA of a cluster
       done = 1;
       break;
     }
   }
-  for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) out[i] = x[i];
+  for (uint32_t r = threadIdx.x; r < R; r += T) g.out[g.lo + r] = y[b * ys + r] / total;
   *it_out = it;
   *done_out = done;
   *change_out = change;
+}
+
+// Row boundary k of C of a graph: the first row i with i + off[i] (from the
+// graph's start) at least k / C of its rows plus arcs.
+__device__ __forceinline__ uint32_t ego_bound(const uint32_t* off, uint32_t g_lo, uint32_t g_hi,
+                                              uint32_t k, uint32_t C) {
+  const uint64_t all = (uint64_t)(g_hi - g_lo) + (off[g_hi] - off[g_lo]);
+  const uint64_t want = all * k / C;
+  uint32_t lo = g_lo, hi = g_hi;
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if ((uint64_t)(mid - g_lo) + (off[mid] - off[g_lo]) >= want) hi = mid; else lo = mid + 1;
+  }
+  return lo;
+}
+
+template <int C, class MT>
+__device__ __forceinline__ void ego_solve(EgoGraph g, uint32_t g_hi, const EgoParams& prm,
+                          uint32_t sm_bytes, uint32_t* bounds, double* sh, double* slots,
+                          int32_t* it, int32_t* done, double* ch) {
+  uint32_t amax;
+  if constexpr (C == 1) {
+    g.lo = g.g_lo;
+    g.hi = g_hi;
+    g.rmax = g.nk;
+    amax = g.op.off[g_hi] - g.op.off[g.g_lo];
+  } else {
+    if (threadIdx.x <= C)
+      bounds[threadIdx.x] = ego_bound(g.op.off, g.g_lo, g_hi, threadIdx.x, C);
+    __syncthreads();
+    const unsigned rank = cg::this_cluster().block_rank();
+    g.lo = bounds[rank];
+    g.hi = bounds[rank + 1];
+    g.rmax = 0;
+    amax = 0;
+    for (int k = 0; k < C; ++k) {  // the same in every CTA: all take the same tier
+      g.rmax = max(g.rmax, bounds[k + 1] - bounds[k]);
+      amax = max(amax, g.op.off[bounds[k + 1]] - g.op.off[bounds[k]]);
+    }
+  }
+  const size_t vec = ego_vector_bytes(g.nk, g.rmax, g.pers != nullptr);
+  size_t value_bytes = 0;
+  if constexpr (!std::is_void<MT>::value) value_bytes = sizeof(MT);
+  const size_t arcs = ego_arc_bytes(amax, value_bytes);
+  if (vec + arcs <= sm_bytes && g.nk <= 65536u)
+    ego_iterate<C, EGO_SMEM, MT>(g, prm, sh, slots, it, done, ch);
+  else if (vec <= sm_bytes)
+    ego_iterate<C, EGO_ARCS_GLOBAL, MT>(g, prm, sh, slots, it, done, ch);
+  else
+    ego_iterate<C, EGO_GLOBAL, MT>(g, prm, sh, slots, it, done, ch);
 }
 
 // The persistent launch. With clusters of C > 1 CTAs, each cluster first
@@ -203,18 +369,24 @@ __device__ void ego_solve(const OpView<double>& op, const double* __restrict__ o
 // are hardware barriers every CTA of the cluster executes the same number of
 // times: the graph index comes from rank 0's shared memory, and every CTA
 // stops a graph's iteration on the same bits.
-template <int C>
-__global__ void ego_pagerank(OpView<double> op, const double* __restrict__ outstr,
-                             const uint32_t* __restrict__ node_off, const uint32_t* __restrict__ order,
-                             uint32_t count, uint32_t nbig, unsigned int* __restrict__ queue,
-                             EgoParams prm, const double* __restrict__ pers,
-                             const double* __restrict__ psum, double* __restrict__ xa,
-                             double* __restrict__ xb, double* __restrict__ zb,
-                             double* __restrict__ out, int32_t* __restrict__ iters,
-                             int32_t* __restrict__ status, double* __restrict__ changes) {
-  __shared__ double sh[64];
-  __shared__ double slots[8];
+template <int C, class MT>
+__global__ void __launch_bounds__(1024, 1)
+ego_pagerank(EgoGraph g, const uint32_t* __restrict__ node_off,
+             const uint32_t* __restrict__ order, uint32_t count, uint32_t nbig,
+             unsigned int* __restrict__ queue, EgoParams prm, const double* __restrict__ psum,
+             uint32_t sm_bytes, int32_t* __restrict__ iters, int32_t* __restrict__ status,
+             double* __restrict__ changes) {
+  __shared__ double sh[2 * 3 * 32];
+  __shared__ double slots[2 * C * 4];
+  __shared__ uint32_t bounds[C + 1];
   __shared__ uint32_t g_sh;
+  auto take = [&](uint32_t graph) {
+    g.g_lo = node_off[graph];
+    const uint32_t g_hi = node_off[graph + 1];
+    g.nk = g_hi - g.g_lo;
+    if (g.pers) g.ps = psum[graph];
+    return g_hi;
+  };
   if constexpr (C > 1) {
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
@@ -225,13 +397,10 @@ __global__ void ego_pagerank(OpView<double> op, const double* __restrict__ outst
       cl.sync();  // every CTA has read it before rank 0 picks again or leaves
       if (gi >= nbig) break;
       const uint32_t graph = order[gi];
-      const uint32_t g_lo = node_off[graph], g_hi = node_off[graph + 1];
-      const uint32_t per = (g_hi - g_lo + C - 1) / C;
-      const uint32_t lo = min(g_hi, g_lo + rank * per), hi = min(g_hi, lo + per);
+      const uint32_t g_hi = take(graph);
       int32_t it = 0, done = 0;
       double ch = 0.0;
-      ego_solve<C>(op, outstr, g_lo, g_hi, lo, hi, prm, pers, pers ? psum[graph] : 1.0, xa, xb,
-                   zb, out, &it, &done, &ch, sh, slots);
+      ego_solve<C, MT>(g, g_hi, prm, sm_bytes, bounds, sh, slots, &it, &done, &ch);
       if (rank == 0 && threadIdx.x == 0) {
         iters[graph] = it;
         status[graph] = done ? 0 : 1;
@@ -246,19 +415,11 @@ __global__ void ego_pagerank(OpView<double> op, const double* __restrict__ outst
     __syncthreads();
     if (gi >= count) return;
     const uint32_t graph = order[gi];
-    const uint32_t g_lo = node_off[graph], g_hi = node_off[graph + 1];
-    if (g_hi == g_lo) {
-      if (threadIdx.x == 0) {
-        iters[graph] = 0;
-        status[graph] = 0;
-        changes[graph] = 0.0;
-      }
-      continue;
-    }
+    const uint32_t g_hi = take(graph);
     int32_t it = 0, done = 0;
     double ch = 0.0;
-    ego_solve<1>(op, outstr, g_lo, g_hi, g_lo, g_hi, prm, pers, pers ? psum[graph] : 1.0, xa, xb,
-                 zb, out, &it, &done, &ch, sh, slots);
+    if (g.nk == 0) done = 1;
+    else ego_solve<1, MT>(g, g_hi, prm, sm_bytes, bounds, sh, slots, &it, &done, &ch);
     if (threadIdx.x == 0) {
       iters[graph] = it;
       status[graph] = done ? 0 : 1;
@@ -295,35 +456,73 @@ void set_ego_threads(int t) { g_ego_threads = t; }
 void set_ego_cluster(int c) { g_ego_cluster = c; }
 void set_ego_big_nodes(int64_t v) { g_ego_big = v; }
 
-// Clusters of C CTAs of `threads` that fit on the device at once (0 if none),
-// per device and shape.
-template <int C>
-static int ego_clusters(int threads) {
+// The most dynamic shared memory a CTA can get (4 KB cover the static arrays
+// and what the driver takes).
+static uint32_t ego_most_smem() {
+  int dev = 0, optin = 0;
+  KNB_CUDA(cudaGetDevice(&dev));
+  KNB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  return (uint32_t)optin - 4096;
+}
+
+// Shape of a launch.
+struct EgoShape {
+  int threads = 256;
+  int cluster = 1;    // CTAs that split a large graph: 1, 4, 8 or 16
+  uint32_t smem = 0;  // dynamic shared memory per CTA
+  bool operator==(const EgoShape& o) const {
+    return threads == o.threads && cluster == o.cluster && smem == o.smem;
+  }
+};
+
+// In a batch, shared memory for the small graphs (about 600 nodes of 12 arcs,
+// in 1,200 vectors only) and the rest of the SM's 256 KB to L1, which serves the
+// gathers of the graphs that do not fit: 2,000 graphs of up to 50,000 nodes
+// take 1.24 ms with 32 KB a CTA, 2.3 ms with all there is.
+constexpr uint32_t EGO_BATCH_SMEM = 32768;
+
+// CTAs (C == 1) or clusters of C CTAs of `threads` that fit on the device at
+// once with their shared memory (0 if none), per device and shape.
+template <int C, class MT>
+static int ego_resident(int threads, uint32_t smem) {
   static std::mutex mu;
-  static std::map<std::pair<int, int>, int> cache;
+  static std::map<std::tuple<int, int, uint32_t>, int> cache;
   int dev = 0;
   KNB_CUDA(cudaGetDevice(&dev));
+  if (C > 8)
+    set_func_attr((const void*)ego_pagerank<C, MT>,
+                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  set_func_attr((const void*)ego_pagerank<C, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                (int)ego_most_smem());
   std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find({dev, threads});
+  auto it = cache.find({dev, threads, smem});
   if (it != cache.end()) return it->second;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(C);
-  cfg.blockDim = dim3(threads);
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)ego_pagerank<C>, &cfg) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    clusters = 0;
+  int fit = 0;
+  if constexpr (C == 1) {
+    int per_sm = 0, sms = 0;
+    KNB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ego_pagerank<1, MT>, threads,
+                                                           smem));
+    KNB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    fit = std::max(1, per_sm) * sms;
+  } else {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&fit, (const void*)ego_pagerank<C, MT>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      fit = 0;
+    }
   }
-  cache[{dev, threads}] = clusters;
-  return clusters;
+  cache[{dev, threads, smem}] = fit;
+  return fit;
 }
 
 // A packed batch kept per operator between calls: the graph offsets and the
@@ -338,13 +537,12 @@ struct EgoPlan : Workspace {
   bool pers = false;
   EgoParams prm{};
   std::vector<uint32_t> sizes;  // node counts of the graphs, largest first
-  int tuned_threads = 0;       // this batch's choice (0: not chosen yet)
-  int tuned_cluster = 0;
-  int threads = 0;             // of the instantiated launch
-  int cluster = 1;             // CTAs per cluster of the instantiated launch
+  bool tuned = false;          // this batch's shape is chosen
+  EgoShape pick;
+  EgoShape shape;              // of the instantiated launch
   uint32_t nbig = 0;           // graphs it gives to clusters
   DevBuf<uint32_t> doff, dorder;
-  DevBuf<double> dpers, dpsum, xa, xb, zb, dout;
+  DevBuf<double> dpers, dpsum, y, z, dout;
   DevBuf<int32_t> iters, status;
   DevBuf<double> changes;
   DevBuf<unsigned int> queue;
@@ -363,6 +561,11 @@ struct EgoPlan : Workspace {
     exec = nullptr;
     graph = nullptr;
   }
+};
+
+template <class T>
+struct TypeIs {
+  using type = T;
 };
 
 static bool same_params(const EgoParams& a, const EgoParams& b) {
@@ -438,13 +641,11 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     });
     KNB_CUDA(cudaMemcpyAsync(P.dorder.get(), order.data(), (size_t)count * 4,
                              cudaMemcpyHostToDevice, s));
-    P.tuned_threads = 0;
-    P.tuned_cluster = 0;
+    P.tuned = false;
     P.sizes.resize(count);
     for (uint32_t k = 0; k < count; ++k) P.sizes[k] = hoff[order[k] + 1] - hoff[order[k]];
-    P.xa.alloc(n);
-    P.xb.alloc(n);
-    P.zb.alloc(n);
+    P.y.alloc((size_t)2 * n);
+    P.z.alloc((size_t)2 * n);
     P.dout.alloc(n);
     P.iters.alloc(count);
     P.status.alloc(count);
@@ -475,28 +676,46 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   // cluster; the others go one per CTA. Returns the graphs given to clusters.
   auto big_count = [&](uint64_t ctas) {
     const int64_t pin_big = g_ego_big.load();
-    const uint64_t big = pin_big > 0 ? (uint64_t)pin_big
-                                       : std::max<uint64_t>(4096, (uint64_t)n / std::max<uint64_t>(ctas, 1));
+    const uint64_t big =
+        pin_big > 0 ? (uint64_t)pin_big
+        : count == 1 ? 1  // the shape chosen for it says whether it is split
+                     : std::max<uint64_t>(4096, (uint64_t)n / std::max<uint64_t>(ctas, 1));
     uint32_t nb = 0;
     while (nb < count && P.sizes[nb] >= big) ++nb;
     return nb;
   };
-  auto launch = [&](int threads, int C, cudaStream_t st) -> uint32_t {
+  EgoGraph base{};
+  base.op = op.view64();
+  base.vals32 = op.has_vals && op.vals32_exact ? op.vals32.get() : nullptr;
+  base.inv_out = op.inv_out64.get();
+  base.pers = pers ? P.dpers.get() : nullptr;
+  base.ps = 1.0;
+  base.y = P.y.get();
+  base.z = P.z.get();
+  base.n = n;
+  base.out = P.dout.get();
+  auto launch_as = [&](auto mt, const EgoShape& shape, cudaStream_t st) -> uint32_t {
+    using MT = typename decltype(mt)::type;
     KNB_CUDA(cudaMemsetAsync(P.queue.get(), 0, 8, st));
-    const uint64_t fit = (uint64_t)sms * (2048 / threads);
+    const int threads = shape.threads, C = shape.cluster;
+    const uint32_t smem = shape.smem;
     int clusters = 0;
-    if (C == 4) clusters = ego_clusters<4>(threads);
-    if (C == 8) clusters = ego_clusters<8>(threads);
+    if (C == 4) clusters = ego_resident<4, MT>(threads, smem);
+    if (C == 8) clusters = ego_resident<8, MT>(threads, smem);
+    if (C == 16) clusters = ego_resident<16, MT>(threads, smem);
     const uint32_t nbig = clusters > 0 ? big_count((uint64_t)clusters * C) : 0;
+    const double* psum = pers ? P.dpsum.get() : nullptr;
     if (nbig == 0) {
-      const unsigned grid = (unsigned)std::min<uint64_t>(count, fit);
-      ego_pagerank<1><<<grid, threads, 0, st>>>(
-          op.view64(), op.colsum.get(), P.doff.get(), P.dorder.get(), count, 0u, P.queue.get(),
-          prm, pers ? P.dpers.get() : nullptr, pers ? P.dpsum.get() : nullptr, P.xa.get(),
-          P.xb.get(), P.zb.get(), P.dout.get(), P.iters.get(), P.status.get(), P.changes.get());
+      const unsigned grid =
+          (unsigned)std::min<uint64_t>(count, (uint64_t)ego_resident<1, MT>(threads, smem));
+      ego_pagerank<1, MT><<<grid, threads, smem, st>>>(base, P.doff.get(), P.dorder.get(), count, 0u,
+                                                   P.queue.get(), prm, psum, smem, P.iters.get(),
+                                                   P.status.get(), P.changes.get());
       KNB_LAUNCH("ego_pagerank");
       return 0;
     }
+    // no more clusters than there is work for
+    if (nbig == count) clusters = (int)std::min<uint32_t>((uint32_t)clusters, nbig);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)C;
@@ -505,76 +724,91 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * C));
     cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     auto args = [&](auto fn) {
-      KNB_CUDA(cudaLaunchKernelEx(&cfg, fn, op.view64(), (const double*)op.colsum.get(),
-                                  (const uint32_t*)P.doff.get(), (const uint32_t*)P.dorder.get(),
-                                  count, nbig, P.queue.get(), prm,
-                                  (const double*)(pers ? P.dpers.get() : nullptr),
-                                  (const double*)(pers ? P.dpsum.get() : nullptr), P.xa.get(),
-                                  P.xb.get(), P.zb.get(), P.dout.get(), P.iters.get(),
-                                  P.status.get(), P.changes.get()));
+      KNB_CUDA(cudaLaunchKernelEx(&cfg, fn, base, (const uint32_t*)P.doff.get(),
+                                  (const uint32_t*)P.dorder.get(), count, nbig, P.queue.get(), prm,
+                                  psum, smem, P.iters.get(), P.status.get(), P.changes.get()));
     };
-    if (C == 4) args(ego_pagerank<4>);
-    else args(ego_pagerank<8>);
+    if (C == 4) args(ego_pagerank<4, MT>);
+    else if (C == 8) args(ego_pagerank<8, MT>);
+    else args(ego_pagerank<16, MT>);
     KNB_LAUNCH("ego_pagerank");
     return nbig;
+  };
+  auto launch = [&](const EgoShape& shape, cudaStream_t st) -> uint32_t {
+    if (!op.has_vals) return launch_as(TypeIs<void>{}, shape, st);
+    if (base.vals32) return launch_as(TypeIs<float>{}, shape, st);
+    return launch_as(TypeIs<double>{}, shape, st);
   };
   if (!P.t0) {
     KNB_CUDA(cudaEventCreate(&P.t0));
     KNB_CUDA(cudaEventCreate(&P.t1));
   }
-  // Threads per CTA and CTAs per cluster, unless pinned (tuning keys 6 and
-  // 16): for a batch of at least 2^20 arcs, timed once per batch layout on
-  // the batch itself; smaller batches, whose launch takes microseconds, take
-  // clusters of 8 and 1024 threads when they have fewer graphs than the GPU
-  // has SMs (a single graph: 0.54 ms for C1 against 0.77 ms at 256), else
-  // 256. Results do not depend on the choice beyond the association of a
-  // split graph's sums.
+  // The launch's shape, unless pinned (tuning keys 6 and 16). Results do not
+  // depend on it beyond the association of a split graph's sums.
+  // - One graph: from 400 nodes on a cluster of 8 (500 nodes: 270 us a call
+  //   against 292 on one CTA, 200 nodes: 258 against 208), as many threads as
+  //   its CTAs have rows, and all the shared memory; a graph too large for
+  //   that takes a cluster of 16 and leaves the memory to L1.
+  // - A batch of at least 2^20 arcs: timed once per batch layout on the batch
+  //   itself.
+  // - Smaller batches: 1,024 threads and clusters of 16 when a graph is large
+  //   enough to be split (100 graphs up to 20,000 nodes: 390 us against 626
+  //   with 256 threads), else 256 threads.
   const int pin_t = g_ego_threads.load(), pin_c = g_ego_cluster.load();
-  if (P.tuned_threads == 0) {
-    int pick_t = pin_t ? pin_t : ((int)count < sms ? 1024 : 256);
-    int pick_c = pin_c ? pin_c : 8;
-    if ((pin_t == 0 || pin_c == 0) && op.nnz >= (1u << 20)) {
-      float best = 1e30f;
-      for (int t : {128, 256, 512, 1024}) {
-        if (pin_t != 0 && t != pin_t) continue;
-        for (int c : {1, 4, 8}) {
-          if (pin_c != 0 && c != pin_c) continue;
+  if (!P.tuned) {
+    EgoShape pick;
+    const uint32_t most = ego_most_smem();
+    if (count == 1) {
+      const size_t vb = !op.has_vals ? 0 : base.vals32 ? 4 : 8;
+      const bool fits = ego_vector_bytes(n, n / 8 + n / 16, pers) +
+                            ego_arc_bytes(op.nnz / 8 + op.nnz / 32, vb) <= most;
+      const uint32_t rows = fits ? n / 8 : n / 16;
+      pick.cluster = n < 400 ? 1 : fits ? 8 : 16;
+      pick.threads = n < 400 || rows <= 256 ? 256 : rows <= 512 ? 512 : 1024;
+      pick.smem = fits ? most : 4096;
+    } else {
+      const bool split = P.sizes[0] >= 4096;
+      pick = {split ? 1024 : 256, split ? 16 : 8, EGO_BATCH_SMEM};
+      if ((pin_t == 0 || pin_c == 0) && op.nnz >= (1u << 20)) {
+        float best = 1e30f;
+        for (EgoShape c : {EgoShape{256, 8, EGO_BATCH_SMEM}, EgoShape{256, 16, EGO_BATCH_SMEM},
+                           EgoShape{512, 16, EGO_BATCH_SMEM}, EgoShape{1024, 16, EGO_BATCH_SMEM}}) {
+          if (c.cluster == 16 && c.threads == 256 && !split) continue;
           KNB_CUDA(cudaEventRecord(P.t0, s));
-          launch(t, c, s);
+          launch(c, s);
           KNB_CUDA(cudaEventRecord(P.t1, s));
           KNB_CUDA(cudaEventSynchronize(P.t1));
           float ms = 0;
           KNB_CUDA(cudaEventElapsedTime(&ms, P.t0, P.t1));
           if (ms < best) {
             best = ms;
-            pick_t = t;
-            pick_c = c;
+            pick = c;
           }
         }
       }
     }
-    P.tuned_threads = pick_t;
-    P.tuned_cluster = pick_c;
+    P.pick = pick;
+    P.tuned = true;
   }
-  const int threads = pin_t ? pin_t : P.tuned_threads;
-  const int cluster = pin_c ? pin_c : P.tuned_cluster;
-  if (!P.exec || P.threads != threads || P.cluster != cluster || P.pers != pers ||
-      !same_params(P.prm, prm)) {
+  EgoShape shape = P.pick;
+  if (pin_t) shape.threads = pin_t;
+  if (pin_c) shape.cluster = pin_c;
+  if (!P.exec || !(P.shape == shape) || P.pers != pers || !same_params(P.prm, prm)) {
     P.drop_graph();
     cudaStream_t cs;
     KNB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     KNB_CUDA(cudaStreamSynchronize(s));
     KNB_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    P.nbig = launch(threads, cluster, cs);
+    P.nbig = launch(shape, cs);
     KNB_CUDA(cudaStreamEndCapture(cs, &P.graph));
     KNB_CUDA(cudaGraphInstantiate(&P.exec, P.graph, 0));
     KNB_CUDA(cudaStreamDestroy(cs));
-    P.threads = threads;
-    P.cluster = cluster;
+    P.shape = shape;
     P.pers = pers;
     P.prm = prm;
     ++P.instantiations;
@@ -603,8 +837,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   KNB_CUDA(cudaStreamSynchronize(s));
   if (res) {
     res->seconds = ms * 1e-3;
-    res->threads = threads;
-    res->cluster = P.nbig ? cluster : 1;
+    res->threads = shape.threads;
+    res->cluster = P.nbig ? shape.cluster : 1;
     res->split_graphs = (int32_t)P.nbig;
     res->instantiations = P.instantiations;
     int64_t tot = 0, mx = 0;
