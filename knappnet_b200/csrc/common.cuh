@@ -238,6 +238,19 @@ struct PlainMemory {
   PlainMemory(const PlainMemory&) = delete;
 };
 
+// Page-locked host memory of the calling thread for small copies (a copy from
+// or to pageable memory costs about 10 us and waits; freed with the thread).
+// The lower half is for copies to the device, the upper for copies back, and
+// whoever uses it waits for its copies before returning.
+constexpr size_t STAGING_HALF = size_t(512) << 10;
+struct HostStaging {
+  unsigned char* p = nullptr;  // null where none could be had
+  HostStaging();
+  ~HostStaging();
+  HostStaging(const HostStaging&) = delete;
+};
+HostStaging& host_staging();
+
 // Device memory owned by RAII.
 template <class T>
 struct DevBuf {

@@ -542,9 +542,8 @@ struct EgoPlan : Workspace {
   EgoShape shape;              // of the instantiated launch
   uint32_t nbig = 0;           // graphs it gives to clusters
   DevBuf<uint32_t> doff, dorder;
-  DevBuf<double> dpers, dpsum, y, z, dout;
-  DevBuf<int32_t> iters, status;
-  DevBuf<double> changes;
+  DevBuf<double> dpers, y, z;
+  DevBuf<double> result;  // scores (n), changes (count), iterations and statuses (2 count int32)
   DevBuf<unsigned int> queue;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -646,24 +645,30 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     for (uint32_t k = 0; k < count; ++k) P.sizes[k] = hoff[order[k] + 1] - hoff[order[k]];
     P.y.alloc((size_t)2 * n);
     P.z.alloc((size_t)2 * n);
-    P.dout.alloc(n);
-    P.iters.alloc(count);
-    P.status.alloc(count);
-    P.changes.alloc(count);
+    P.result.alloc((size_t)n + 2 * (size_t)count);
     P.queue.alloc(2);
     P.dpers.release();
-    P.dpsum.release();
     KNB_CUDA(cudaStreamSynchronize(s));
     P.hoff = hoff;
   }
-  if (pers && !P.dpers.get()) {
-    P.dpers.alloc(n);
-    P.dpsum.alloc(count);
-  }
-  if (pers) {
-    KNB_CUDA(cudaMemcpyAsync(P.dpers.get(), in.personalization, (size_t)n * 8,
-                             cudaMemcpyHostToDevice, s));
-    KNB_CUDA(cudaMemcpyAsync(P.dpsum.get(), ps.data(), (size_t)count * 8, cudaMemcpyHostToDevice, s));
+  double* const scores = P.result.get();
+  double* const changes = scores + n;
+  int32_t* const iters = reinterpret_cast<int32_t*>(changes + count);
+  int32_t* const status = iters + count;
+  unsigned char* const stage = host_staging().p;
+  if (pers) {  // the vectors, then their sums
+    if (!P.dpers.get()) P.dpers.alloc((size_t)n + count);
+    if (stage && ((size_t)n + count) * 8 <= STAGING_HALF) {
+      memcpy(stage, in.personalization, (size_t)n * 8);
+      memcpy(stage + (size_t)n * 8, ps.data(), (size_t)count * 8);
+      KNB_CUDA(cudaMemcpyAsync(P.dpers.get(), stage, ((size_t)n + count) * 8,
+                               cudaMemcpyHostToDevice, s));
+    } else {
+      KNB_CUDA(cudaMemcpyAsync(P.dpers.get(), in.personalization, (size_t)n * 8,
+                               cudaMemcpyHostToDevice, s));
+      KNB_CUDA(cudaMemcpyAsync(P.dpers.get() + n, ps.data(), (size_t)count * 8,
+                               cudaMemcpyHostToDevice, s));
+    }
   }
   const EgoParams prm{in.damping, in.tol, (int32_t)std::min<int64_t>(in.max_iter, INT32_MAX),
                       in.dangling == 1 ? 1 : 0};
@@ -693,7 +698,7 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   base.y = P.y.get();
   base.z = P.z.get();
   base.n = n;
-  base.out = P.dout.get();
+  base.out = scores;
   auto launch_as = [&](auto mt, const EgoShape& shape, cudaStream_t st) -> uint32_t {
     using MT = typename decltype(mt)::type;
     KNB_CUDA(cudaMemsetAsync(P.queue.get(), 0, 8, st));
@@ -704,13 +709,13 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     if (C == 8) clusters = ego_resident<8, MT>(threads, smem);
     if (C == 16) clusters = ego_resident<16, MT>(threads, smem);
     const uint32_t nbig = clusters > 0 ? big_count((uint64_t)clusters * C) : 0;
-    const double* psum = pers ? P.dpsum.get() : nullptr;
+    const double* psum = pers ? P.dpers.get() + n : nullptr;
     if (nbig == 0) {
       const unsigned grid =
           (unsigned)std::min<uint64_t>(count, (uint64_t)ego_resident<1, MT>(threads, smem));
       ego_pagerank<1, MT><<<grid, threads, smem, st>>>(base, P.doff.get(), P.dorder.get(), count, 0u,
-                                                   P.queue.get(), prm, psum, smem, P.iters.get(),
-                                                   P.status.get(), P.changes.get());
+                                                   P.queue.get(), prm, psum, smem, iters, status,
+                                                   changes);
       KNB_LAUNCH("ego_pagerank");
       return 0;
     }
@@ -731,7 +736,7 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     auto args = [&](auto fn) {
       KNB_CUDA(cudaLaunchKernelEx(&cfg, fn, base, (const uint32_t*)P.doff.get(),
                                   (const uint32_t*)P.dorder.get(), count, nbig, P.queue.get(), prm,
-                                  psum, smem, P.iters.get(), P.status.get(), P.changes.get()));
+                                  psum, smem, iters, status, changes));
     };
     if (C == 4) args(ego_pagerank<4, MT>);
     else if (C == 8) args(ego_pagerank<8, MT>);
@@ -816,13 +821,23 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   KNB_CUDA(cudaEventRecord(P.t0, s));
   KNB_CUDA(cudaGraphLaunch(P.exec, s));
   KNB_CUDA(cudaEventRecord(P.t1, s));
-  std::vector<int32_t> hst(count), hit(count);
-  double change0 = 0.0;
-  KNB_CUDA(cudaMemcpyAsync(hst.data(), P.status.get(), (size_t)count * 4, cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaMemcpyAsync(hit.data(), P.iters.get(), (size_t)count * 4, cudaMemcpyDeviceToHost, s));
-  if (count == 1)
-    KNB_CUDA(cudaMemcpyAsync(&change0, P.changes.get(), 8, cudaMemcpyDeviceToHost, s));
+  // what the launch reports, and with it, where both are small, the scores:
+  // one copy through page-locked memory
+  const size_t meta = (size_t)count * 16, all = (size_t)n * 8 + meta;
+  const bool together = stage && !in.out_on_device && all <= STAGING_HALF;
+  std::vector<unsigned char> own;
+  unsigned char* back = stage + STAGING_HALF;
+  if (!stage || meta > STAGING_HALF) {
+    own.resize(meta);
+    back = own.data();
+  }
+  KNB_CUDA(cudaMemcpyAsync(back, together ? scores : changes, together ? all : meta,
+                           cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
+  const double* hscores = reinterpret_cast<const double*>(back);
+  const double* hchange = together ? hscores + n : hscores;
+  const int32_t* hit = reinterpret_cast<const int32_t*>(hchange + count);
+  const int32_t* hst = hit + count;
   float ms = 0;
   KNB_CUDA(cudaEventElapsedTime(&ms, P.t0, P.t1));
   for (uint32_t k = 0; k < count; ++k)
@@ -830,11 +845,14 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
       throw Error("PageRank did not converge to tolerance " + std::to_string(in.tol) +
                   " within " + std::to_string(in.max_iter) + " iterations" +
                   (count > 1 ? " (graph " + std::to_string(k) + " of the batch)" : ""));
-  if (in.out_on_device)
-    KNB_CUDA(cudaMemcpyAsync(out, P.dout.get(), (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
-  else
-    KNB_CUDA(cudaMemcpyAsync(out, P.dout.get(), (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaStreamSynchronize(s));
+  if (together) {
+    memcpy(out, hscores, (size_t)n * 8);
+  } else {
+    KNB_CUDA(cudaMemcpyAsync(out, scores, (size_t)n * 8,
+                             in.out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                             s));
+    KNB_CUDA(cudaStreamSynchronize(s));
+  }
   if (res) {
     res->seconds = ms * 1e-3;
     res->threads = shape.threads;
@@ -847,7 +865,7 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
       mx = std::max<int64_t>(mx, hit[k]);
     }
     res->total_iterations = tot;
-    res->change = change0;
+    res->change = count == 1 ? hchange[0] : 0.0;
     res->max_iterations = mx;
     if (in.iterations_out)
       for (uint32_t k = 0; k < count; ++k) in.iterations_out[k] = hit[k];

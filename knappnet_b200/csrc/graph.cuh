@@ -168,8 +168,7 @@ struct GraphHandleImpl {
   int device = 0;
   DevBuf<uint32_t> src, tgt;  // edges in input order
   DevBuf<double> w;
-  std::vector<uint32_t> h_src, h_tgt;  // host copies (components, acyclicity)
-  std::vector<double> h_w;
+  uint64_t first_negative = ~0ull;  // first edge of negative weight (~0: none), from the build
   DevCsr out;                  // out-arcs (all arcs for undirected graphs)
   DevCsr inc;                  // in-arcs, directed graphs only
   std::unique_ptr<DevCsr> und; // directions ignored, directed graphs only (lazy)

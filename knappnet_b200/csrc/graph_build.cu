@@ -101,6 +101,19 @@ void device_free(const DeviceBlock& b) noexcept {
   }
 }
 
+HostStaging::HostStaging() {
+  void* q = nullptr;
+  if (cudaMallocHost(&q, 2 * STAGING_HALF) == cudaSuccess) p = static_cast<unsigned char*>(q);
+  else cudaGetLastError();
+}
+HostStaging::~HostStaging() {
+  if (p) cudaFreeHost(p);
+}
+HostStaging& host_staging() {
+  thread_local HostStaging s;
+  return s;
+}
+
 void device_pool_trim() {
   int dev = 0;
   KNB_CUDA(cudaGetDevice(&dev));
