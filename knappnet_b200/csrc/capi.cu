@@ -614,19 +614,17 @@ int32_t net_katz(const GraphHandle* h, double alpha, const double* beta, int64_t
       throw Error("alpha is " + fmt_g(alpha) +
                   "; it must be a nonnegative number below 1 / lambda_max");
     const uint32_t n = g.n;
-    std::vector<double> b;
-    if (beta_len == 1) b.assign(n, beta[0]);
-    else if ((uint64_t)beta_len == n) b.assign(beta, beta + n);
-    else
+    if (beta_len != 1 && (uint64_t)beta_len != n)
       throw Error("beta: expected length " + std::to_string(n) + ", found " +
                   std::to_string(beta_len));
-    for (double v : b)
-      if (!std::isfinite(v)) throw Error("beta must be finite");
+    if (n > 0)
+      for (int64_t i = 0; i < beta_len; ++i)
+        if (!std::isfinite(beta[i])) throw Error("beta must be finite");
     if (n == 0) return;
     cudaStream_t s = knb::thread_stream();
     if (p.weighted) check_nonnegative(g, "Katz centrality", s);
     knb::SeriesResult r;
-    knb::katz(g, alpha, b, normalized != 0, p, out, &r, s);
+    knb::katz(g, alpha, beta, beta_len == 1, normalized != 0, p, out, &r, s);
   });
 }
 

@@ -1270,6 +1270,64 @@ __global__ void scale_by(double* x, size_t dim, double f, int divide) {
     x[i] = divide ? x[i] / f : x[i] * f;
 }
 
+// Negative entries to 0, then the maximum, the sum and the sum of squares of x
+// into the state (xinf, sum, xx); the last CTA joins the CTAs' values in order.
+__global__ void __launch_bounds__(VB_T)
+clamp_stats(double* __restrict__ x, size_t dim, double* __restrict__ part, LzState* st) {
+  __shared__ double sh[VB_T / 32];
+  double m = 0.0, t = 0.0, q = 0.0;
+  for (size_t i = blockIdx.x * (size_t)VB_T + threadIdx.x; i < dim;
+       i += (size_t)gridDim.x * VB_T) {
+    double v = x[i];
+    if (v < 0.0) x[i] = v = 0.0;
+    m = fmax(m, v);
+    t += v;
+    q += v * v;
+  }
+  m = block_max(m, sh);
+  t = block_sum(t, sh);
+  q = block_sum(q, sh);
+  if (threadIdx.x == 0) {
+    part[3 * blockIdx.x] = m;
+    part[3 * blockIdx.x + 1] = t;
+    part[3 * blockIdx.x + 2] = q;
+  }
+  if (!lz_last(&st->ticket)) return;
+  if (threadIdx.x < 32) {
+    const volatile double* p = part;
+    double a = 0.0;
+    for (uint32_t k = threadIdx.x; k < gridDim.x; k += 32) a = fmax(a, p[3 * k]);
+    a = warp_max(a);
+    const double b = fixed_block_sum(part, gridDim.x, 3, 1);
+    const double c = fixed_block_sum(part, gridDim.x, 3, 2);
+    if (threadIdx.x == 0) {
+      st->xinf = a;
+      st->sum = b;
+      st->xx = c;
+      st->ticket = 0;
+    }
+  }
+}
+
+// x /= its maximum (how 0), sum (1) or Euclidean length (2), as clamp_stats
+// left them, unless that is 0.
+__global__ void scale_by_stats(double* x, size_t dim, const LzState* st, int how) {
+  const double d = how == 0 ? st->xinf : how == 1 ? st->sum : sqrt(st->xx);
+  if (!(d > 0.0)) return;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < dim;
+       i += (size_t)gridDim.x * blockDim.x)
+    x[i] = x[i] / d;
+}
+
+// x[nodes[i]] = u[i] (u . s), the dot product as lz_dots left it (xy).
+__global__ void scatter_by_dot(const uint32_t* __restrict__ nodes, uint32_t k,
+                               const double* __restrict__ u, const LzState* st,
+                               double* __restrict__ x) {
+  const double f = st->xy;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x)
+    x[nodes[i]] = u[i] * f;
+}
+
 __global__ void to_float(const double* __restrict__ x, size_t dim, float* __restrict__ y) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < dim;
        i += (size_t)gridDim.x * blockDim.x)
@@ -1840,22 +1898,6 @@ __global__ void hits_col_sums(OpView<double> at, double* __restrict__ col_sum,
 }
 
 
-void hits_rescale(std::vector<double>& x, int how) {
-  for (double& v : x)
-    if (v < 0.0) v = 0.0;
-  double d = 0.0;
-  if (how == 0) {
-    for (double v : x) d = std::max(d, v);
-  } else if (how == 1) {
-    for (double v : x) d += v;
-  } else {
-    for (double v : x) d += v * v;
-    d = std::sqrt(d);
-  }
-  if (d > 0.0)
-    for (double& v : x) v /= d;
-}
-
 }  // namespace
 
 // What hubs and authorities on one operator can reuse: the blocks, their
@@ -1870,13 +1912,14 @@ struct HitsPlan : Workspace {
   std::vector<size_t> order;
   struct Block {
     DevOp ab, abt;
-    DevBuf<double> sdev;
-    std::vector<double> sv;
+    DevBuf<uint32_t> auths;   // its authorities
+    DevBuf<double> sdev, v;   // A_b^T 1, and its last solve's eigenvector
   };
   std::map<size_t, std::unique_ptr<Block>> blocks;
-  DevBuf<uint32_t> hub_index, auth_index, nodes_h, nodes_a;
-  DevBuf<double> vdev;
+  DevBuf<uint32_t> hub_index, auth_index, nodes_h;
+  DevBuf<double> hubs, auth;  // the scores, n each
   LzBuffers lz;
+  SpmvScratch sc;             // of the products outside the Lanczos process
 };
 
 // The blocks, their bounds and their order (spectral.rs:757-836), computed
@@ -1957,7 +2000,8 @@ static void hits_prepare(HitsPlan& plan, const OpView<double>& a64, const OpView
   plan.hub_index.alloc(n);
   plan.auth_index.alloc(n);
   plan.nodes_h.alloc(n);
-  plan.nodes_a.alloc(n);
+  plan.hubs.alloc(n);
+  plan.auth.alloc(n);
   KNB_CUDA(cudaMemsetAsync(plan.hub_index.get(), 0xFF, (size_t)n * 4, s));
   KNB_CUDA(cudaMemsetAsync(plan.auth_index.get(), 0xFF, (size_t)n * 4, s));
   plan.ready = true;
@@ -1999,10 +2043,9 @@ void hits(GraphHandleImpl& g, const HitsParams& p, double* hubs_out, double* aut
   const double TIE = 1e-9;
   double best = 0.0;
   struct Solved {
-    size_t b;
     double value;
-    std::vector<double> v;
-    const std::vector<double>* sv;
+    HitsPlan::Block* blk;
+    uint32_t na;
   };
   std::vector<Solved> solved;
   int launches = 0;
@@ -2011,59 +2054,58 @@ void hits(GraphHandleImpl& g, const HitsParams& p, double* hubs_out, double* aut
     const uint32_t nh = (uint32_t)bh[b].size(), na = (uint32_t)ba[b].size();
     std::unique_ptr<HitsPlan::Block>& blk = plan.blocks[b];
     if (!blk) {
-      blk = std::make_unique<HitsPlan::Block>();
+      auto made = std::make_unique<HitsPlan::Block>();
       DevBuf<uint32_t>& nodes_h = plan.nodes_h;
-      DevBuf<uint32_t>& nodes_a = plan.nodes_a;
+      DevBuf<uint32_t>& nodes_a = made->auths;
+      nodes_a.alloc(std::max<uint32_t>(na, 1));
       KNB_CUDA(cudaMemcpyAsync(nodes_h.get(), bh[b].data(), (size_t)nh * 4, cudaMemcpyHostToDevice, s));
       KNB_CUDA(cudaMemcpyAsync(nodes_a.get(), ba[b].data(), (size_t)na * 4, cudaMemcpyHostToDevice, s));
       scatter_local<<<grid_for(nh, 256), 256, 0, s>>>(nodes_h.get(), nh, plan.hub_index.get());
       scatter_local<<<grid_for(na, 256), 256, 0, s>>>(nodes_a.get(), na, plan.auth_index.get());
       DevBuf<uint32_t> tmp_nodes(std::max(nh, na));
-      mapped_submatrix(a64, bh[b], plan.auth_index.get(), tmp_nodes, blk->ab, s);
-      mapped_submatrix(t64, ba[b], plan.hub_index.get(), tmp_nodes, blk->abt, s);
+      mapped_submatrix(a64, bh[b], plan.auth_index.get(), tmp_nodes, made->ab, s);
+      mapped_submatrix(t64, ba[b], plan.hub_index.get(), tmp_nodes, made->abt, s);
       unscatter_local<<<grid_for(nh, 256), 256, 0, s>>>(nodes_h.get(), nh, plan.hub_index.get());
       unscatter_local<<<grid_for(na, 256), 256, 0, s>>>(nodes_a.get(), na, plan.auth_index.get());
       // Kleinberg's first authority vector A_b^T 1
       DevBuf<double> ones(std::max<uint32_t>(nh, 1));
-      blk->sdev.alloc(std::max<uint32_t>(na, 1));
+      made->sdev.alloc(std::max<uint32_t>(na, 1));
+      made->v.alloc(std::max<uint32_t>(na, 1));
       fill_value<<<grid_for(nh, 256), 256, 0, s>>>(ones.get(), nh, 1.0);
-      SpmvScratch sc;
-      launches += 6 + spmv(blk->abt, ones.get(), nullptr, blk->sdev.get(), sc, nullptr, s);
-      blk->sv.resize(na);
-      KNB_CUDA(cudaMemcpyAsync(blk->sv.data(), blk->sdev.get(), (size_t)na * 8,
-                               cudaMemcpyDeviceToHost, s));
+      launches += 6 + spmv(made->abt, ones.get(), nullptr, made->sdev.get(), plan.sc, nullptr, s);
       KNB_CUDA(cudaStreamSynchronize(s));
+      blk = std::move(made);
     }
-    if (plan.vdev.n < na) plan.vdev.alloc(na);
     Leading res;
-    if (!symmetric_leading(blk->ab, p.tol, 0.0, p.max_iter, false, plan.vdev.get(), &res,
-                           &launches, s, &blk->abt, blk->sdev.get(), &plan.lz))
+    if (!symmetric_leading(blk->ab, p.tol, 0.0, p.max_iter, false, blk->v.get(), &res, &launches,
+                           s, &blk->abt, blk->sdev.get(), &plan.lz))
       throw Error("hub and authority scores did not converge to tolerance " + fmt_g(p.tol) +
                   " within " + std::to_string(p.max_iter) +
                   " matrix-vector products; a larger iteration cap may help");
-    Solved sol;
-    sol.b = b;
-    sol.value = res.value;
-    sol.v.resize(na);
-    sol.sv = &blk->sv;
-    KNB_CUDA(cudaMemcpyAsync(sol.v.data(), plan.vdev.get(), (size_t)na * 8, cudaMemcpyDeviceToHost,
-                             s));
-    KNB_CUDA(cudaStreamSynchronize(s));
     best = std::max(best, res.value);
-    solved.push_back(std::move(sol));
+    solved.push_back({res.value, blk.get(), na});
   }
-  std::vector<double> auth(n, 0.0);
+  // The tied blocks' authorities, each block's vector v weighted by v . s, and
+  // the hubs A a; clamped and rescaled where they are, one copy each to the
+  // host (on host vectors this took 10 of 16 ms of a call on R-MAT 20).
+  const unsigned gv = grid_for(n, VB_T, 148 * 8);
+  LzBuffers::grow(plan.lz.st, 1);
+  LzBuffers::grow(plan.lz.part, std::max<size_t>((size_t)gv * 3, 3 * ((size_t)n / VB + 1)) + 64);
+  LzState* st = plan.lz.st.get();
+  double* part = plan.lz.part.get();
+  double* auth = plan.auth.get();
+  double* hubs = plan.hubs.get();
+  KNB_CUDA(cudaMemsetAsync(st, 0, sizeof(LzState), s));
+  KNB_CUDA(cudaMemsetAsync(auth, 0, (size_t)n * 8, s));
   int tied = 0;
   for (const Solved& sol : solved) {
     if (sol.value < best * (1.0 - TIE)) continue;
     ++tied;
-    double weight = 0.0;
-    for (size_t i = 0; i < sol.v.size(); ++i) weight += sol.v[i] * (*sol.sv)[i];
-    for (size_t i = 0; i < ba[sol.b].size(); ++i) auth[ba[sol.b][i]] = sol.v[i] * weight;
+    lz_dots<<<(unsigned)((sol.na + VB - 1) / VB), VB_T, 0, s>>>(
+        sol.blk->v.get(), sol.blk->sdev.get(), sol.na, part, st);
+    scatter_by_dot<<<grid_for(sol.na, 256), 256, 0, s>>>(sol.blk->auths.get(), sol.na,
+                                                         sol.blk->v.get(), st, auth);
   }
-  // hubs = A auth (device product)
-  DevBuf<double> ad(n), hd(n);
-  KNB_CUDA(cudaMemcpyAsync(ad.get(), auth.data(), (size_t)n * 8, cudaMemcpyHostToDevice, s));
   DevOp full;
   full.n = A.n;
   full.nnz = A.nnz;
@@ -2071,17 +2113,29 @@ void hits(GraphHandleImpl& g, const HitsParams& p, double* hubs_out, double* aut
   full.cols = A.rows->tgt.get();
   full.v64 = A.has_vals ? A.vals64.get() : nullptr;
   full.part = &A.partition(EIG_TILE, s);
-  SpmvScratch sc;
-  spmv(full, ad.get(), nullptr, hd.get(), sc, nullptr, s);
-  std::vector<double> hubs(n);
-  KNB_CUDA(cudaMemcpyAsync(hubs.data(), hd.get(), (size_t)n * 8, cudaMemcpyDeviceToHost, s));
+  spmv(full, auth, nullptr, hubs, plan.sc, nullptr, s);
+  for (double* x : {auth, hubs}) {
+    clamp_stats<<<gv, VB_T, 0, s>>>(x, n, part, st);
+    scale_by_stats<<<gv, VB_T, 0, s>>>(x, n, st, p.scale);
+  }
+  KNB_LAUNCH("hub and authority scores");
+  KNB_CUDA(cudaMemcpyAsync(hubs_out, hubs, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
+  KNB_CUDA(cudaMemcpyAsync(auth_out, auth, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
-  hits_rescale(auth, p.scale);
-  hits_rescale(hubs, p.scale);
-  memcpy(hubs_out, hubs.data(), (size_t)n * 8);
-  memcpy(auth_out, auth.data(), (size_t)n * 8);
   *value = best;
   *unique = tied == 1 ? 1 : 0;
+}
+
+// x (n values, device) over its Euclidean length, unless that is 0; part holds
+// at least 3 values for each 4096 of x and 3 more, st one LzState.
+size_t normalize_scratch(size_t n) { return 3 * (n / VB + 1) * sizeof(double) + sizeof(LzState); }
+void normalize_length(double* x, size_t n, void* scratch, cudaStream_t s) {
+  LzState* st = static_cast<LzState*>(scratch);
+  double* part = reinterpret_cast<double*>(st + 1);
+  KNB_CUDA(cudaMemsetAsync(st, 0, sizeof(LzState), s));
+  lz_dots<<<(unsigned)((n + VB - 1) / VB), VB_T, 0, s>>>(x, nullptr, n, part, st);
+  scale_by_state<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(x, n, st, 1);
+  KNB_LAUNCH("normalize_length");
 }
 
 // ======================================================================= driver

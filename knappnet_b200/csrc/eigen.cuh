@@ -76,6 +76,11 @@ bool symmetric_eigen_device(const double* a, int n, double* vals, double* vecs, 
 void leading_eigen(GraphHandleImpl& g, bool weighted, int64_t* membership, double* q,
                    int64_t* splits, int* launches, cudaStream_t s);
 
+// x (n values, device) over its Euclidean length (unless that is 0), with
+// normalize_scratch(n) bytes of device scratch.
+size_t normalize_scratch(size_t n);
+void normalize_length(double* x, size_t n, void* scratch, cudaStream_t s);
+
 // FP64 products y = A x on merge-path warp tiles over the rows of `v`
 // (offsets from 0) with the partition build_partition makes for
 // product_tile() items per tile; the scratch grows on first use.

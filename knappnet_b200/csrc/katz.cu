@@ -377,18 +377,23 @@ __global__ void dense_back(const double* a, double* x, uint32_t n, const DenseSt
 }
 
 // ----------------------------------------------------------------- host parts
-template <class Epi>
-void sweep(const OpView<double>& v, const Partition& P, const double* x, const Epi& e,
+// One sweep on a persistent grid of the CTAs that fit at once (48 warps per
+// SM), each warp taking tile after tile. MT: FP32 arc values where all are
+// exact there (8 bytes less per arc).
+template <class MT, class Epi>
+void sweep(const OpView<MT>& v, const Partition& P, const double* x, const Epi& e,
            double* carry, double* head, double* part1, double* part2, IterState* st,
            cudaStream_t s) {
   constexpr size_t smem = warp_smem_bytes<double, K_IPT, K_WPB>();
-  const unsigned grid = (P.ntiles + K_WPB - 1) / K_WPB;
-  fit_warp_carveout<double, double, Epi, K_IPT, K_WPB>();
-  warp_spmv<double, double, Epi, K_IPT, K_WPB><<<grid, K_WPB * 32, smem, s>>>(
+  const unsigned grid = std::min((P.ntiles + K_WPB - 1) / K_WPB,
+                                 148u * (unsigned)warp_min_blocks<double, K_IPT, K_WPB>());
+  fit_warp_carveout<double, MT, Epi, K_IPT, K_WPB>();
+  warp_spmv<double, MT, Epi, K_IPT, K_WPB><<<grid, K_WPB * 32, smem, s>>>(
       v, x, e, P.coords.get(), P.ntiles, carry, head, part1, st, 0xFFFFFFFFu);
   KNB_LAUNCH("series sweep");
   split_rows<double, Epi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(
-      P.split.get(), P.nsplit, P.nshort, carry, head, e, part1, P.ntiles, part2, st);
+      P.split.get(), P.nsplit, P.nshort, carry, head, e, part1,
+      std::min<uint32_t>(P.ntiles, grid * K_WPB), part2, st);
   KNB_LAUNCH("series split rows");
 }
 
@@ -607,7 +612,7 @@ const double* series(const Operator& op, const double* d_b, double t, double q, 
   is.tol = tol;
   is.max_iter = (int32_t)std::min<int64_t>(max_iter, INT32_MAX);
   KNB_CUDA(cudaMemcpyAsync(sc.st.get(), &is, sizeof(is), cudaMemcpyHostToDevice, s));
-  const OpView<double> v = op.view64();
+  const bool f32 = op.has_vals && op.vals32_exact;
   SeriesEpi e;
   e.b = d_b;
   e.t = t;
@@ -617,8 +622,12 @@ const double* series(const Operator& op, const double* d_b, double t, double q, 
     for (int k = 0; k < 8; ++k) {
       e.x_old = xb[k & 1].get();
       e.y_new = xb[1 - (k & 1)].get();
-      sweep(v, P, xb[k & 1].get(), e, sc.carry.get(), sc.head.get(), sc.part1.get(),
-            sc.part2.get(), sc.st.get(), s);
+      if (f32)
+        sweep(op.view32(), P, xb[k & 1].get(), e, sc.carry.get(), sc.head.get(), sc.part1.get(),
+              sc.part2.get(), sc.st.get(), s);
+      else
+        sweep(op.view64(), P, xb[k & 1].get(), e, sc.carry.get(), sc.head.get(), sc.part1.get(),
+              sc.part2.get(), sc.st.get(), s);
     }
     KNB_CUDA(cudaMemcpyAsync(&hs, sc.st.get(), sizeof(hs), cudaMemcpyDeviceToHost, s));
     KNB_CUDA(cudaStreamSynchronize(s));
@@ -637,7 +646,7 @@ double seconds_since(std::chrono::steady_clock::time_point t0) {
 
 }  // namespace
 
-void katz(GraphHandleImpl& g, double alpha, const std::vector<double>& beta, bool normalized,
+void katz(GraphHandleImpl& g, double alpha, const double* beta, bool uniform, bool normalized,
           const SeriesParams& p, double* out, SeriesResult* r, cudaStream_t s) {
   const auto t0 = std::chrono::steady_clock::now();
   const uint32_t n = g.n;
@@ -649,18 +658,22 @@ void katz(GraphHandleImpl& g, double alpha, const std::vector<double>& beta, boo
                                : 0.0;
   r->radius = alpha > 0.0 ? q / alpha : 0.0;
   DevBuf<double> b(n), xb[2] = {DevBuf<double>(n), DevBuf<double>(n)};
-  KNB_CUDA(cudaMemcpyAsync(b.get(), beta.data(), (size_t)n * 8, cudaMemcpyHostToDevice, s));
-  const double* x = series(op, b.get(), alpha, q, p.tol, p.max_iter, "Katz centrality", xb,
-                           &r->iterations, s);
-  KNB_CUDA(cudaMemcpyAsync(out, x, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaStreamSynchronize(s));
-  if (normalized) {
-    double ss = 0.0;
-    for (uint32_t i = 0; i < n; ++i) ss += out[i] * out[i];
-    const double norm = std::sqrt(ss);
-    if (norm > 0.0)
-      for (uint32_t i = 0; i < n; ++i) out[i] /= norm;
+  if (uniform) {
+    fill_d<<<grid_for(n, KT), KT, 0, s>>>(b.get(), n, beta[0]);
+    KNB_LAUNCH("fill_d");
+  } else {
+    KNB_CUDA(cudaMemcpyAsync(b.get(), beta, (size_t)n * 8, cudaMemcpyHostToDevice, s));
   }
+  const double* xs = series(op, b.get(), alpha, q, p.tol, p.max_iter, "Katz centrality", xb,
+                            &r->iterations, s);
+  DevBuf<unsigned char> scratch;
+  if (normalized) {  // xs is one of xb, which are ours
+    double* x = xs == xb[0].get() ? xb[0].get() : xb[1].get();
+    scratch.alloc(normalize_scratch(n));
+    normalize_length(x, n, scratch.get(), s);
+  }
+  KNB_CUDA(cudaMemcpyAsync(out, xs, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
+  KNB_CUDA(cudaStreamSynchronize(s));
   r->seconds = seconds_since(t0);
 }
 

@@ -25,9 +25,9 @@ struct SeriesResult {
   int kernel_launches = 0;
 };
 
-// Katz centrality x = alpha A x + beta (spectral.rs:365-407); beta holds 1
-// or n values. Writes n scores to host `out`. Throws knb::Error.
-void katz(GraphHandleImpl& g, double alpha, const std::vector<double>& beta, bool normalized,
+// Katz centrality x = alpha A x + beta (spectral.rs:365-407); beta (host) holds
+// one value (uniform) or n. Writes n scores to host `out`. Throws knb::Error.
+void katz(GraphHandleImpl& g, double alpha, const double* beta, bool uniform, bool normalized,
           const SeriesParams& p, double* out, SeriesResult* r, cudaStream_t s);
 
 // Bonacich power centrality (spectral.rs:596-655): (I - exponent A)^-1 A 1,
