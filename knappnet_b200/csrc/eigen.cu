@@ -1407,12 +1407,13 @@ struct DevOp {
   const uint32_t* cols = nullptr;
   const double* v64 = nullptr;
   const float* v32 = nullptr;
-  const Partition* part = nullptr;
+  const Partition* part = nullptr;    // tiles of EIG_TILE items
+  const Partition* part32 = nullptr;  // tiles of EIG_TILE32, where FP32 products run
   // owned storage for submatrices
   DevBuf<uint32_t> own_off, own_cols;
   DevBuf<double> own_v64;
   DevBuf<float> own_v32;
-  std::unique_ptr<Partition> own_part;
+  std::unique_ptr<Partition> own_part, own_part32;
   OpView<double> view64() const { return {n, nnz, off, cols, v64}; }
   OpView<float> view32() const { return {n, nnz, off, cols, v32}; }
 };
@@ -1432,9 +1433,13 @@ struct SpmvScratch {
   }
 };
 
-constexpr int EIG_IPT = 8;
-constexpr int EIG_WPB = 16;                      // warps per CTA of the product
-constexpr uint32_t EIG_TILE = 32u * EIG_IPT;     // merge items per warp tile
+// Items per lane of a warp tile: 8 in FP32 and 4 in FP64, which both keep 48
+// warps per SM resident (8 FP64 items need registers for 16 warps only: an
+// FP64 product on symmetrised R-MAT 20 took 199 us, 136 us with 4).
+constexpr int EIG_IPT = 4, EIG_IPT32 = 8;
+constexpr int EIG_WPB = 16;                        // warps per CTA of the product
+constexpr uint32_t EIG_TILE = 32u * EIG_IPT;       // merge items per warp tile
+constexpr uint32_t EIG_TILE32 = 32u * EIG_IPT32;   // ... of FP32 products
 
 // One product with epilogue e: merge-path warp tiles (warp_spmv) on a
 // persistent grid of the CTAs that fit at once, then split_rows for the rows
@@ -1500,15 +1505,15 @@ constexpr double FP32_FLOOR = 1e-5;
 // y = A x (FP64 or, with x32 given, FP32 products accumulated in FP32).
 static int spmv(const DevOp& A, const double* x, const float* x32, double* y, SpmvScratch& sc,
                 const IterState* ist, cudaStream_t s) {
-  const Partition& P = *A.part;
-  sc.ensure(P.ntiles);
+  sc.ensure(A.part->ntiles);
   if (x32) {
     PlainEpi<float> e{y};
-    eig_product<float, float>(A.view32(), x32, e, P, sc.carry32.get(), sc.head32.get(),
-                              sc.part1.get(), sc.part2.get(), ist, s);
+    eig_product<float, float, PlainEpi<float>, EIG_IPT32>(
+        A.view32(), x32, e, *A.part32, sc.carry32.get(), sc.head32.get(), sc.part1.get(),
+        sc.part2.get(), ist, s);
   } else {
     PlainEpi<double> e{y};
-    eig_product<double, double>(A.view64(), x, e, P, sc.carry64.get(), sc.head64.get(),
+    eig_product<double, double>(A.view64(), x, e, *A.part, sc.carry64.get(), sc.head64.get(),
                                 sc.part1.get(), sc.part2.get(), ist, s);
   }
   KNB_LAUNCH("spmv");
@@ -2376,6 +2381,7 @@ void eigenvector(GraphHandleImpl& g, const EigenParams& p, double* out, EigenRes
         A.v64 = op.has_vals ? op.vals64.get() : nullptr;
         A.v32 = op.has_vals ? op.vals32.get() : nullptr;
         A.part = &op.partition(EIG_TILE, s);
+        if (p.precision == 1) A.part32 = &op.partition(EIG_TILE32, s);
       } else if (build_sub) {
         const uint32_t* nodes_d = plan.members_d.get() + start[c];
         scatter_local<<<grid_for(kn, 256), 256, 0, s>>>(nodes_d, kn, local.get());
@@ -2402,6 +2408,10 @@ void eigenvector(GraphHandleImpl& g, const EigenParams& p, double* out, EigenRes
         A.v32 = op.has_vals ? A.own_v32.get() : nullptr;
         A.own_part = build_partition(kn, nnz, A.off, EIG_TILE, s);
         A.part = A.own_part.get();
+      }
+      if (k != 1 && p.precision == 1 && !A.part32) {
+        A.own_part32 = build_partition(kn, A.nnz, A.off, EIG_TILE32, s);
+        A.part32 = A.own_part32.get();
       }
       Solved sv;
       sv.c = c;
