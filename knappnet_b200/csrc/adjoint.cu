@@ -324,7 +324,6 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
   constexpr size_t smem = warp_smem_bytes<double, IPT, WPB>();
   const unsigned grid =
       std::min((P.ntiles + WPB - 1) / WPB, 148u * (unsigned)warp_min_blocks<double, IPT, WPB>());
-  const uint32_t npart = std::min<uint32_t>(P.ntiles, grid * WPB);
   const OpView<double> v = tr->view64();
   fit_warp_carveout<double, double, AdjointEpi, IPT, WPB>();
   fit_warp_carveout<double, double, RowSumEpi, IPT, WPB>();
@@ -347,12 +346,12 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
       e.jump = jump;
       e.d = prm.damping;
       e.pu = 1.0 / n;
-      warp_spmv<double, double, AdjointEpi, IPT, WPB><<<grid, WPB * 32, smem, s>>>(
-          v, buffer(k), e, P.coords.get(), P.ntiles, W.carry.get(), W.head.get(), W.part1.get(),
-          st, 0xFFFFFFFFu);
-      split_rows<double, AdjointEpi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(
-          P.split.get(), P.nsplit, P.nshort, W.carry.get(), W.head.get(), e, W.part1.get(), npart,
-          W.part2.get(), st);
+      launch_chained(warp_spmv<double, double, AdjointEpi, IPT, WPB>, grid, WPB * 32, smem, s, v,
+                     buffer(k), e, P.coords.get(), P.ntiles, W.carry.get(), W.head.get(),
+                     W.part1.get(), st, 0xFFFFFFFFu);
+      launch_chained(split_rows<double, AdjointEpi>, split_grid(P.nsplit, P.nshort, grid),
+                     SPMV_THREADS, 0, s, P.split.get(), P.nsplit, P.nshort, W.carry.get(),
+                     W.head.get(), e, W.part1.get(), grid, W.part2.get(), st);
       launches += 2;
       if ((k + 1) % CYCLE == 0) {
         adj_extrapolate<<<gv, 256, 0, s>>>(W.lam[2].get(), W.lam[3].get(), buffer(k),
@@ -388,12 +387,12 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
   // (M^T lambda)_j numerators with the final lambda, then the edge gradients
   {
     RowSumEpi e{W.r.get()};
-    warp_spmv<double, double, RowSumEpi, IPT, WPB><<<grid, WPB * 32, smem, s>>>(
-        v, lam_final, e, P.coords.get(), P.ntiles, W.carry.get(), W.head.get(), W.part1.get(),
-        nullptr, 0xFFFFFFFFu);
-    split_rows<double, RowSumEpi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(
-        P.split.get(), P.nsplit, P.nshort, W.carry.get(), W.head.get(), e, W.part1.get(), npart,
-        W.part2.get(), nullptr);
+    launch_chained(warp_spmv<double, double, RowSumEpi, IPT, WPB>, grid, WPB * 32, smem, s, v,
+                   lam_final, e, P.coords.get(), P.ntiles, W.carry.get(), W.head.get(),
+                   W.part1.get(), nullptr, 0xFFFFFFFFu);
+    launch_chained(split_rows<double, RowSumEpi>, split_grid(P.nsplit, P.nshort, grid),
+                   SPMV_THREADS, 0, s, P.split.get(), P.nsplit, P.nshort, W.carry.get(),
+                   W.head.get(), e, W.part1.get(), grid, W.part2.get(), nullptr);
     adj_node_terms<<<grid_for(n, 256), 256, 0, s>>>(d_x, fwd->inv_out64.get(), W.r.get(), n,
                                                     prm.damping, W.terms.get());
     if (g.m)

@@ -607,6 +607,7 @@ inline unsigned project_groups(int k, int mode) {
 __global__ void __launch_bounds__(VB_T)
 lz_project(const double* __restrict__ V, size_t dim, int lo, int hi, const double* __restrict__ w,
            int mode, double* __restrict__ part, LzState* st, const IterState* ist) {
+  chain_wait();
   if (ist && iteration_done(ist)) return;
   if (mode == 2 && !st->need2) return;
   const int K = hi - lo, slots = lz_project_slots(K, mode);
@@ -671,6 +672,7 @@ lz_project(const double* __restrict__ V, size_t dim, int lo, int hi, const doubl
 __global__ void __launch_bounds__(VB_T)
 lz_subtract(const double* __restrict__ V, size_t dim, int lo, int hi, double* __restrict__ w,
             int mode, double* __restrict__ part, LzState* st, const IterState* ist) {
+  chain_wait();
   if (ist && iteration_done(ist)) return;
   if (mode == 2 && !st->need2) return;
   const int K = hi - lo;
@@ -740,6 +742,7 @@ lz_subtract(const double* __restrict__ V, size_t dim, int lo, int hi, double* __
 
 // Start of a step: zero the coefficients.
 __global__ void lz_begin(LzState* st, const IterState* ist) {
+  chain_wait();
   if (ist && iteration_done(ist)) return;
   if (threadIdx.x < MAXB) st->coef[threadIdx.x] = 0.0;
   if (threadIdx.x == 0) st->need2 = 0;
@@ -748,6 +751,7 @@ __global__ void lz_begin(LzState* st, const IterState* ist) {
 // End of a step: coefficients into the projected matrix, beta, breakdown
 // (eigenvector.rs:786-796).
 __global__ void lz_end(LzState* st, IterState* ist, double* hm, int m, int j) {
+  chain_wait();
   if (iteration_done(ist)) return;
   if (threadIdx.x < j + 1) {
     hm[threadIdx.x * m + j] = st->coef[threadIdx.x];
@@ -769,6 +773,7 @@ __global__ void lz_end(LzState* st, IterState* ist, double* hm, int m, int j) {
 __global__ void lz_next(double* __restrict__ V, size_t dim, int col, const double* __restrict__ w,
                         float* __restrict__ v32, double* hm, int m, const LzState* st,
                         const IterState* ist, int set_hm) {
+  chain_wait();
   if (ist && iteration_done(ist)) return;
   const double beta = st->beta;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < dim;
@@ -1470,12 +1475,11 @@ static void eig_product(const OpView<MT>& v, const VT* x, const Epi& e, const Pa
     cap = it->second;
   }
   const unsigned grid = std::max(1u, std::min((P.ntiles + EIG_WPB - 1) / EIG_WPB, cap));
-  const uint32_t npart = std::min<uint32_t>(P.ntiles, grid * EIG_WPB);
-  fnp<<<grid, EIG_WPB * 32, smem, s>>>(v, x, e, P.coords.get(), P.ntiles, carry, head, part1, st,
-                                      0u);
-  split_rows<VT, Epi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(P.split.get(), P.nsplit, P.nshort,
-                                                          carry, head, e, part1, npart, part2,
-                                                          const_cast<IterState*>(st));
+  launch_chained(fnp, grid, EIG_WPB * 32, smem, s, v, x, e, P.coords.get(), P.ntiles, carry, head,
+                 part1, st, 0u);
+  launch_chained(split_rows<VT, Epi>, split_grid(P.nsplit, P.nshort, grid), SPMV_THREADS, 0, s,
+                 P.split.get(), P.nsplit, P.nshort, carry, head, e, part1, grid, part2,
+                 const_cast<IterState*>(st));
 }
 // FP64 products for row shards of PageRank (shard.cu): the same warp tiles
 // and split-row pass over a view whose offsets start at 0, with 4 items per
@@ -1648,21 +1652,21 @@ static bool symmetric_leading(const DevOp& A, double tol, double shift, int64_t 
           break;
         }
         const double* vj = V.get() + (size_t)jj * dim;
-        lz_begin<<<1, 32, 0, s>>>(st.get(), ist.get());
+        launch_chained(lz_begin, 1, 32, 0, s, st.get(), ist.get());
         *launches += 1 + apply(vj, use32 ? v32.get() : nullptr, w.get(), ist.get());
         const int cols = jj + 1, lo = cols >= 2 ? cols - 2 : 0;
-        const dim3 local(nb, project_groups(cols - lo, 0)), full(nb, project_groups(cols, 1));
-        lz_project<<<local, VB_T, 0, s>>>(V.get(), dim, lo, cols, w.get(), 0, part.get(), st.get(), ist.get());
-        lz_subtract<<<nb, VB_T, 0, s>>>(V.get(), dim, lo, cols, w.get(), 0, part.get(), st.get(), ist.get());
-        lz_project<<<full, VB_T, 0, s>>>(V.get(), dim, 0, cols, w.get(), 1, part.get(), st.get(), ist.get());
-        lz_subtract<<<nb, VB_T, 0, s>>>(V.get(), dim, 0, cols, w.get(), 1, part.get(), st.get(), ist.get());
-        lz_project<<<full, VB_T, 0, s>>>(V.get(), dim, 0, cols, w.get(), 2, part.get(), st.get(), ist.get());
-        lz_subtract<<<nb, VB_T, 0, s>>>(V.get(), dim, 0, cols, w.get(), 2, part.get(), st.get(), ist.get());
-        lz_end<<<1, 32, 0, s>>>(st.get(), ist.get(), hm_d.get(), m, jj);
+        for (int mode = 0; mode < 3; ++mode) {
+          const int from = mode == 0 ? lo : 0;
+          launch_chained(lz_project, dim3(nb, project_groups(cols - from, mode)), VB_T, 0, s,
+                         V.get(), dim, from, cols, w.get(), mode, part.get(), st.get(), ist.get());
+          launch_chained(lz_subtract, nb, VB_T, 0, s, V.get(), dim, from, cols, w.get(), mode,
+                         part.get(), st.get(), ist.get());
+        }
+        launch_chained(lz_end, 1, 32, 0, s, st.get(), ist.get(), hm_d.get(), m, jj);
         *launches += 7;
         if (jj < jc) {
-          lz_next<<<gv, 256, 0, s>>>(V.get(), dim, jj + 1, w.get(), use32 ? v32.get() : nullptr,
-                                     hm_d.get(), m, st.get(), ist.get(), 1);
+          launch_chained(lz_next, gv, 256, 0, s, V.get(), dim, jj + 1, w.get(),
+                         use32 ? v32.get() : nullptr, hm_d.get(), m, st.get(), ist.get(), 1);
           ++*launches;
         }
       }

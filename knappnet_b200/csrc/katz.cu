@@ -388,13 +388,10 @@ void sweep(const OpView<MT>& v, const Partition& P, const double* x, const Epi& 
   const unsigned grid = std::min((P.ntiles + K_WPB - 1) / K_WPB,
                                  148u * (unsigned)warp_min_blocks<double, K_IPT, K_WPB>());
   fit_warp_carveout<double, MT, Epi, K_IPT, K_WPB>();
-  warp_spmv<double, MT, Epi, K_IPT, K_WPB><<<grid, K_WPB * 32, smem, s>>>(
-      v, x, e, P.coords.get(), P.ntiles, carry, head, part1, st, 0xFFFFFFFFu);
-  KNB_LAUNCH("series sweep");
-  split_rows<double, Epi><<<SPLIT_CTAS, SPMV_THREADS, 0, s>>>(
-      P.split.get(), P.nsplit, P.nshort, carry, head, e, part1,
-      std::min<uint32_t>(P.ntiles, grid * K_WPB), part2, st);
-  KNB_LAUNCH("series split rows");
+  launch_chained(warp_spmv<double, MT, Epi, K_IPT, K_WPB>, grid, K_WPB * 32, smem, s, v, x, e,
+                 P.coords.get(), P.ntiles, carry, head, part1, st, 0xFFFFFFFFu);
+  launch_chained(split_rows<double, Epi>, split_grid(P.nsplit, P.nshort, grid), SPMV_THREADS, 0, s,
+                 P.split.get(), P.nsplit, P.nshort, carry, head, e, part1, grid, part2, st);
 }
 
 struct Scratch {

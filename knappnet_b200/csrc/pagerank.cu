@@ -4,8 +4,8 @@
 // One sweep is two kernels: the sparse product with the PageRank update
 // fused into its epilogue (by default the sliced sweep slice_spmv, else a
 // merge-path kernel, with PagerankEpi) and the split-row / reduction kernel
-// (split_rows). A third, normally idle, kernel computes the exact L1 change
-// when the fused estimate is too close to the tolerance.
+// (split_rows), whose last CTA also computes the exact L1 change when the
+// fused estimate is too close to the tolerance.
 //
 // Normalisation is folded into the next sweep. The device stores the
 // unnormalised iterate y_k and z_k = y_k / out (0 for dangling nodes); with
@@ -18,7 +18,7 @@
 // sum |u_i - x_k,i| instead, which differs from it by at most |1 - T_{k+1}|
 // (T is 1 up to rounding since the transition matrix is column
 // stochastic). When the estimate is within that bound of the tolerance, the
-// exact change is computed by pr_exact_change before deciding.
+// exact change is computed before deciding.
 //
 // Mixed precision runs the same trajectory: FP32 sweeps (FP32 arc values,
 // iterate and row sums; FP64 reductions) from the uniform start, then one
@@ -46,6 +46,7 @@ template <class VT, bool PV, bool JU, bool EXACT>
 struct PagerankEpi {
   static constexpr int NACC = 3;
   static constexpr bool SUMS = true;  // total, dangling mass, change
+  static constexpr bool DECIDES = EXACT;
   const VT* y_old;
   VT* y_new;
   VT* z_new;
@@ -53,6 +54,7 @@ struct PagerankEpi {
   const double* p;  // personalization (rescaled), when PV
   double d;
   double pu;        // 1 / n
+  uint32_t n;
   VT c_it = 0, c_dt = 0;
 
   __device__ __forceinline__ void prepare(const IterState* st) {
@@ -88,6 +90,11 @@ struct PagerankEpi {
     row_in(g, s, fetch(g), a);
   }
 
+  // |x_new - x_old| of node i once the total T is known (y_new comes from
+  // other CTAs, past L1)
+  __device__ __forceinline__ double exact_change(uint32_t i, double T, double ip) const {
+    return fabs((double)__ldcg(y_new + i) / T - (double)y_old[i] * ip);
+  }
   __device__ void finish(IterState* st, const double* tot) const {
     const double T = tot[0], D = tot[1], ch = tot[2];
     st->prev_inv_total = st->inv_total;
@@ -123,6 +130,7 @@ template <class VT, bool ANCHOR, bool PV, bool JU, bool EXACT>
 struct RefineEpi {
   static constexpr int NACC = 3;
   static constexpr bool SUMS = true;
+  static constexpr bool DECIDES = EXACT;
   const double* y_ref;
   double* s_ref;        // written by the anchor sweep, read by refinement sweeps
   const float* e_old;   // refinement sweeps: e of the input iterate
@@ -132,6 +140,7 @@ struct RefineEpi {
   const double* p;
   double d;
   double pu;
+  uint32_t n;
   double c_it = 0, c_dt = 0;
 
   __device__ __forceinline__ void prepare(const IterState* st) {
@@ -183,6 +192,11 @@ struct RefineEpi {
     row_in(g, s_in, fetch(g), a);
   }
 
+  __device__ __forceinline__ double exact_change(uint32_t i, double T, double ip) const {
+    const double yr = y_ref[i];
+    const double yo = ANCHOR ? yr : yr + (double)e_old[i];
+    return fabs((yr + (double)__ldcg(e_new + i)) / T - yo * ip);
+  }
   __device__ void finish(IterState* st, const double* tot) const {
     PagerankEpi<double, PV, JU, EXACT> base;
     base.finish(st, tot);
@@ -244,59 +258,6 @@ __global__ void pr_init(VT* __restrict__ y, VT* __restrict__ z, const VT* __rest
     st->total = r[0];
     st->prev_inv_total = 1.0;
     st->ticket = 0;
-  }
-}
-
-// Exact L1 change sum |y_new / T - y_old * prev_inv_total| when the fused
-// estimate cannot decide (see the file comment).
-__global__ void pr_exact_change(const double* __restrict__ y_old, const double* __restrict__ y_new,
-                                uint32_t n, double* __restrict__ part, IterState* st) {
-  if (!st->ambiguous || st->converged || st->stopped) return;
-  __shared__ double sh[VT_THREADS / 32];
-  const double T = st->total, ip = st->prev_inv_total;
-  double a = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    a += fabs(y_new[i] / T - y_old[i] * ip);
-  a = block_sum(a, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = a;
-  if (!last_block(&st->ticket2)) return;
-  double r[1];
-  reduce_parts<1>(part, gridDim.x, r, sh);
-  if (threadIdx.x == 0) {
-    st->change = r[0];
-    st->ambiguous = 0;
-    if (r[0] <= st->tol) st->converged = 1;
-    else if (st->iter >= st->max_iter) st->stopped = 1;
-    st->ticket2 = 0;
-  }
-}
-
-// The exact change for refinement sweeps, whose iterates are y_ref + e
-// (e_old null: the anchor sweep, whose input iterate is y_ref itself).
-__global__ void pr_exact_change_ref(const double* __restrict__ y_ref,
-                                    const float* __restrict__ e_old,
-                                    const float* __restrict__ e_new, uint32_t n,
-                                    double* __restrict__ part, IterState* st) {
-  if (!st->ambiguous || st->converged || st->stopped) return;
-  __shared__ double sh[VT_THREADS / 32];
-  const double T = st->total, ip = st->prev_inv_total;
-  double a = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double yr = y_ref[i];
-    const double yo = e_old ? yr + (double)e_old[i] : yr;
-    a += fabs((yr + (double)e_new[i]) / T - yo * ip);
-  }
-  a = block_sum(a, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = a;
-  if (!last_block(&st->ticket2)) return;
-  double r[1];
-  reduce_parts<1>(part, gridDim.x, r, sh);
-  if (threadIdx.x == 0) {
-    st->change = r[0];
-    st->ambiguous = 0;
-    if (r[0] <= st->tol) st->converged = 1;
-    else if (st->iter >= st->max_iter) st->stopped = 1;
-    st->ticket2 = 0;
   }
 }
 
@@ -616,8 +577,9 @@ static unsigned launch_slice(const SlicedOp& so, const VT* x, const Epi& e, VT* 
   const unsigned grid = slice_grid<VT, MT, Epi, U, WPB, HOT ? 1 : MINB, GNA>(smem);
   const uint64_t hot32 = hot_setting() >= 0 ? (uint64_t)hot_setting() : 49152u;
   const uint32_t l1_hot = (uint32_t)std::min<uint64_t>(hot32 * 4 / sizeof(VT), 0xFFFFFFFFull);
-  fnp<<<grid, WPB * 32, smem, s>>>(so.view<MT>(), x, e, carry, head, part1, st, l1_hot, smem_n);
-  return grid * WPB;
+  launch_chained(fnp, grid, WPB * 32, smem, s, so.view<MT>(), x, e, carry, head, part1, st, l1_hot,
+                 smem_n);
+  return grid;
 }
 
 // Bulk-staged sliced sweeps (bulk.cuh): U arc positions per chunk, S stages
@@ -670,7 +632,7 @@ static unsigned launch_slice_bulk(const SlicedOp& so, const VT* x, const Epi& e,
 template <class VT, class MT, class Epi, int VAR, int IPT>
 static void launch_spmv(const Operator& op, const Partition& P, const OpView<MT>& v,
                         const VT* x, const Epi& e, VT* carry, VT* head, double* part1,
-                        double* part2, IterState* st, cudaStream_t s, unsigned g2,
+                        double* part2, IterState* st, cudaStream_t s,
                         cudaEvent_t ev0, cudaEvent_t ev1, const SlicedOp* so = nullptr) {
   if (ev0) KNB_CUDA(cudaEventRecord(ev0, s));
   uint32_t npart = P.ntiles;  // partials the sweep leaves for split_rows
@@ -685,9 +647,9 @@ static void launch_spmv(const Operator& op, const Partition& P, const OpView<MT>
       KNB_LAUNCH("slice_spmv");
     }
     if (ev1) KNB_CUDA(cudaEventRecord(ev1, s));
-    split_rows<VT, Epi><<<g2, SPMV_THREADS, 0, s>>>(so->split.get(), so->nsplit, so->nshort,
-                                                     carry, head, e, part1, npart, part2, st);
-    KNB_LAUNCH("split_rows");
+    launch_chained(split_rows<VT, Epi>, split_grid(so->nsplit, so->nshort, npart), SPMV_THREADS, 0,
+                   s, so->split.get(), so->nsplit, so->nshort, carry, head, e, part1, npart, part2,
+                   st);
     return;
   } else if constexpr (VAR == VAR_HOT || VAR == VAR_HOT16) {
     constexpr int WPB = VAR == VAR_HOT ? 32 : 16;
@@ -760,22 +722,19 @@ static void launch_spmv(const Operator& op, const Partition& P, const OpView<MT>
     const uint32_t l1_hot = hot_setting() >= 0 ? (uint32_t)std::min<int64_t>(
                                                      hot_setting(), 0xFFFFFFFFll)
                                                : 24576u;
-    npart = std::min<uint32_t>(P.ntiles, grid * WPB);
-    warp_spmv<VT, MT, Epi, IPT, WPB, GNA><<<grid, WPB * 32, smem, s>>>(
-        v, x, e, P.coords.get(), P.ntiles, carry, head,
-        part1, st, l1_hot);
+    npart = grid;
+    launch_chained(fnp, grid, WPB * 32, smem, s, v, x, e, P.coords.get(), P.ntiles, carry, head,
+                   part1, st, l1_hot);
   }
   KNB_LAUNCH("sweep");
   if (ev1) KNB_CUDA(cudaEventRecord(ev1, s));
-  split_rows<VT, Epi><<<g2, SPMV_THREADS, 0, s>>>(P.split.get(), P.nsplit, P.nshort,
-                                                   carry, head, e,
-                                                   part1, npart, part2, st);
-  KNB_LAUNCH("split_rows");
+  launch_chained(split_rows<VT, Epi>, split_grid(P.nsplit, P.nshort, npart), SPMV_THREADS, 0, s,
+                 P.split.get(), P.nsplit, P.nshort, carry, head, e, part1, npart, part2, st);
 }
 
 template <class VT, class MT, bool PV, bool JU, bool EXACT, int VAR, int IPT>
 static void launch_sweep(const Operator& op, const Partition& P, const SweepBuffers& B, int buf,
-                         double d, cudaStream_t s, unsigned g2, cudaEvent_t ev0, cudaEvent_t ev1) {
+                         double d, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1) {
   using Epi = PagerankEpi<VT, PV, JU, EXACT>;
   Epi e;
   e.y_old = (const VT*)B.y[buf];
@@ -785,19 +744,15 @@ static void launch_sweep(const Operator& op, const Partition& P, const SweepBuff
   e.p = B.p;
   e.d = d;
   e.pu = 1.0 / (double)op.n;
+  e.n = op.n;
   OpView<MT> v;
   if constexpr (sizeof(MT) == 8) v = B.v64; else v = B.v32;
   launch_spmv<VT, MT, Epi, VAR, IPT>(op, P, v, (const VT*)B.z[buf], e, (VT*)B.carry,
-                                     (VT*)B.head, B.part1, B.part2, B.st, s, g2, ev0, ev1, B.so);
-  if (EXACT) {
-    pr_exact_change<<<grid_for(op.n, VT_THREADS, 1184), VT_THREADS, 0, s>>>(
-        (const double*)B.y[buf], (const double*)B.y[1 - buf], op.n, B.part3, B.st);
-    KNB_LAUNCH("pr_exact_change");
-  }
+                                     (VT*)B.head, B.part1, B.part2, B.st, s, ev0, ev1, B.so);
 }
 
 using SweepFn = void (*)(const Operator&, const Partition&, const SweepBuffers&, int, double,
-                         cudaStream_t, unsigned, cudaEvent_t, cudaEvent_t);
+                         cudaStream_t, cudaEvent_t, cudaEvent_t);
 
 template <class VT, class MT, bool EXACT, int VAR, int IPT>
 static SweepFn pick_pv(bool pv, bool ju) {
@@ -846,7 +801,7 @@ static SweepFn pick_kernel(int var, int ipt, bool pv, bool ju) {
 // B.y[1 - buf] and B.z[1 - buf] out; FP32 arc values.
 template <bool PV, bool JU, int VAR, int IPT>
 static void launch_refine(const Operator& op, const Partition& P, const SweepBuffers& B, int buf,
-                          double d, cudaStream_t s, unsigned g2, cudaEvent_t ev0,
+                          double d, cudaStream_t s, cudaEvent_t ev0,
                           cudaEvent_t ev1) {
   using Epi = RefineEpi<float, false, PV, JU, true>;
   Epi e;
@@ -859,12 +814,10 @@ static void launch_refine(const Operator& op, const Partition& P, const SweepBuf
   e.p = B.p;
   e.d = d;
   e.pu = 1.0 / (double)op.n;
+  e.n = op.n;
   launch_spmv<float, float, Epi, VAR, IPT>(op, P, B.v32, (const float*)B.z[buf], e,
                                            (float*)B.carry, (float*)B.head, B.part1, B.part2,
-                                           B.st, s, g2, ev0, ev1, B.so);
-  pr_exact_change_ref<<<grid_for(op.n, VT_THREADS, 1184), VT_THREADS, 0, s>>>(
-      B.y_ref, (const float*)B.y[buf], (const float*)B.y[1 - buf], op.n, B.part3, B.st);
-  KNB_LAUNCH("pr_exact_change_ref");
+                                           B.st, s, ev0, ev1, B.so);
 }
 
 // The anchor sweep: an FP64 sweep gathering z_ref = y_ref / out that keeps
@@ -873,7 +826,7 @@ static void launch_refine(const Operator& op, const Partition& P, const SweepBuf
 template <class MT, bool PV, bool JU, int VAR, int IPT>
 static void launch_anchor(const Operator& op, const Partition& P, const SweepBuffers& B,
                           const double* z_ref, double* carry64, double* head64, double d,
-                          cudaStream_t s, unsigned g2, cudaEvent_t ev0, cudaEvent_t ev1) {
+                          cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1) {
   using Epi = RefineEpi<double, true, PV, JU, true>;
   Epi e;
   e.y_ref = B.y_ref;
@@ -885,17 +838,15 @@ static void launch_anchor(const Operator& op, const Partition& P, const SweepBuf
   e.p = B.p;
   e.d = d;
   e.pu = 1.0 / (double)op.n;
+  e.n = op.n;
   OpView<MT> v;
   if constexpr (sizeof(MT) == 8) v = B.v64; else v = B.v32;
   launch_spmv<double, MT, Epi, VAR, IPT>(op, P, v, z_ref, e, carry64, head64, B.part1, B.part2,
-                                         B.st, s, g2, ev0, ev1, B.so);
-  pr_exact_change_ref<<<grid_for(op.n, VT_THREADS, 1184), VT_THREADS, 0, s>>>(
-      B.y_ref, nullptr, (const float*)B.y[0], op.n, B.part3, B.st);
-  KNB_LAUNCH("pr_exact_change_ref");
+                                         B.st, s, ev0, ev1, B.so);
 }
 
 using AnchorFn = void (*)(const Operator&, const Partition&, const SweepBuffers&, const double*,
-                          double*, double*, double, cudaStream_t, unsigned, cudaEvent_t,
+                          double*, double*, double, cudaStream_t, cudaEvent_t,
                           cudaEvent_t);
 
 // Refinement and anchor sweeps come in the warp-tile variants (4, 8 or 16
@@ -1001,11 +952,10 @@ struct PhaseResult {
 // one batch of `U` sweeps in flight ahead of the state it inspects, so the
 // GPU never waits for the host; sweeps after convergence exit at once.
 static PhaseResult run_phase(SweepFn fn, const Operator& op, const Partition& P,
-                             const SweepBuffers& B, double d, bool exact, cudaStream_t s,
+                             const SweepBuffers& B, double d, cudaStream_t s,
                              PrWorkspace& ws, IterState* h_state /* pinned, 2 slots */,
                              double* timing_ms, int64_t* timing_n, int32_t iter0 = 0) {
   const int U = 8;
-  const unsigned g2 = SPLIT_CTAS;
   PhaseResult r;
   int batch = 0;
   size_t nev = 0;
@@ -1017,8 +967,8 @@ static PhaseResult run_phase(SweepFn fn, const Operator& op, const Partition& P,
         e0 = ws.timing_event(nev++);
         e1 = ws.timing_event(nev++);
       }
-      fn(op, P, B, k & 1, d, s, g2, e0, e1);
-      r.launches += exact ? 3 : 2;
+      fn(op, P, B, k & 1, d, s, e0, e1);
+      r.launches += 2;
     }
     KNB_CUDA(cudaMemcpyAsync(&h_state[b & 1], B.st, sizeof(IterState), cudaMemcpyDeviceToHost, s));
     KNB_CUDA(cudaEventRecord(ws.done[b & 1], s));
@@ -1152,10 +1102,10 @@ static double time_candidate(Operator& op, const SweepPick& c, int cls, bool use
   // one untimed sweep, then the fastest of three timed ones (each between its
   // own events), which a passing disturbance of the GPU does not inflate
   constexpr int TIMED = 3;
-  fn(op, *P, B, 0, 0.85, s, SPLIT_CTAS, nullptr, nullptr);
+  fn(op, *P, B, 0, 0.85, s, nullptr, nullptr);
   for (int k = 0; k < TIMED; ++k) {
     KNB_CUDA(cudaEventRecord(ws.timing_event(2 * k), s));
-    fn(op, *P, B, (k + 1) & 1, 0.85, s, SPLIT_CTAS, nullptr, nullptr);
+    fn(op, *P, B, (k + 1) & 1, 0.85, s, nullptr, nullptr);
     KNB_CUDA(cudaEventRecord(ws.timing_event(2 * k + 1), s));
   }
   int32_t fault = 0;
@@ -1370,7 +1320,7 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
                    ws.head32.get(), ws.part1.get(), ws.part2.get(), ws.part3.get(), st};
     B.so = SO;
     SweepFn fn = pick_kernel<float, float, false>(var32, ipt32, pv, ju);
-    r32 = run_phase(fn, op, *P32, B, prm.damping, false, s, ws, hstate, &tms32, &tn32);
+    r32 = run_phase(fn, op, *P32, B, prm.damping, s, ws, hstate, &tms32, &tn32);
     launches += r32.launches;
     if (r32.stopped && !r32.converged)
       throw Error("PageRank did not converge to tolerance " + std::to_string(prm.tol) +
@@ -1404,10 +1354,10 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
       AnchorFn af = use32 ? pick_anchor<float>(var64, ipt64, pv, ju)
                           : pick_anchor<double>(var64, ipt64, pv, ju);
       af(op, *P64, R, ws.z64[0].get(), ws.carry64.get(), ws.head64.get(), prm.damping, s,
-         SPLIT_CTAS, g_timing_on ? ws.a0 : nullptr, g_timing_on ? ws.a1 : nullptr);
-      launches += 3;
+         g_timing_on ? ws.a0 : nullptr, g_timing_on ? ws.a1 : nullptr);
+      launches += 2;
       SweepFn fr = pick_refine(var_r, ipt_r, pv, ju);
-      r64 = run_phase(fr, op, *PR, R, prm.damping, true, s, ws, hstate, &tmsr, &tnr, 1);
+      r64 = run_phase(fr, op, *PR, R, prm.damping, s, ws, hstate, &tmsr, &tnr, 1);
       if (g_timing_on) {
         float ms = 0;
         KNB_CUDA(cudaEventElapsedTime(&ms, ws.a0, ws.a1));
@@ -1421,7 +1371,7 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
       B.so = SO;
       SweepFn fn = use32 ? pick_kernel<double, float, true>(var64, ipt64, pv, ju)
                          : pick_kernel<double, double, true>(var64, ipt64, pv, ju);
-      r64 = run_phase(fn, op, *P64, B, prm.damping, true, s, ws, hstate, &tms64, &tn64);
+      r64 = run_phase(fn, op, *P64, B, prm.damping, s, ws, hstate, &tms64, &tn64);
     }
     launches += r64.launches;
     if (!r64.converged)

@@ -23,7 +23,7 @@
 // Neither part uses shared memory, so L1 keeps the SM's whole 256 KB for the
 // gathers in flight and the most gathered values. The epilogue (PageRank
 // update, plain store) runs on every row, with coalesced accesses for the
-// slices, and reduces the epilogue's scalars to one partial per warp. Every
+// slices, and reduces the epilogue's scalars to one partial per CTA. Every
 // sum has a fixed association, so results are identical from run to run.
 #pragma once
 
@@ -109,8 +109,8 @@ __device__ __forceinline__ VT slice_long_sum(const SliceView<MT>& op, const VT* 
 }
 
 // One sweep: every warp first takes pieces t = global warp, + all warps,
-// then slices the same way, and leaves one partial of the epilogue's
-// scalars at part[global warp] (all warps of the grid write one). With
+// then slices the same way, and each CTA leaves one partial of the epilogue's
+// scalars at part[CTA]. With
 // smem_n > 0 each CTA first copies x[0, smem_n) (the most gathered values;
 // smem_n a multiple of 16 / sizeof(VT)) into shared memory, and gathers of
 // those columns read it there instead of sending a request to L1 and L2.
@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(WPB * 32, MINB)
 slice_spmv(SliceView<MT> op, const VT* __restrict__ xg, Epi epi_in, VT* __restrict__ carry,
            VT* __restrict__ head, double* __restrict__ part, const IterState* __restrict__ st,
            uint32_t l1_hot, uint32_t smem_n) {
+  chain_wait();
   if (st && iteration_done(st)) return;
   extern __shared__ __align__(16) unsigned char slice_smem[];
   const VT* hot = nullptr;
@@ -203,7 +204,7 @@ slice_spmv(SliceView<MT> op, const VT* __restrict__ xg, Epi epi_in, VT* __restri
       else epi.row(r, s, acc);
     }
   }
-  warp_store_partials<Epi>(acc, part, gw, lane);
+  cta_store_partials<Epi, WPB>(acc, part, threadIdx.x >> 5, lane);
 }
 
 }  // namespace knb

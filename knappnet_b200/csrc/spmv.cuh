@@ -28,6 +28,8 @@
 // by rounding).
 #pragma once
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace knb {
@@ -366,6 +368,23 @@ __device__ __forceinline__ void warp_store_partials(const double* a, double* __r
   }
 }
 
+// One partial per CTA: its warps' scalars added in warp order.
+template <class Epi, int WPB>
+__device__ __forceinline__ void cta_store_partials(const double* a, double* __restrict__ part,
+                                                   int warp, int lane) {
+  constexpr int NA = Epi::NACC;
+  if constexpr (NA > 0) {
+    __shared__ double sh[WPB * NA];
+    warp_store_partials<Epi>(a, sh, (uint32_t)warp, lane);
+    __syncthreads();
+    if (threadIdx.x < NA) {
+      double t = sh[threadIdx.x];
+      for (int w = 1; w < WPB; ++w) t = Epi::combine(threadIdx.x, t, sh[w * NA + threadIdx.x]);
+      part[(size_t)blockIdx.x * NA + threadIdx.x] = t;
+    }
+  }
+}
+
 // Up to 32 bytes of gathered values per lane (8 FP32 or 4 FP64 items) the
 // kernel is built for 48 resident warps per SM (at most 42 registers);
 // wider tiles keep the registers they need.
@@ -377,9 +396,8 @@ constexpr int warp_min_blocks() {
 // A warp takes tiles t = global warp, + all warps of the grid: launched with
 // one warp per tile it does one tile; launched with the CTAs that fit on the
 // GPU at once (a persistent grid) it loops, and a launch after convergence
-// retires a few thousand CTAs instead of one per tile. Each warp leaves one
-// partial of the epilogue's scalars, at part[global warp]: the partials
-// number min(warps launched, ntiles).
+// retires a few thousand CTAs instead of one per tile. Each CTA leaves one
+// partial of the epilogue's scalars, at part[CTA].
 // GNA: gathers allocate in L1 (0), never (1), or only for columns below
 // l1_hot (2), so that the most gathered values stay in L1 while one-off
 // gathers pass through.
@@ -390,11 +408,11 @@ warp_spmv(OpView<MT> op, const VT* __restrict__ xg, Epi epi_in,
           VT* __restrict__ head, double* __restrict__ part, const IterState* __restrict__ st,
           uint32_t l1_hot) {
   using S = WarpSmem<VT, IPT>;
+  chain_wait();
   if (st && iteration_done(st)) return;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t gw = blockIdx.x * WPB + wib;
   uint32_t t = gw;
-  if (t >= ntiles) return;
   Epi epi = epi_in;
   epi.prepare(st);
   double acc[Epi::NACC > 0 ? Epi::NACC : 1];
@@ -448,7 +466,7 @@ warp_spmv(OpView<MT> op, const VT* __restrict__ xg, Epi epi_in,
                                    acc, lane);
     __syncwarp();  // the next tile reuses this warp's buffers
   }
-  warp_store_partials<Epi>(acc, part, gw, lane);
+  cta_store_partials<Epi, WPB>(acc, part, wib, lane);
 }
 
 // -------------------------------------------------------------------- kernel 1 (hot-node cache)
@@ -618,7 +636,30 @@ constexpr size_t tile_smem_bytes() {
 // Epi::finish. Every
 // sum has a fixed association, so results do not change from run to run.
 // Partials written by other CTAs are read with ld.global.cg (L2, not L1).
+// Epilogues that may leave the decision open (st->ambiguous) declare DECIDES
+// and give the exact change of node i: the last CTA sums it alone (about one
+// solve in a thousand, when the fused change is within rounding of the
+// tolerance; a kernel of its own for that, launched after every sweep, took 2
+// us and a launch's gap each time).
 constexpr int SPLIT_CTAS = 296;
+
+template <class E, class = void>
+struct EpiDecides {
+  static constexpr bool value = false;
+};
+template <class E>
+struct EpiDecides<E, std::void_t<decltype(E::DECIDES)>> {
+  static constexpr bool value = E::DECIDES;
+};
+
+// CTAs of split_rows: what its rows and partials need, at most SPLIT_CTAS (a
+// sweep of 3.6M arcs spent 9 us in 296).
+inline unsigned split_grid(uint32_t nsplit, uint32_t nshort, uint32_t npart) {
+  const uint32_t want = std::max({(nshort + SPMV_THREADS - 1) / SPMV_THREADS,
+                                  (nsplit - nshort + SPMV_THREADS / 32 - 1) / (SPMV_THREADS / 32),
+                                  (npart + SPMV_THREADS - 1) / SPMV_THREADS, 1u});
+  return std::min<uint32_t>(want, SPLIT_CTAS);
+}
 
 template <class VT, class Epi>
 __global__ void __launch_bounds__(SPMV_THREADS)
@@ -628,6 +669,7 @@ split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort,
            uint32_t npart, double* __restrict__ part2, IterState* st) {
   constexpr int T = SPMV_THREADS;
   constexpr int NA = Epi::NACC;
+  chain_wait();
   if (st && iteration_done(st)) return;
   Epi epi = epi_in;
   epi.prepare(st);
@@ -704,6 +746,20 @@ split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort,
   if (tid == 0) {
     epi.finish(st, tot);
     st->ticket = 0;
+  }
+  if constexpr (EpiDecides<Epi>::value) {
+    __syncthreads();
+    if (st->ambiguous == 0) return;
+    const double T2 = st->total, ip = st->prev_inv_total;
+    double ch = 0;
+    for (uint32_t i = tid; i < epi.n; i += T) ch += epi.exact_change(i, T2, ip);
+    ch = block_sum(ch, red[0]);
+    if (tid == 0) {
+      st->change = ch;
+      st->ambiguous = 0;
+      if (ch <= st->tol) st->converged = 1;
+      else if (st->iter >= st->max_iter) st->stopped = 1;
+    }
   }
 }
 
