@@ -421,7 +421,8 @@ NET_API void net_set_sweep_timing(int32_t on);
  * looping over tiles (1, default); 9 = mixed precision ends with one FP64
  * anchor sweep and refinement sweeps that gather the FP32 correction (1,
  * default) or with FP64 sweeps (0); 10 = sliced sweeps: rows of at least
- * this many arcs (1..65535) are taken by whole warps (0: automatic); 11 =
+ * this many arcs (1..65535) are taken by whole warps (0: automatic, 32 or 255
+ * or the tuner's choice); 11 =
  * FP32 values kernel 11 keeps in shared memory (-1: 32,768); 12 = pick the
  * sweep kernel per operator by timing (1, default) or always use kernel 9
  * (0); 13 = CTAs per SM kernel 12 sizes its shared memory for (0: 4, 1..8);

@@ -1125,6 +1125,13 @@ static double time_candidate(Operator& op, const SweepPick& c, int cls, bool use
 // microseconds, too little to tell the candidates apart.
 constexpr uint64_t AUTOTUNE_MIN_ARCS = 1u << 21;
 
+// Long rows of the sliced layout unless tuned or pinned. A sweep of an operator
+// below the tuner's size waits for its longest lane: with 254 arcs in one
+// lane an R-MAT graph of 400,000 arcs took 2,080 us a solve, with rows of 32
+// arcs and more on whole warps 830 us (16: 760, but 1,587 against 1,377 us on
+// an Erdos-Renyi graph of 3.6M arcs).
+static uint32_t default_long_row(uint64_t nnz) { return nnz < AUTOTUNE_MIN_ARCS ? 32u : 255u; }
+
 // The sweep kernel for an operator, picked on its first large solve by
 // timing each candidate (time_candidate) and kept for the operator's life,
 // per precision class (0: solves that start with FP32 sweeps, 1: FP64
@@ -1239,7 +1246,8 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
   const Relabeled* R = rl ? &op.relabeled(s) : nullptr;
   const SlicedOp* SO =
       sl ? &op.sliced(pick.long_row > 0 ? (uint32_t)pick.long_row
-                                        : tu.long_row > 0 ? (uint32_t)tu.long_row : 255u,
+                                        : tu.long_row > 0 ? (uint32_t)tu.long_row
+                                                          : default_long_row(op.nnz),
                       slice_pieces(), s)
          : nullptr;
   static const Partition no_partition;  // sliced sweeps cut their own work
