@@ -846,14 +846,18 @@ int32_t net_components(const GraphHandle* h, int32_t kind, int32_t* membership, 
     // ComponentKind::from_code (crates/engine/src/metrics/topography.rs:152-163)
     if (kind != 0 && kind != 1) throw Error("unknown component kind code " + std::to_string(kind));
     cudaStream_t s = knb::thread_stream();
-    knb::Comps c = kind == 1 && g.directed ? knb::strong_components(g, nullptr, false, nullptr, s)
-                                           : knb::weak_components(g, s);
-    for (uint32_t v = 0; v < g.n; ++v) {
-      if (c.membership[v] > (uint32_t)INT32_MAX)
-        throw Error("component count " + std::to_string(c.membership[v]) + " is too large");
-      membership[v] = (int32_t)c.membership[v];
+    if (g.n == 0) {
+      *count = 0;
+      return;
     }
-    *count = (int64_t)c.count();
+    const knb::DevComps c = kind == 1 && g.directed
+                                ? knb::strong_components_device(g, nullptr, false, nullptr, s)
+                                : knb::weak_components_device(g, s);
+    if (c.count > (uint32_t)INT32_MAX)
+      throw Error("component count " + std::to_string(c.count - 1) + " is too large");
+    KNB_CUDA(cudaMemcpyAsync(membership, c.label.get(), (size_t)g.n * 4, cudaMemcpyDeviceToHost, s));
+    KNB_CUDA(cudaStreamSynchronize(s));
+    *count = (int64_t)c.count;
   });
 }
 

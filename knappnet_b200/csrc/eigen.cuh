@@ -33,6 +33,14 @@ struct Comps {
   std::vector<uint32_t> sizes;
   size_t count() const { return sizes.size(); }
 };
+// The same on the device.
+struct DevComps {
+  DevBuf<uint32_t> label, sizes;
+  uint32_t count = 0;
+};
+DevComps weak_components_device(GraphHandleImpl& g, cudaStream_t s);
+DevComps strong_components_device(GraphHandleImpl& g, const double* w, bool both, int* launches,
+                                  cudaStream_t s);
 // Weak components of the handle's edges (device union-find; each
 // component's label follows its smallest node).
 Comps weak_components(GraphHandleImpl& g, cudaStream_t s);
