@@ -220,17 +220,24 @@ __global__ void scan_sums(T* sums, size_t nb, T* total) {
   if (threadIdx.x == 0) *total = carry;
 }
 
+// `sums`: room for one value per tile and the total, which ends in the last.
 template <class T>
-T exclusive_scan(const T* in, T* out, size_t n, cudaStream_t s) {
-  if (n == 0) return 0;
-  size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-  DevBuf<T> sums(nb + 1);
+static void scan_launch(const T* in, T* out, size_t n, DevBuf<T>& sums, cudaStream_t s) {
+  const size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
   scan_reduce<T><<<(unsigned)nb, SCAN_T, 0, s>>>(in, n, sums.get());
   KNB_LAUNCH("scan_reduce");
   scan_sums<T><<<1, SCAN_T, 0, s>>>(sums.get(), nb, sums.get() + nb);
   KNB_LAUNCH("scan_sums");
   scan_down<T><<<(unsigned)nb, SCAN_T, 0, s>>>(in, out, n, sums.get());
   KNB_LAUNCH("scan_down");
+}
+
+template <class T>
+T exclusive_scan(const T* in, T* out, size_t n, cudaStream_t s) {
+  if (n == 0) return 0;
+  const size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+  DevBuf<T> sums(nb + 1);
+  scan_launch<T>(in, out, n, sums, s);
   T total = 0;
   KNB_CUDA(cudaMemcpyAsync(&total, sums.get() + nb, sizeof(T), cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
@@ -242,8 +249,17 @@ template uint64_t exclusive_scan<uint64_t>(const uint64_t*, uint64_t*, size_t, c
 // ======================================================================= radix sort
 // Stable LSD radix sort of 64-bit keys with a 32-bit payload, 8 bits a pass.
 // Stability inside a tile comes from ranking elements warp by warp in input
-// order (__match_any_sync groups equal digits of a round), so equal keys keep
+// order (eight ballots group equal digits of a round), so equal keys keep
 // their input order, exactly like the reference's stable counting sorts.
+//
+// A pass moves 24 bytes an element. Written from registers in input order, its
+// stores went to up to 32 places a warp, 8 and 4 bytes each; a tile is
+// therefore put in digit order in shared memory first, so that neighbouring
+// lanes write neighbouring elements. 2^28 elements, one B200, a pass's
+// scatter: 10.3 -> 2.2 ms on random digits, 4.7 -> 1.8 ms on skewed ones (of
+// this, ballots in place of __match_any_sync: 3.6 -> 2.2 ms); 4,000,001
+// elements 62 -> 35 us. Tiles of 4096 and 8192 elements write longer runs but
+// took 2.0-2.4 ms, and at 300,000 elements up to twice as long as 2048.
 constexpr int RS_T = 256, RS_IPT = 8, RS_TILE = RS_T * RS_IPT;
 
 __global__ void radix_hist(const uint64_t* __restrict__ keys, size_t n, int shift,
@@ -260,56 +276,88 @@ __global__ void radix_hist(const uint64_t* __restrict__ keys, size_t n, int shif
   hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-__global__ void radix_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                              uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, size_t n,
-                              int shift, const uint32_t* __restrict__ offs, uint32_t ntiles) {
-  __shared__ uint32_t wcount[RS_T / 32][256];
-  __shared__ uint32_t base_d[256];
+__global__ void __launch_bounds__(RS_T, 4)
+radix_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+              uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, size_t n, int shift,
+              const uint32_t* __restrict__ offs, uint32_t ntiles) {
+  static_assert(RS_T == 256, "one thread per digit");
+  constexpr int W = RS_T / 32;
+  __shared__ uint64_t tkey[RS_TILE];
+  __shared__ uint32_t tval[RS_TILE];
+  __shared__ uint16_t wcount[W][256];
+  __shared__ uint32_t start[256], to[256], wsum[W];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   for (int d = lane; d < 256; d += 32) wcount[w][d] = 0;
   __syncwarp();
-  const size_t wbase = (size_t)blockIdx.x * RS_TILE + (size_t)w * 32 * RS_IPT;
+  const size_t tbase = (size_t)blockIdx.x * RS_TILE;
+  const size_t wbase = tbase + (size_t)w * 32 * RS_IPT;
   uint64_t key[RS_IPT];
-  uint32_t val[RS_IPT], rank[RS_IPT], dig[RS_IPT];
+  uint32_t rank[RS_IPT];
   const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
   for (int r = 0; r < RS_IPT; ++r) {
-    size_t i = wbase + (size_t)r * 32 + lane;
-    bool ok = i < n;
-    key[r] = ok ? kin[i] : 0;
-    val[r] = ok ? vin[i] : 0;
-    uint32_t d = ok ? (uint32_t)((key[r] >> shift) & 255u) : 256u;
-    dig[r] = d;
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
-    uint32_t before = __popc(peers & lt);
-    uint32_t seen = ok ? wcount[w][d] : 0;
+    const size_t i = wbase + (size_t)r * 32 + lane;
+    key[r] = i < n ? kin[i] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < RS_IPT; ++r) {
+    const bool ok = wbase + (size_t)r * 32 + lane < n;
+    const uint32_t d = (uint32_t)(key[r] >> shift) & 255u;
+    uint32_t peers = __ballot_sync(0xffffffffu, ok);
+    if (!ok) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const bool bit = (d >> b) & 1u;
+      const uint32_t ones = __ballot_sync(0xffffffffu, bit);
+      peers &= bit ? ones : ~ones;
+    }
+    const uint32_t before = __popc(peers & lt);
+    const uint32_t seen = ok ? wcount[w][d] : 0;
     rank[r] = seen + before;
     __syncwarp();
-    if (ok && before == 0) wcount[w][d] = seen + __popc(peers);
+    if (ok && before == 0) wcount[w][d] = (uint16_t)(seen + __popc(peers));
     __syncwarp();
   }
   __syncthreads();
   {
-    int d = tid;  // one digit per thread (256 threads)
-    uint32_t run = 0;
+    uint32_t count = 0;  // of digit tid in the tile, then its place in digit order
 #pragma unroll
-    for (int ww = 0; ww < RS_T / 32; ++ww) {
-      uint32_t c = wcount[ww][d];
-      wcount[ww][d] = run;
-      run += c;
+    for (int k = 0; k < W; ++k) {
+      const uint32_t c = wcount[k][tid];
+      wcount[k][tid] = (uint16_t)count;
+      count += c;
     }
-    base_d[d] = offs[(size_t)d * ntiles + blockIdx.x];
+    uint32_t upto = count;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    if (lane == 31) wsum[w] = upto;
+    __syncthreads();
+    uint32_t at = upto - count;
+    for (int k = 0; k < w; ++k) at += wsum[k];
+    start[tid] = at;
+    to[tid] = offs[(size_t)tid * ntiles + blockIdx.x] - at;  // modulo 2^32
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < RS_IPT; ++r) {
-    size_t i = wbase + (size_t)r * 32 + lane;
+    const size_t i = wbase + (size_t)r * 32 + lane;
     if (i < n) {
-      uint32_t d = dig[r];
-      size_t pos = (size_t)base_d[d] + wcount[w][d] + rank[r];
-      kout[pos] = key[r];
-      vout[pos] = val[r];
+      const uint32_t d = (uint32_t)(key[r] >> shift) & 255u;
+      const uint32_t p = start[d] + wcount[w][d] + rank[r];
+      tkey[p] = key[r];
+      tval[p] = vin[i];
     }
+  }
+  __syncthreads();
+  const uint32_t count = (uint32_t)(n - tbase < RS_TILE ? n - tbase : RS_TILE);
+#pragma unroll 4
+  for (uint32_t k = tid; k < count; k += RS_T) {
+    const uint64_t x = tkey[k];
+    const uint32_t g = to[(uint32_t)(x >> shift) & 255u] + k;
+    kout[g] = x;
+    vout[g] = tval[k];
   }
 }
 
@@ -321,6 +369,7 @@ void radix_sort(uint64_t* keys, uint32_t* vals, size_t n, int bits, cudaStream_t
   DevBuf<uint64_t> k2(n);
   DevBuf<uint32_t> v2(n);
   DevBuf<uint32_t> hist((size_t)256 * ntiles);
+  DevBuf<uint32_t> sums(((size_t)256 * ntiles + SCAN_TILE - 1) / SCAN_TILE + 1);
   uint64_t* ka = keys;
   uint32_t* va = vals;
   uint64_t* kb = k2.get();
@@ -330,7 +379,7 @@ void radix_sort(uint64_t* keys, uint32_t* vals, size_t n, int bits, cudaStream_t
     int shift = 8 * p;
     radix_hist<<<ntiles, RS_T, 0, s>>>(ka, n, shift, hist.get(), ntiles);
     KNB_LAUNCH("radix_hist");
-    exclusive_scan<uint32_t>(hist.get(), hist.get(), (size_t)256 * ntiles, s);
+    scan_launch<uint32_t>(hist.get(), hist.get(), (size_t)256 * ntiles, sums, s);
     radix_scatter<<<ntiles, RS_T, 0, s>>>(ka, va, kb, vb, n, shift, hist.get(), ntiles);
     KNB_LAUNCH("radix_scatter");
     std::swap(ka, kb);
