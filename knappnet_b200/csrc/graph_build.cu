@@ -785,28 +785,21 @@ __global__ void permuted_lengths(const uint32_t* __restrict__ off, const uint32_
     len[k] = k < n ? off[perm[k] + 1] - off[perm[k]] : 0u;
 }
 
-// Arc q of the renumbered operator: its row by binary search over the new
-// offsets, copied from the same position of the old row, column renamed.
+// Arc q of the renumbered operator, copied from the same position of the old row, column renamed.
 __global__ void permuted_arcs(const uint32_t* __restrict__ off, const uint32_t* __restrict__ cols,
                               const double* __restrict__ v64, const float* __restrict__ v32,
                               const uint32_t* __restrict__ perm, const uint32_t* __restrict__ iperm,
                               const uint32_t* __restrict__ noff, uint32_t n, uint64_t nnz,
                               uint32_t* __restrict__ ncols, double* __restrict__ nv64,
                               float* __restrict__ nv32) {
-  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < nnz;
-       q += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = n;  // largest k with noff[k] <= q
-    while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (noff[mid] <= q) lo = mid; else hi = mid;
-    }
-    uint64_t src = (uint64_t)off[perm[lo]] + (q - noff[lo]);
+  for_arcs(noff, n, nnz, [&](uint64_t q, uint32_t row) {
+    const uint64_t src = (uint64_t)off[perm[row]] + (q - noff[row]);
     ncols[q] = iperm[cols[src]];
     if (v64) {
       nv64[q] = v64[src];
       nv32[q] = v32[src];
     }
-  }
+  });
 }
 
 template <class T>
@@ -846,7 +839,7 @@ const Relabeled& Operator::relabeled(cudaStream_t s) {
   KNB_LAUNCH("relabel");
   exclusive_scan<uint32_t>(r->off.get(), r->off.get(), (size_t)n + 1, s);
   if (nnz) {
-    permuted_arcs<<<grid_for(nnz, 256), 256, 0, s>>>(
+    permuted_arcs<<<grid_for(nnz, ARCS_PER_CTA), 256, 0, s>>>(
         rows->off.get(), rows->tgt.get(), has_vals ? vals64.get() : nullptr,
         has_vals ? vals32.get() : nullptr, r->perm.get(), r->iperm.get(), r->off.get(), n, nnz,
         r->cols.get(), has_vals ? r->vals64.get() : nullptr, has_vals ? r->vals32.get() : nullptr);
@@ -893,21 +886,14 @@ __global__ void slice_count_long(const uint32_t* __restrict__ len, uint32_t n, u
     if (len[k] >= lw && (k + 1 == n || len[k + 1] < lw)) *out = k + 1;
 }
 
-// Arc a of the operator: key (new row, new column), payload a. The old row
-// comes from a binary search over the old offsets.
+// Arc a of the operator: key (new row, new column), payload a.
 __global__ void slice_arc_keys(const uint32_t* __restrict__ off, const uint32_t* __restrict__ cols,
                                const uint32_t* __restrict__ iperm, uint32_t n, uint64_t nnz,
                                int cbits, uint64_t* __restrict__ keys, uint32_t* __restrict__ ids) {
-  for (uint64_t a = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; a < nnz;
-       a += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = n;  // largest i with off[i] <= a
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (off[mid] <= a) lo = mid; else hi = mid;
-    }
-    keys[a] = ((uint64_t)iperm[lo] << cbits) | iperm[cols[a]];
+  for_arcs(off, n, nnz, [&](uint64_t a, uint32_t row) {
+    keys[a] = ((uint64_t)iperm[row] << cbits) | iperm[cols[a]];
     ids[a] = (uint32_t)a;
-  }
+  });
 }
 
 // Elements of slice s: 32 times the length of its first row (the longest).
@@ -1053,7 +1039,7 @@ const SlicedOp& Operator::sliced(uint32_t lw, uint32_t pieces, cudaStream_t s) {
     const int cbits = std::max(1, bits_for(n));
     DevBuf<uint64_t> keys(nnz);
     DevBuf<uint32_t> ids(nnz);
-    slice_arc_keys<<<grid_for(nnz, 256), 256, 0, s>>>(rows->off.get(), rows->tgt.get(),
+    slice_arc_keys<<<grid_for(nnz, ARCS_PER_CTA), 256, 0, s>>>(rows->off.get(), rows->tgt.get(),
                                                        r->iperm.get(), n, nnz, cbits, keys.get(),
                                                        ids.get());
     KNB_LAUNCH("slice_arc_keys");
