@@ -20,6 +20,7 @@
 // the second term being the derivative of the row (out-strength)
 // normalisation. An undirected edge adds the terms of its two arcs. Dangling
 // nodes stay dangling for positive weights, so D does not move.
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -89,28 +90,25 @@ struct RowSumEpi {
   __device__ void finish(IterState*, const double*) const {}
 };
 
-// Sums of v and w over the CTAs of the grid (each CTA's value in thread 0),
-// in a fixed order; true in the last CTA, which gets them.
-__device__ __forceinline__ bool last_sums(double v, double w, double* part, unsigned int* ticket,
-                                          double* sh, double* t, double* u) {
+// Sums of v[0..N-1] over the grid in CTA order, in the CTA that comes last.
+template <int N>
+__device__ __forceinline__ bool last_sums(double (&v)[N], double* __restrict__ part,
+                                          uint32_t* ticket, double* sh) {
   __shared__ bool last;
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = v;
-    part[2 * blockIdx.x + 1] = w;
-  }
+  if (threadIdx.x == 0)
+    for (int k = 0; k < N; ++k) part[N * blockIdx.x + k] = v[k];
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  double x = 0, y = 0;
-  for (uint32_t q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
-    x += __ldcg(part + 2 * q);
-    y += __ldcg(part + 2 * q + 1);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    double x = 0;
+    for (uint32_t q = threadIdx.x; q < gridDim.x; q += blockDim.x) x += __ldcg(part + N * q + k);
+    v[k] = block_sum(x, sh);
   }
-  *t = block_sum(x, sh);
-  *u = block_sum(y, sh);
   return true;
 }
 
@@ -127,12 +125,10 @@ adj_init(const double* __restrict__ g, const double* __restrict__ jump, uint32_t
     a += (jump ? jump[i] : pu) * v;
     b += fabs(v);
   }
-  a = block_sum(a, sh);
-  b = block_sum(b, sh);
-  double t, u;
-  if (!last_sums(a, b, part, &st->ticket, sh, &t, &u) || threadIdx.x != 0) return;
-  st->dterm = t;
-  st->tol = tol * fmax(1.0, u);
+  double v[2] = {block_sum(a, sh), block_sum(b, sh)};
+  if (!last_sums(v, part, &st->ticket, sh) || threadIdx.x != 0) return;
+  st->dterm = v[0];
+  st->tol = tol * fmax(1.0, v[1]);
   st->ticket = 0;
 }
 
@@ -147,37 +143,54 @@ adj_init(const double* __restrict__ g, const double* __restrict__ jump, uint32_t
 // change and the same stopping rule come from one pass over four vectors, and
 // E is taken only where that change is below half of the plain one: a graph
 // whose error has no such part keeps the plain iteration.
+//
+// The plain iteration's last sweeps move every node the same way, by d of the
+// sweep before, until all of them round to what they were. E is past that: what
+// is left of its error changes sign and may stay at one unit in the last place
+// of every node, back and forth, for good. So E is not taken where the tolerance
+// is below ROUNDED of lambda's size (n nodes at one unit each come to at most
+// 2^-52 of it), and a solve whose change, above the tolerance, has not come down
+// to `stall` of that a cycle before is stopped; the caller then iterates plainly
+// from the start.
 constexpr int SPAN = 6;
 constexpr int CYCLE = 24;  // an extrapolation is tried every CYCLE sweeps
+constexpr double ROUNDED = 4.0 * DBL_EPSILON;
 
 __global__ void __launch_bounds__(256)
 adj_extrapolate(const double* __restrict__ a0, const double* __restrict__ a,
                 const double* __restrict__ b0, const double* __restrict__ b, double c, double d,
-                const double* __restrict__ jump, uint32_t n, double* __restrict__ part,
-                IterState* st) {
+                double stall, const double* __restrict__ jump, uint32_t n,
+                double* __restrict__ part, IterState* st) {
   if (iteration_done(st)) return;
   __shared__ double sh[8];
-  double ch = 0, jd = 0;
+  double ch = 0, jd = 0, size = 0;
   const double pu = 1.0 / n;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double av = a[i], bv = b[i];
+    size += fabs(bv);
     ch += fabs((1.0 + c) * (bv - b0[i]) - c * (av - a0[i]));
     jd += (jump ? jump[i] : pu) * (bv + c * (bv - av));
   }
-  ch = block_sum(ch, sh);
-  jd = block_sum(jd, sh);
-  double t, u;
-  if (!last_sums(ch, jd, part, &st->ticket, sh, &t, &u) || threadIdx.x != 0) return;
+  double v[3] = {block_sum(ch, sh), block_sum(jd, sh), block_sum(size, sh)};
+  if (!last_sums(v, part, &st->ticket, sh) || threadIdx.x != 0) return;
   st->ticket = 0;
-  if (!(t < 0.5 * st->change)) return;
-  if (!st->ambiguous) {
-    st->ambiguous = 1;
-    st->prev_inv_total = st->iter + ceil(log(st->tol / st->change) / log(d));
+  const double before = st->slack;  // the change a cycle ago
+  if (v[0] < 0.5 * st->change && st->tol >= ROUNDED * v[2]) {
+    if (!st->ambiguous) {
+      st->ambiguous = 1;
+      st->prev_inv_total = st->iter + ceil(log(st->tol / st->change) / log(d));
+      st->slack = INFINITY;
+    }
+    st->top = 1.0;  // adj_take replaces b by E
+    st->change = v[0];
+    st->dterm = v[1];
+    adj_decide(st);
   }
-  st->top = 1.0;  // adj_take replaces b by E
-  st->change = t;
-  st->dterm = u;
-  adj_decide(st);
+  if (st->ambiguous) {
+    if (st->slack == before && st->change > st->tol && !(st->change <= stall * before))
+      st->stopped = 1;
+    st->slack = st->change;
+  }
 }
 
 __global__ void adj_take(const double* __restrict__ a, double* __restrict__ b, double c,
@@ -254,7 +267,7 @@ struct AdjointWorkspace : Workspace {
     head.alloc(ntiles + 1);
     part1.alloc((size_t)ntiles * AdjointEpi::NACC + 4);
     part2.alloc((size_t)SPLIT_CTAS * AdjointEpi::NACC + 4);
-    part3.alloc(2 * 1184 + 2);
+    part3.alloc(3 * 1184 + 2);
     st.alloc(1);
     KNB_CUDA(cudaEventCreate(&t0));
     KNB_CUDA(cudaEventCreate(&t1));
@@ -310,14 +323,9 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
     jump = W.jump.get();
   }
   IterState* st = W.st.get();
-  W.hst[0] = IterState{};
-  W.hst[0].max_iter = (int32_t)std::min<int64_t>(prm.max_iter, INT32_MAX);
-  KNB_CUDA(cudaMemcpyAsync(st, &W.hst[0], sizeof(IterState), cudaMemcpyHostToDevice, s));
   KNB_CUDA(cudaEventRecord(W.t0, s));
   const unsigned gv = grid_for(n, 256, 1184);
-  adj_init<<<gv, 256, 0, s>>>(d_gx, jump, n, prm.tol, W.lam[0].get(), W.part3.get(), st);
-  KNB_LAUNCH("adj_init");
-  int launches = 1;
+  int launches = 0;
   // one CTA of 16 warps takes tiles until none is left; as many CTAs as fit
   // at once (against one tile per warp and 4 warps per CTA: 104 -> 79 us a
   // sweep on R-MAT 20)
@@ -328,6 +336,7 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
   fit_warp_carveout<double, double, AdjointEpi, IPT, WPB>();
   fit_warp_carveout<double, double, RowSumEpi, IPT, WPB>();
   const double dspan = std::pow(prm.damping, SPAN), c = dspan / (1.0 - dspan);
+  const double stall = std::pow(prm.damping, CYCLE / 2);
   // Sweep k turns iterate k into iterate k + 1. Iterates alternate between
   // two buffers, but the two that an extrapolation looks back on (SPAN + 1
   // and SPAN sweeps before the end of a cycle) have buffers of their own.
@@ -336,7 +345,7 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
     return W.lam[at == CYCLE - SPAN - 1 ? 2 : at == CYCLE - SPAN ? 3 : k & 1].get();
   };
   int k = 0;
-  auto enqueue = [&](int slot) {
+  auto enqueue = [&](int slot, bool extrapolate) {
     for (int q = 0; q < 8; ++q, ++k) {
       AdjointEpi e;
       e.g = d_gx;
@@ -353,10 +362,10 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
                      SPMV_THREADS, 0, s, P.split.get(), P.nsplit, P.nshort, W.carry.get(),
                      W.head.get(), e, W.part1.get(), grid, W.part2.get(), st);
       launches += 2;
-      if ((k + 1) % CYCLE == 0) {
+      if (extrapolate && (k + 1) % CYCLE == 0) {
         adj_extrapolate<<<gv, 256, 0, s>>>(W.lam[2].get(), W.lam[3].get(), buffer(k),
-                                           buffer(k + 1), c, prm.damping, jump, n, W.part3.get(),
-                                           st);
+                                           buffer(k + 1), c, prm.damping, stall, jump, n,
+                                           W.part3.get(), st);
         adj_take<<<gv, 256, 0, s>>>(W.lam[3].get(), buffer(k + 1), c, n, st);
         launches += 2;
       }
@@ -367,20 +376,31 @@ void pagerank_grad(GraphHandleImpl& g, const double* d_w, const double* d_x, con
   };
   // one batch of sweeps in flight ahead of the state the host looks at;
   // sweeps after the end exit at once
-  enqueue(0);
-  for (int slot = 0;; slot ^= 1) {
-    enqueue(slot ^ 1);
-    KNB_CUDA(cudaEventSynchronize(W.done[slot]));
-    if (W.hst[slot].converged || W.hst[slot].stopped) {
-      KNB_CUDA(cudaEventSynchronize(W.done[slot ^ 1]));
-      break;
+  auto solve = [&](bool extrapolate) -> IterState {
+    W.hst[0] = IterState{};
+    W.hst[0].max_iter = (int32_t)std::min<int64_t>(prm.max_iter, INT32_MAX);
+    KNB_CUDA(cudaMemcpyAsync(st, &W.hst[0], sizeof(IterState), cudaMemcpyHostToDevice, s));
+    adj_init<<<gv, 256, 0, s>>>(d_gx, jump, n, prm.tol, W.lam[0].get(), W.part3.get(), st);
+    KNB_LAUNCH("adj_init");
+    ++launches;
+    k = 0;
+    enqueue(0, extrapolate);
+    for (int slot = 0;; slot ^= 1) {
+      enqueue(slot ^ 1, extrapolate);
+      KNB_CUDA(cudaEventSynchronize(W.done[slot]));
+      if (W.hst[slot].converged || W.hst[slot].stopped) {
+        KNB_CUDA(cudaEventSynchronize(W.done[slot ^ 1]));
+        break;
+      }
     }
-  }
-  const IterState h = W.hst[0].iter > W.hst[1].iter ? W.hst[0] : W.hst[1];
-  // The cap counts the sweeps of the plain iteration.
-  const bool within =
-      h.converged && (!h.ambiguous || h.prev_inv_total <= (double)prm.max_iter);
-  if (!within)
+    return W.hst[0].iter > W.hst[1].iter ? W.hst[0] : W.hst[1];
+  };
+  IterState h = solve(true);
+  // The cap counts the sweeps of the plain iteration, which st->prev_inv_total
+  // foretells: only a solve that is clearly within it stands.
+  if (h.ambiguous && !(h.converged && h.prev_inv_total + CYCLE <= (double)prm.max_iter))
+    h = solve(false);
+  if (!h.converged)
     throw Error("the PageRank adjoint did not converge within " + std::to_string(prm.max_iter) +
                 " iterations");
   const double* lam_final = buffer(h.iter);
