@@ -62,12 +62,20 @@ struct AdjointEpi {
   static __device__ __forceinline__ double identity(int) { return 0.0; }
   static __device__ __forceinline__ double combine(int, double a, double b) { return a + b; }
   static __device__ __forceinline__ double warp_combine(int, double v) { return warp_sum(v); }
-  __device__ __forceinline__ void row(uint32_t j, double r, double* a) const {
-    const double io = inv_out[j];
-    const double v = g[j] + d * (io > 0.0 ? r * io : jdot);
+  struct In {
+    double io, gj, lo, jj;
+  };
+  __device__ __forceinline__ In fetch(uint32_t j) const {
+    return {inv_out[j], g[j], lam_old[j], jump ? jump[j] : pu};
+  }
+  __device__ __forceinline__ void row_in(uint32_t j, double r, const In& in, double* a) const {
+    const double v = in.gj + d * (in.io > 0.0 ? r * in.io : jdot);
     lam_new[j] = v;
-    a[0] += fabs(v - lam_old[j]);
-    a[1] += (jump ? jump[j] : pu) * v;
+    a[0] += fabs(v - in.lo);
+    a[1] += in.jj * v;
+  }
+  __device__ __forceinline__ void row(uint32_t j, double r, double* a) const {
+    row_in(j, r, fetch(j), a);
   }
   __device__ void finish(IterState* st, const double* tot) const {
     st->change = tot[0];

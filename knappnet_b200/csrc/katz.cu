@@ -223,11 +223,18 @@ struct SeriesEpi {
   static __device__ __forceinline__ double identity(int) { return 0.0; }
   static __device__ __forceinline__ double combine(int, double a, double c) { return fmax(a, c); }
   static __device__ __forceinline__ double warp_combine(int, double v) { return warp_max(v); }
-  __device__ __forceinline__ void row(uint32_t g, double s, double* a) const {
-    const double y = __dadd_rn(b[g], __dmul_rn(t, s));
+  struct In {
+    double bg, xo;
+  };
+  __device__ __forceinline__ In fetch(uint32_t g) const { return {b[g], x_old[g]}; }
+  __device__ __forceinline__ void row_in(uint32_t g, double s, const In& in, double* a) const {
+    const double y = __dadd_rn(in.bg, __dmul_rn(t, s));
     y_new[g] = y;
-    a[0] = fmax(a[0], fabs(y - x_old[g]));
+    a[0] = fmax(a[0], fabs(y - in.xo));
     a[1] = fmax(a[1], fabs(y));
+  }
+  __device__ __forceinline__ void row(uint32_t g, double s, double* a) const {
+    row_in(g, s, fetch(g), a);
   }
   __device__ void finish(IterState* st, const double* tot) const {
     st->change = tot[0];

@@ -641,7 +641,52 @@ constexpr size_t tile_smem_bytes() {
 // solve in a thousand, when the fused change is within rounding of the
 // tolerance; a kernel of its own for that, launched after every sweep, took 2
 // us and a launch's gap each time).
-constexpr int SPLIT_CTAS = 296;
+//
+// Bound by latency: the bytes are few, but each row is a chain of loads (the
+// row, its partials, its node's inputs). So all that does not depend on the
+// sums is loaded first (the next row, the node's inputs, the head, the CTA's
+// partials), up to eight of a lane's partials are in flight at once and added
+// in the same order, and short and long rows go to different ends of the grid
+// (3.6M arcs, FP64: 1.78 -> 1.68 ms a solve; R-MAT with 2^24 arcs: HITS 7.5 ->
+// 7.0, a gradient 10.1 -> 9.7, Katz 8.0 -> 7.8 ms; level with 2^28 arcs, where
+// the next kernel's wait hides it).
+constexpr int SPLIT_CTAS = 592;
+
+template <class E, class = void>
+struct EpiFetch {  // epilogues whose inputs are not loaded ahead
+  struct In {};
+  static __device__ __forceinline__ In get(const E&, uint32_t) { return {}; }
+  template <class VT>
+  static __device__ __forceinline__ void row(const E& e, uint32_t r, VT s, const In&, double* a) {
+    e.row(r, s, a);
+  }
+};
+template <class E>
+struct EpiFetch<E, std::void_t<typename E::In>> {
+  using In = typename E::In;
+  static __device__ __forceinline__ In get(const E& e, uint32_t r) { return e.fetch(r); }
+  template <class VT>
+  static __device__ __forceinline__ void row(const E& e, uint32_t r, VT s, const In& in,
+                                             double* a) {
+    e.row_in(r, s, in, a);
+  }
+};
+
+// sum + carry[q], carry[q + STEP], ... below `last`, added in that order with
+// U of them in flight.
+template <int U, int STEP, class VT>
+__device__ __forceinline__ VT add_carries(VT sum, const VT* __restrict__ carry, uint32_t q,
+                                          uint32_t last) {
+  for (; q < last; q += U * STEP) {
+    VT c[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) c[k] = q + k * STEP < last ? __ldcg(carry + q + k * STEP) : VT(0);
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (q + k * STEP < last) sum += c[k];
+  }
+  return sum;
+}
 
 template <class E, class = void>
 struct EpiDecides {
@@ -652,12 +697,12 @@ struct EpiDecides<E, std::void_t<decltype(E::DECIDES)>> {
   static constexpr bool value = E::DECIDES;
 };
 
-// CTAs of split_rows: what its rows and partials need, at most SPLIT_CTAS (a
-// sweep of 3.6M arcs spent 9 us in 296).
+// CTAs of split_rows: what its rows and partials need, at most SPLIT_CTAS
+// (four per SM; a sweep of 3.6M arcs spent 9 us in 296 that it did not need).
 inline unsigned split_grid(uint32_t nsplit, uint32_t nshort, uint32_t npart) {
-  const uint32_t want = std::max({(nshort + SPMV_THREADS - 1) / SPMV_THREADS,
-                                  (nsplit - nshort + SPMV_THREADS / 32 - 1) / (SPMV_THREADS / 32),
-                                  (npart + SPMV_THREADS - 1) / SPMV_THREADS, 1u});
+  const uint32_t rows = (nshort + SPMV_THREADS - 1) / SPMV_THREADS +
+                        (nsplit - nshort + SPMV_THREADS / 32 - 1) / (SPMV_THREADS / 32);
+  const uint32_t want = std::max({rows, (npart + SPMV_THREADS - 1) / SPMV_THREADS, 1u});
   return std::min<uint32_t>(want, SPLIT_CTAS);
 }
 
@@ -678,33 +723,56 @@ split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double a[NA > 0 ? NA : 1];
   Epi::init(a);
+  using Fetch = EpiFetch<Epi>;
+  // this CTA's slice of the sweep's partials, in order per thread
+  const uint32_t per = (npart + gridDim.x - 1) / gridDim.x;
+  const uint32_t q0 = blockIdx.x * per, q1 = min(npart, q0 + per);
+  uint32_t pq = q0 + tid;
+  double pa[NA > 0 ? NA : 1];
+#pragma unroll
+  for (int s = 0; s < NA; ++s) pa[s] = pq < q1 ? __ldcg(part1 + (size_t)pq * NA + s) : 0.0;
   // short split rows (few tiles): one thread each, carries added in tile order
-  for (uint32_t s = blockIdx.x * T + tid; s < nshort; s += gridDim.x * T) {
-    const SplitRow r = sr[s];
-    VT sum = VT(0);
-    for (uint32_t q = r.first; q < r.last; ++q) sum += __ldcg(carry + q);
-    sum += __ldcg(head + r.last);
-    epi.row(r.row, sum, a);
+  {
+    uint32_t s = blockIdx.x * T + tid;
+    SplitRow next = {};
+    if (s < nshort) next = sr[s];
+    while (s < nshort) {
+      const SplitRow r = next;
+      s += gridDim.x * T;
+      if (s < nshort) next = sr[s];
+      const auto in = Fetch::get(epi, r.row);
+      const VT h = __ldcg(head + r.last);
+      Fetch::row(epi, r.row, add_carries<4, 1>(VT(0), carry, r.first, r.last) + h, in, a);
+    }
   }
-  // long split rows (hubs): one warp each
-  const uint32_t gwarp = blockIdx.x * (T / 32) + warp, nwarps = gridDim.x * (T / 32);
-  for (uint32_t s = nshort + gwarp; s < nsr; s += nwarps) {
-    const SplitRow r = sr[s];
-    VT sum = VT(0);
-    for (uint32_t q = r.first + lane; q < r.last; q += 32) sum += __ldcg(carry + q);
-    sum = warp_sum(sum);
-    if (lane == 0) {
-      sum += __ldcg(head + r.last);
-      epi.row(r.row, sum, a);
+  // long split rows (hubs): one warp each, from the grid's other end
+  {
+    const uint32_t nwarps = gridDim.x * (T / 32);
+    uint32_t s = nshort + nwarps - 1 - (blockIdx.x * (T / 32) + warp);
+    SplitRow next = {};
+    if (s < nsr) next = sr[s];
+    while (s < nsr) {
+      const SplitRow r = next;
+      s += nwarps;
+      if (s < nsr) next = sr[s];
+      typename Fetch::In in{};
+      VT h = VT(0);
+      if (lane == 0) {
+        in = Fetch::get(epi, r.row);
+        h = __ldcg(head + r.last);
+      }
+      const VT sum = warp_sum(add_carries<8, 32>(VT(0), carry, r.first + lane, r.last));
+      if (lane == 0) Fetch::row(epi, r.row, sum + h, in, a);
     }
   }
   if constexpr (NA > 0) {
-    // this CTA's slice of the sweep's partials, in order per thread
-    const uint32_t per = (npart + gridDim.x - 1) / gridDim.x;
-    const uint32_t q0 = blockIdx.x * per, q1 = min(npart, q0 + per);
-    for (uint32_t q = q0 + tid; q < q1; q += T)
+    if (pq < q1) {
 #pragma unroll
-      for (int s = 0; s < NA; ++s) a[s] = Epi::combine(s, a[s], __ldcg(part1 + (size_t)q * NA + s));
+      for (int s = 0; s < NA; ++s) a[s] = Epi::combine(s, a[s], pa[s]);
+    }
+    for (pq += T; pq < q1; pq += T)
+#pragma unroll
+      for (int s = 0; s < NA; ++s) a[s] = Epi::combine(s, a[s], __ldcg(part1 + (size_t)pq * NA + s));
 #pragma unroll
     for (int s = 0; s < NA; ++s) {
       double v = Epi::warp_combine(s, a[s]);
@@ -735,12 +803,27 @@ split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort,
 #pragma unroll
   for (int s = 0; s < NA; ++s) tot[s] = Epi::identity(s);
   if constexpr (NA > 0) {
-    if (warp == 0) {
-      for (uint32_t q = lane; q < gridDim.x; q += 32)
+    constexpr int EACH = (SPLIT_CTAS + T - 1) / T;
+    double v[EACH][NA];
 #pragma unroll
-        for (int s = 0; s < NA; ++s) tot[s] = Epi::combine(s, tot[s], __ldcg(part2 + (size_t)q * NA + s));
+    for (int k = 0; k < EACH; ++k)
 #pragma unroll
-      for (int s = 0; s < NA; ++s) tot[s] = Epi::warp_combine(s, tot[s]);
+      for (int s = 0; s < NA; ++s) {
+        const uint32_t q = tid + k * T;
+        v[k][s] = q < gridDim.x ? __ldcg(part2 + (size_t)q * NA + s) : Epi::identity(s);
+      }
+#pragma unroll
+    for (int s = 0; s < NA; ++s) {
+#pragma unroll
+      for (int k = 0; k < EACH; ++k) tot[s] = Epi::combine(s, tot[s], v[k][s]);
+      tot[s] = Epi::warp_combine(s, tot[s]);
+      if (lane == 0) red[s][warp] = tot[s];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < NA; ++s) {
+      tot[s] = lane < T / 32 ? red[s][lane] : Epi::identity(s);
+      tot[s] = Epi::warp_combine(s, tot[s]);
     }
   }
   if (tid == 0) {
