@@ -565,12 +565,11 @@ def run_c4a(args):
     arcs = int(g.csr(1)[0][-1])
     hbm, peak_kind = peaks()
     # Algorithmic bytes of the sweeps, each array counted once: every sweep
-    # reads the row offsets, the column indices and the gathered n x B block
-    # (4 or 8 bytes a value, all columns: a node's B values are one run);
-    # each column still active in a sweep also reads its previous iterate
-    # and writes its new iterate and scaled iterate (3 n values). Converged
-    # columns are left alone, so active column-sweeps come from the solve's
-    # own counts per phase.
+    # reads the row offsets and the column indices; each column still active
+    # in a sweep also has its n values gathered (4 or 8 bytes a value), reads
+    # its previous iterate and writes its new iterate and scaled iterate (3 n
+    # values). Converged columns are left alone and packed away, so active
+    # column-sweeps, from the solve's own counts per phase, are what counts.
     s32, s64 = int(dinfo.sweeps_fp32), int(dinfo.sweeps - dinfo.sweeps_fp32)
     c32 = int(dinfo.column_iterations_fp32)
     c64 = int(dinfo.column_iterations) - c32
@@ -581,24 +580,24 @@ def run_c4a(args):
         # e and z_e written: 24 bytes a node and column) and refinement sweeps
         # (FP32 gathers; y_ref, s_ref and e read, e and z_e written: 28 bytes)
         alg64 = (base + 8.0 * n * B + B * 24.0 * n +
-                 (s64 - 1) * (base + 4.0 * n * B) + (c64 - B) * 28.0 * n)
+                 (s64 - 1) * base + (c64 - B) * (4.0 + 28.0) * n)
         rows64 = (base + 8.0 * arcs * B + B * 24.0 * n +
-                  (s64 - 1) * (base + 4.0 * arcs * B) + (c64 - B) * 28.0 * n)
+                  (s64 - 1) * base + (c64 - B) * (4.0 * arcs + 28.0 * n))
     else:
-        alg64 = s64 * (base + 8.0 * n * B) + c64 * 24.0 * n
-        rows64 = s64 * (base + 8.0 * arcs * B) + c64 * 24.0 * n
-    alg = s32 * (base + 4.0 * n * B) + c32 * 12.0 * n + alg64
+        alg64 = s64 * base + c64 * (8.0 + 24.0) * n
+        rows64 = s64 * base + c64 * (8.0 * arcs + 24.0 * n)
+    alg = s32 * base + c32 * (4.0 + 12.0) * n + alg64
     ach = alg / dinfo.sweep_seconds / 1e9
-    # The same sweeps if every arc's gathered row (B values) came from DRAM,
+    # The same sweeps if every arc's gathered row (its active columns) came from DRAM,
     # as it must when the n x B iterate (4.3 GB in FP32) cannot stay in L2:
     # what the kernel moves, against the bandwidth.
-    rows = s32 * (base + 4.0 * arcs * B) + c32 * 12.0 * n + rows64
+    rows = s32 * base + c32 * (4.0 * arcs + 12.0 * n) + rows64
     ach_rows = rows / dinfo.sweep_seconds / 1e9
     return {"workload": f"c4a: R-MAT {scale} directed, 256 personalisation vectors (uniform over "
                         "1-64 seed nodes), batched SpMM PageRank, mixed precision, tol 1e-10",
             "device_pointers": {"solve_ms": round(dsec * 1e3, 2),
                                 "sweeps_ms": round(dinfo.sweep_seconds * 1e3, 2),
-                                "gteps_b_per_sweep": round(arcs * B * dinfo.sweeps /
+                                "gteps_b_per_sweep": round(arcs * int(dinfo.column_iterations) /
                                                            dinfo.sweep_seconds / 1e9, 2),
                                 "same_scores_as_host_call": same,
                                 "fp64_phase": ("one anchor sweep, then refinement sweeps gathering "
@@ -609,19 +608,19 @@ def run_c4a(args):
                                     "peak_kind": peak_kind, "unit": "GB/s",
                                     "frac": round(ach / hbm, 4),
                                     "bytes_per_sweep_avg": round(alg / max(dinfo.sweeps, 1)),
-                                    "bytes": "offsets, indices and the gathered n x B block per "
-                                             "sweep; previous, new and scaled iterate of each "
+                                    "bytes": "offsets and indices per sweep; gathered, "
+                                             "previous, new and scaled iterate of each "
                                              "active column",
                                     "with_row_gathers": {
                                         "achieved": round(ach_rows, 1),
                                         "frac": round(ach_rows / hbm, 4),
-                                        "bytes": "as above, but one gathered row of B values per "
-                                                 "arc instead of the n x B block once"}}},
+                                        "bytes": "as above, but one gathered value per arc and "
+                                                 "active column instead of each value once"}}},
             "metric": "GTEPS*B per sweep", "unit": "GTEPS*B/sweep", "higher_is_better": True,
-            "value": round(arcs * B * info.sweeps / sec / 1e9, 2),
+            "value": round(arcs * int(info.column_iterations) / sec / 1e9, 2),
             "solve_ms": round(sec * 1e3, 2),
             "sweeps_ms": round(info.sweep_seconds * 1e3, 2),
-            "gteps_b_per_sweep_device": round(arcs * B * info.sweeps / info.sweep_seconds / 1e9, 2),
+            "gteps_b_per_sweep_device": round(arcs * int(info.column_iterations) / info.sweep_seconds / 1e9, 2),
             "sweeps": int(info.sweeps),
             "sweeps_fp32": int(info.sweeps_fp32), "arcs": arcs,
             "l1_vs_oracle_sampled_columns": errs,

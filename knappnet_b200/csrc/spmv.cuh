@@ -58,7 +58,8 @@ struct OpView {
 };
 
 // Scalars shared by the kernels of one iteration. Written by the last CTA of
-// the split-row kernel (and the exact-change kernel), read by the next sweep.
+// the split-row kernel, read by the next sweep. The adjoint's solves keep the
+// foretold plain sweeps in prev_inv_total and a cycle's change in slack.
 struct IterState {
   double inv_total;       // 1 / sum of the current (unnormalised) iterate
   double dterm;           // dangling mass of the normalised current iterate
@@ -67,7 +68,7 @@ struct IterState {
   double dang;            // its dangling mass
   double change;          // L1 change of the last sweep (see PagerankEpi)
   double tol;             // stopping tolerance of this phase
-  double slack;           // |change - exact change| bound used to call K3
+  double slack;           // bound on |change - exact change|
   double top;             // power iteration: largest entry of the newest iterate
   int32_t iter;           // sweeps done
   int32_t max_iter;       // sweep cap
