@@ -4,13 +4,15 @@
 //
 // Graphs are taken off queues largest first (so the last graphs to start are
 // the small ones) and each runs the reference's iteration on its own
-// (crates/engine/src/metrics/spectral.rs:247-280), every sum in a fixed order,
-// so each graph gets what a separate net_pagerank call on it returns, up to
-// the association of sums. A large graph would keep one CTA busy long after
-// the rest of the batch is done, so the launch runs in thread-block clusters:
-// each cluster first splits the large graphs over its CTAs, then every CTA
-// takes small graphs alone. A single small graph's solve runs here too, as a
-// batch of one.
+// (crates/engine/src/metrics/spectral.rs:247-280), every sum in a fixed order.
+// Scores are those of a separate net_pagerank call on the graph up to rounding
+// (sums are associated in another way and the division by the total comes a
+// sweep later), and the sweep a graph stops on is that of the iteration which
+// divides by the total in every sweep (ego_normalising): it decides where
+// rounding could. A large graph would keep one CTA busy long after the rest of
+// the batch is done, so the launch runs in thread-block clusters: each cluster
+// first splits the large graphs over its CTAs, then every CTA takes small
+// graphs alone. A single small graph's solve runs here too, as a batch of one.
 //
 // What bounds an iteration of a graph this small is latency: the chain from a
 // row's offsets over its columns to the gathered values, the sums, and the
@@ -18,8 +20,7 @@
 // values, out-strengths, and z = x / out in two buffers of which an iteration
 // reads one and writes the other), and an iteration has one reduction and one
 // barrier: the division by the total is left to the next iteration's scalars,
-// as in the sweeps (pagerank.cu), with the exact L1 change computed only when
-// the fused one cannot decide. CTAs of a cluster each keep all of z and write
+// as in the sweeps (pagerank.cu). CTAs of a cluster each keep all of z and write
 // every value they compute into all of the copies. Graphs whose arcs do not
 // fit keep those in global memory, graphs whose vectors do not fit keep
 // everything there.
@@ -52,6 +53,16 @@ struct EgoParams {
   double tol;
   int32_t max_iter;
   int32_t jump_uniform;  // dangling nodes jump uniformly (1) or by p (0)
+};
+
+// How the normalising iteration associates its sums, whatever the launch's
+// shape: `threads` partial sums (of every threads-th row) joined warp by warp,
+// for a graph of at least `split` nodes over each of EGO_SHARES equal shares of
+// its rows.
+constexpr int EGO_SHARES = 8;
+struct EgoOrder {
+  uint32_t threads;
+  uint32_t split;
 };
 
 // Fixed-order sums of three values over the threads of a graph's CTAs: warp
@@ -101,6 +112,7 @@ struct EgoGraph {
   OpView<double> op;
   const float* vals32;   // the values in FP32 where all are exact there, else null
   const double* inv_out; // 1 / out-strength, 0 for dangling nodes
+  const double* outstr;  // out-strength
   uint32_t g_lo, nk;     // its nodes [g_lo, g_lo + nk)
   uint32_t lo, hi;       // this CTA's rows
   uint32_t rmax;         // most rows of any CTA of the cluster
@@ -115,6 +127,9 @@ struct EgoGraph {
 // and spread over the warps (the hubs of a skewed graph tend to be neighbours).
 constexpr uint32_t EGO_LONG = 32;
 
+// How a graph's solve ended: at the iteration cap, at the tolerance, or open.
+enum { EGO_CAPPED = 0, EGO_DONE = 1, EGO_OPEN = 2 };
+
 // Where a graph lives: everything in shared memory, all but its arcs, nothing.
 enum { EGO_SMEM = 1, EGO_ARCS_GLOBAL = 2, EGO_GLOBAL = 3 };
 
@@ -125,11 +140,23 @@ __host__ __device__ constexpr size_t ego_arc_bytes(size_t arcs, size_t value_byt
   return ((arcs * value_bytes + 7) & ~size_t(7)) + arcs * 2;
 }
 
+// How far rounding may part the L1 change of this iteration from that of the
+// normalising one: a row of m arcs is off by about sqrt(m) units of its value,
+// `rows` = sum x sqrt(m) over the rows. Measured between the two iterations at
+// the same sweep, 16,000 solves of 20 to 20,000 nodes, with and without hub rows
+// and weights: mean 5e-17, at most 7.6e-16; a graph of 12 arcs a node gets
+// 2e-15 here.
+__device__ __forceinline__ double ego_rounding(double rows, double change) {
+  return DBL_EPSILON * (2.0 + 2.0 * rows + 64.0 * change);
+}
+
 // One graph's iteration. y holds the unnormalised iterate (x = y / T), z =
 // y / out; a sweep forms u = d (s / T + (D / T) jump) + (1 - d) p with D the
 // dangling mass of y. MT: the arc values' type (void: every entry is 1).
+// False, with nothing written to the outputs, where the change comes so near to
+// the tolerance that rounding decides (in all CTAs of a cluster alike).
 template <int C, int TIER, class MT>
-__device__ __forceinline__ void ego_iterate(const EgoGraph& g, const EgoParams& prm, double* sh,
+__device__ __forceinline__ bool ego_iterate(const EgoGraph& g, const EgoParams& prm, double* sh,
                                             double* slots, int32_t* it_out, int32_t* done_out,
                                             double* change_out) {
   extern __shared__ __align__(16) unsigned char ego_smem[];
@@ -139,6 +166,7 @@ __device__ __forceinline__ void ego_iterate(const EgoGraph& g, const EgoParams& 
   const uint32_t lane = threadIdx.x & 31, T = blockDim.x;
   const double inv_n = 1.0 / (double)g.nk;
   const uint32_t a0 = g.op.off[g.lo], na = g.op.off[g.hi] - a0;
+  const float root = sqrtf((float)(g.op.off[g.g_lo + g.nk] - g.op.off[g.g_lo]));
   // z and y in two buffers each: b zs, b ys apart
   double* z;
   double* y;
@@ -287,29 +315,185 @@ __device__ __forceinline__ void ego_iterate(const EgoGraph& g, const EgoParams& 
     }
     ego_sums<C>(acc, sh, slots, turn++);
     // sum |u - x| differs from the change sum |u / T - x| by at most |1 - T|;
-    // where that could decide otherwise, the change itself
+    // where that or rounding could decide otherwise (the rows' errors are at
+    // most sqrt(all arcs) of their units), the change itself and its rounding
     total = acc[0];
     change = acc[2];
     if (fabs(change - prm.tol) <=
-        2.0 * fabs(1.0 - total) + 64.0 * DBL_EPSILON * fmax(change, prm.tol)) {
+        2.0 * fabs(1.0 - total) + ego_rounding(root, fmax(change, prm.tol))) {
       double ex[3] = {0.0, 0.0, 0.0};
-      for (uint32_t r = threadIdx.x; r < R; r += T) ex[0] += fabs(yn[r] / total - yo[r] * c_it);
+      for (uint32_t r = threadIdx.x; r < R; r += T) {
+        const double x = yn[r] / total;
+        ex[0] += fabs(x - yo[r] * c_it);
+        ex[1] += x * sqrtf((float)(off[r + 1] - off[r]));
+      }
       ego_sums<C>(ex, sh, slots, turn++);
       change = ex[0];
+      if (fabs(change - prm.tol) <= ego_rounding(ex[1], fmax(change, prm.tol))) return false;
     }
     c_it = 1.0 / total;
     c_dt = acc[1] * c_it;
     b ^= 1;
     ++it;
     if (change <= prm.tol) {  // the same bits in every CTA of a cluster
-      done = 1;
+      done = EGO_DONE;
       break;
     }
   }
+  // a tolerance that rounding keeps this iteration above may be met by the other
+  if (!done && change <= prm.tol + 32.0 * ego_rounding(root, prm.tol)) return false;
   for (uint32_t r = threadIdx.x; r < R; r += T) g.out[g.lo + r] = y[b * ys + r] / total;
   *it_out = it;
   *done_out = done;
   *change_out = change;
+  return true;
+}
+
+// K sums over the rows [g.g_lo, g_hi) of a graph in the order `o` states:
+// row(i, a) adds row i's terms to a[0, K). The CTAs of a cluster take the
+// shares by turns, each in the launch's own threads, and every CTA adds the
+// shares' sums in order (slots: 2 turns x EGO_SHARES x 2). The barrier in it
+// publishes everything written before it.
+template <int C, int K, class F>
+__device__ __forceinline__ void ego_ordered_sums(const EgoGraph& g, uint32_t g_hi,
+                                                 const EgoOrder& o, double (&out)[K], double* sh,
+                                                 double* slots, int turn, F row) {
+  const uint32_t shares = g.nk >= o.split ? EGO_SHARES : 1;
+  const uint32_t per = (g.nk + shares - 1) / shares;
+  const uint32_t lane = threadIdx.x & 31;
+  double* mine = slots + (turn & 1) * EGO_SHARES * 2;
+  unsigned rank = 0;
+  if constexpr (C > 1) rank = cg::this_cluster().block_rank();
+  for (uint32_t r = rank; r < shares; r += C) {
+    const uint32_t lo = min(g_hi, g.g_lo + r * per), hi = min(g_hi, lo + per);
+    for (uint32_t t = threadIdx.x; t < o.threads; t += blockDim.x) {
+      double a[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j) a[j] = 0.0;
+      for (uint32_t i = lo + t; i < hi; i += o.threads) row(i, a);
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        a[j] = warp_sum(a[j]);
+        if (lane == 0) sh[32 * j + (t >> 5)] = a[j];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < K) {
+      double t = 0.0;
+      for (uint32_t k = 0; k < o.threads / 32; ++k) t += sh[32 * threadIdx.x + k];
+      if constexpr (C == 1) {
+        mine[r * 2 + threadIdx.x] = t;
+      } else {
+        cg::cluster_group cl = cg::this_cluster();
+        for (int q = 0; q < C; ++q)
+          cl.map_shared_rank(mine, (unsigned)q)[r * 2 + threadIdx.x] = t;
+      }
+    }
+    __syncthreads();  // sh is read
+  }
+  if constexpr (C > 1) cg::this_cluster().sync();
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    double t = 0.0;
+    for (uint32_t r = 0; r < shares; ++r) t += mine[r * 2 + j];
+    out[j] = t;
+  }
+}
+
+// The reference's iteration step by step (z = x / out with the dangling mass,
+// A z, the update, the division by the total, the L1 change), with two
+// reductions an iteration and every row's sum in CSR order. It runs, in global
+// memory, for a graph whose other iteration comes so near to the tolerance that
+// rounding would decide the sweep it stops on: about one in a hundred at 1e-12
+// (2,000 graphs: 2.01 ms a call without it, 2.12 with). In batches of 300 and
+// 2,000 graphs at 60 tolerances each, 25 of 1.7 million solves stopped a sweep
+// earlier or later than here without it.
+struct EgoEnd {
+  int32_t it, done;
+  double change;
+};
+template <int C>
+__device__ __noinline__ EgoEnd ego_normalising(const EgoGraph g, const uint32_t g_hi,
+                                               const EgoParams prm, const EgoOrder o, double* sh,
+                                               double* slots) {
+  const double inv_n = 1.0 / (double)g.nk;
+  const OpView<double>& op = g.op;
+  double* x = g.y;
+  double* y = g.y + g.n;
+  double* z = g.z;
+  int turn = 0;
+  double st[1];
+  ego_ordered_sums<C, 1>(g, g_hi, o, st, sh, slots, turn++, [&](uint32_t i, double* a) {
+    x[i] = inv_n;
+    const double out = g.outstr[i];
+    if (out > 0.0) {
+      z[i] = inv_n / out;
+    } else {
+      z[i] = 0.0;
+      a[0] += inv_n;
+    }
+  });
+  double stuck = st[0];
+  int32_t it = 0, done = 0;
+  double change = 0.0;
+  while (it < prm.max_iter) {
+    double tot[1];
+    ego_ordered_sums<C, 1>(g, g_hi, o, tot, sh, slots, turn++, [&](uint32_t i, double* a) {
+      // arcs in CSR order; four gathers in flight before their products
+      // are added in that order
+      double s = 0;
+      uint32_t k = op.off[i];
+      const uint32_t ke = op.off[i + 1];
+      for (; k + 4 <= ke; k += 4) {
+        double zk[4], wk[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          zk[u] = z[op.cols[k + u]];
+          wk[u] = op.vals ? op.vals[k + u] : 1.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s += wk[u] * zk[u];
+      }
+      for (; k < ke; ++k) {
+        const double w = op.vals ? op.vals[k] : 1.0;
+        s += w * z[op.cols[k]];
+      }
+      const double p = g.pers ? g.pers[i] / g.ps : inv_n;
+      const double jmp = prm.jump_uniform ? inv_n : p;
+      const double v = prm.d * (s + stuck * jmp) + (1.0 - prm.d) * p;
+      y[i] = v;
+      a[0] += v;
+    });
+    const double total = tot[0];
+    // the division, the change, and the next z and dangling mass
+    double cs[2];
+    ego_ordered_sums<C, 2>(g, g_hi, o, cs, sh, slots, turn++, [&](uint32_t i, double* a) {
+      const double v = y[i] / total;
+      y[i] = v;
+      a[0] += fabs(v - x[i]);
+      const double out = g.outstr[i];
+      if (out > 0.0) {
+        z[i] = v / out;
+      } else {
+        z[i] = 0.0;
+        a[1] += v;
+      }
+    });
+    change = cs[0];
+    stuck = cs[1];
+    double* t = x;
+    x = y;
+    y = t;
+    ++it;
+    if (change <= prm.tol) {  // the same bits in every CTA of a cluster
+      done = EGO_DONE;
+      break;
+    }
+  }
+  double none[1];
+  ego_ordered_sums<C, 1>(g, g_hi, o, none, sh, slots, turn,
+                         [&](uint32_t i, double*) { g.out[i] = x[i]; });
+  return {it, done, change};
 }
 
 // Row boundary k of C of a graph: the first row i with i + off[i] (from the
@@ -326,10 +510,12 @@ __device__ __forceinline__ uint32_t ego_bound(const uint32_t* off, uint32_t g_lo
   return lo;
 }
 
-template <int C, class MT>
+// A graph's solve; EGO_OPEN in *done where rounding decides and the launch is
+// not to run the normalising iteration itself.
+template <int C, class MT, bool BOTH>
 __device__ __forceinline__ void ego_solve(EgoGraph g, uint32_t g_hi, const EgoParams& prm,
-                          uint32_t sm_bytes, uint32_t* bounds, double* sh, double* slots,
-                          int32_t* it, int32_t* done, double* ch) {
+                          const EgoOrder& order, uint32_t sm_bytes, uint32_t* bounds, double* sh,
+                          double* slots, int32_t* it, int32_t* done, double* ch) {
   uint32_t amax;
   if constexpr (C == 1) {
     g.lo = g.g_lo;
@@ -354,12 +540,32 @@ __device__ __forceinline__ void ego_solve(EgoGraph g, uint32_t g_hi, const EgoPa
   size_t value_bytes = 0;
   if constexpr (!std::is_void<MT>::value) value_bytes = sizeof(MT);
   const size_t arcs = ego_arc_bytes(amax, value_bytes);
-  if (vec + arcs <= sm_bytes && g.nk <= 65536u)
-    ego_iterate<C, EGO_SMEM, MT>(g, prm, sh, slots, it, done, ch);
-  else if (vec <= sm_bytes)
-    ego_iterate<C, EGO_ARCS_GLOBAL, MT>(g, prm, sh, slots, it, done, ch);
-  else
-    ego_iterate<C, EGO_GLOBAL, MT>(g, prm, sh, slots, it, done, ch);
+  bool decided = false;
+  if (prm.tol <= 16.0 * DBL_EPSILON) {  // rounding decides in any case
+  } else if (vec + arcs <= sm_bytes && g.nk <= 65536u) {
+    decided = ego_iterate<C, EGO_SMEM, MT>(g, prm, sh, slots, it, done, ch);
+  } else if (vec <= sm_bytes) {
+    decided = ego_iterate<C, EGO_ARCS_GLOBAL, MT>(g, prm, sh, slots, it, done, ch);
+  } else {
+    decided = ego_iterate<C, EGO_GLOBAL, MT>(g, prm, sh, slots, it, done, ch);
+  }
+  if (decided) return;
+  if constexpr (BOTH) {
+    // every CTA has read the last sums before their places are used anew
+    if constexpr (C > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    const EgoEnd e = ego_normalising<C>(g, g_hi, prm, order, sh, slots);
+    *it = e.it;
+    *done = e.done;
+    *ch = e.change;
+  } else {
+    *done = EGO_OPEN;
+  }
+}
+
+// What a launch reports of a graph: 0 stopped at the tolerance, 1 at the cap, 2 open.
+__device__ __forceinline__ int32_t ego_status(int32_t done) {
+  return done == EGO_DONE ? 0 : done == EGO_CAPPED ? 1 : 2;
 }
 
 // The persistent launch. With clusters of C > 1 CTAs, each cluster first
@@ -368,16 +574,20 @@ __device__ __forceinline__ void ego_solve(EgoGraph g, uint32_t g_hi, const EgoPa
 // other graphs (order[nbig, count)) off queue[1] alone. Cluster barriers
 // are hardware barriers every CTA of the cluster executes the same number of
 // times: the graph index comes from rank 0's shared memory, and every CTA
-// stops a graph's iteration on the same bits.
-template <int C, class MT>
+// stops a graph's iteration on the same bits. BOTH: the launch runs the
+// normalising iteration itself where rounding decides; a single graph's launch
+// leaves that to the host (ego_one), since the call of it costs registers that
+// the other iteration then spills (500 nodes: 175.6 against 177.1 us a call,
+// 10,000 nodes 272 against 278). A large batch nearly always has such graphs.
+template <int C, class MT, bool BOTH>
 __global__ void __launch_bounds__(1024, 1)
 ego_pagerank(EgoGraph g, const uint32_t* __restrict__ node_off,
              const uint32_t* __restrict__ order, uint32_t count, uint32_t nbig,
-             unsigned int* __restrict__ queue, EgoParams prm, const double* __restrict__ psum,
-             uint32_t sm_bytes, int32_t* __restrict__ iters, int32_t* __restrict__ status,
-             double* __restrict__ changes) {
+             unsigned int* __restrict__ queue, EgoParams prm, EgoOrder sums,
+             const double* __restrict__ psum, uint32_t sm_bytes, int32_t* __restrict__ iters,
+             int32_t* __restrict__ status, double* __restrict__ changes) {
   __shared__ double sh[2 * 3 * 32];
-  __shared__ double slots[2 * C * 4];
+  __shared__ double slots[2 * (C > EGO_SHARES / 2 ? C : EGO_SHARES / 2) * 4];
   __shared__ uint32_t bounds[C + 1];
   __shared__ uint32_t g_sh;
   auto take = [&](uint32_t graph) {
@@ -400,10 +610,10 @@ ego_pagerank(EgoGraph g, const uint32_t* __restrict__ node_off,
       const uint32_t g_hi = take(graph);
       int32_t it = 0, done = 0;
       double ch = 0.0;
-      ego_solve<C, MT>(g, g_hi, prm, sm_bytes, bounds, sh, slots, &it, &done, &ch);
+      ego_solve<C, MT, BOTH>(g, g_hi, prm, sums, sm_bytes, bounds, sh, slots, &it, &done, &ch);
       if (rank == 0 && threadIdx.x == 0) {
         iters[graph] = it;
-        status[graph] = done ? 0 : 1;
+        status[graph] = ego_status(done);
         changes[graph] = ch;
       }
     }
@@ -418,14 +628,31 @@ ego_pagerank(EgoGraph g, const uint32_t* __restrict__ node_off,
     const uint32_t g_hi = take(graph);
     int32_t it = 0, done = 0;
     double ch = 0.0;
-    if (g.nk == 0) done = 1;
-    else ego_solve<1, MT>(g, g_hi, prm, sm_bytes, bounds, sh, slots, &it, &done, &ch);
+    if (g.nk == 0) done = EGO_DONE;
+    else ego_solve<1, MT, BOTH>(g, g_hi, prm, sums, sm_bytes, bounds, sh, slots, &it, &done, &ch);
     if (threadIdx.x == 0) {
       iters[graph] = it;
-      status[graph] = done ? 0 : 1;
+      status[graph] = ego_status(done);
       changes[graph] = ch;
     }
     __syncthreads();
+  }
+}
+
+// The normalising iteration of a single graph (nodes [0, g.nk)) on one cluster.
+template <int C>
+__global__ void __launch_bounds__(1024, 1)
+ego_one(EgoGraph g, EgoParams prm, EgoOrder sums, int32_t* __restrict__ iters,
+        int32_t* __restrict__ status, double* __restrict__ changes) {
+  __shared__ double sh[2 * 32];
+  __shared__ double slots[2 * EGO_SHARES * 2];
+  // (the first sums write into every CTA's slots: all have to be there)
+  if constexpr (C > 1) cg::this_cluster().sync();
+  const EgoEnd e = ego_normalising<C>(g, g.nk, prm, sums, sh, slots);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *iters = e.it;
+    *status = ego_status(e.done);
+    *changes = e.change;
   }
 }
 
@@ -483,16 +710,16 @@ constexpr uint32_t EGO_BATCH_SMEM = 32768;
 
 // CTAs (C == 1) or clusters of C CTAs of `threads` that fit on the device at
 // once with their shared memory (0 if none), per device and shape.
-template <int C, class MT>
+template <int C, class MT, bool BOTH>
 static int ego_resident(int threads, uint32_t smem) {
   static std::mutex mu;
   static std::map<std::tuple<int, int, uint32_t>, int> cache;
   int dev = 0;
   KNB_CUDA(cudaGetDevice(&dev));
   if (C > 8)
-    set_func_attr((const void*)ego_pagerank<C, MT>,
+    set_func_attr((const void*)ego_pagerank<C, MT, BOTH>,
                   cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  set_func_attr((const void*)ego_pagerank<C, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  set_func_attr((const void*)ego_pagerank<C, MT, BOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                 (int)ego_most_smem());
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find({dev, threads, smem});
@@ -500,8 +727,8 @@ static int ego_resident(int threads, uint32_t smem) {
   int fit = 0;
   if constexpr (C == 1) {
     int per_sm = 0, sms = 0;
-    KNB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ego_pagerank<1, MT>, threads,
-                                                           smem));
+    KNB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ego_pagerank<1, MT, BOTH>,
+                                                           threads, smem));
     KNB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     fit = std::max(1, per_sm) * sms;
   } else {
@@ -516,7 +743,7 @@ static int ego_resident(int threads, uint32_t smem) {
     cfg.dynamicSmemBytes = smem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&fit, (const void*)ego_pagerank<C, MT>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&fit, (const void*)ego_pagerank<C, MT, BOTH>, &cfg) != cudaSuccess) {
       cudaGetLastError();
       fit = 0;
     }
@@ -693,29 +920,39 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   base.op = op.view64();
   base.vals32 = op.has_vals && op.vals32_exact ? op.vals32.get() : nullptr;
   base.inv_out = op.inv_out64.get();
+  base.outstr = op.colsum.get();
   base.pers = pers ? P.dpers.get() : nullptr;
   base.ps = 1.0;
   base.y = P.y.get();
   base.z = P.z.get();
   base.n = n;
   base.out = scores;
-  auto launch_as = [&](auto mt, const EgoShape& shape, cudaStream_t st) -> uint32_t {
+  // The order of the normalising iteration's sums: that of a launch of clusters
+  // of 8 with the threads that were fastest for such a batch where every solve
+  // took it.
+  const bool many = op.nnz >= (1u << 20);
+  EgoOrder sums;
+  sums.threads = !many ? (count < (uint32_t)sms ? 1024 : 256)
+                 : !count || P.sizes[0] < 4096 ? 256 : n <= (1u << 18) ? 1024 : 512;
+  sums.split = std::max<uint32_t>(4096, n / ((uint32_t)sms * (2048 / sums.threads)));
+  auto launch_as = [&](auto mt, auto both, const EgoShape& shape, cudaStream_t st) -> uint32_t {
     using MT = typename decltype(mt)::type;
+    constexpr bool BOTH = decltype(both)::value;
     KNB_CUDA(cudaMemsetAsync(P.queue.get(), 0, 8, st));
     const int threads = shape.threads, C = shape.cluster;
     const uint32_t smem = shape.smem;
     int clusters = 0;
-    if (C == 4) clusters = ego_resident<4, MT>(threads, smem);
-    if (C == 8) clusters = ego_resident<8, MT>(threads, smem);
-    if (C == 16) clusters = ego_resident<16, MT>(threads, smem);
+    if (C == 4) clusters = ego_resident<4, MT, BOTH>(threads, smem);
+    if (C == 8) clusters = ego_resident<8, MT, BOTH>(threads, smem);
+    if (C == 16) clusters = ego_resident<16, MT, BOTH>(threads, smem);
     const uint32_t nbig = clusters > 0 ? big_count((uint64_t)clusters * C) : 0;
     const double* psum = pers ? P.dpers.get() + n : nullptr;
     if (nbig == 0) {
       const unsigned grid =
-          (unsigned)std::min<uint64_t>(count, (uint64_t)ego_resident<1, MT>(threads, smem));
-      ego_pagerank<1, MT><<<grid, threads, smem, st>>>(base, P.doff.get(), P.dorder.get(), count, 0u,
-                                                   P.queue.get(), prm, psum, smem, iters, status,
-                                                   changes);
+          (unsigned)std::min<uint64_t>(count, (uint64_t)ego_resident<1, MT, BOTH>(threads, smem));
+      ego_pagerank<1, MT, BOTH><<<grid, threads, smem, st>>>(
+          base, P.doff.get(), P.dorder.get(), count, 0u, P.queue.get(), prm, sums, psum, smem,
+          iters, status, changes);
       KNB_LAUNCH("ego_pagerank");
       return 0;
     }
@@ -736,18 +973,46 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     auto args = [&](auto fn) {
       KNB_CUDA(cudaLaunchKernelEx(&cfg, fn, base, (const uint32_t*)P.doff.get(),
                                   (const uint32_t*)P.dorder.get(), count, nbig, P.queue.get(), prm,
-                                  psum, smem, iters, status, changes));
+                                  sums, psum, smem, iters, status, changes));
     };
-    if (C == 4) args(ego_pagerank<4, MT>);
-    else if (C == 8) args(ego_pagerank<8, MT>);
-    else args(ego_pagerank<16, MT>);
+    if (C == 4) args(ego_pagerank<4, MT, BOTH>);
+    else if (C == 8) args(ego_pagerank<8, MT, BOTH>);
+    else args(ego_pagerank<16, MT, BOTH>);
     KNB_LAUNCH("ego_pagerank");
     return nbig;
   };
   auto launch = [&](const EgoShape& shape, cudaStream_t st) -> uint32_t {
-    if (!op.has_vals) return launch_as(TypeIs<void>{}, shape, st);
-    if (base.vals32) return launch_as(TypeIs<float>{}, shape, st);
-    return launch_as(TypeIs<double>{}, shape, st);
+    auto with = [&](auto mt) {
+      return count > 1 ? launch_as(mt, std::true_type{}, shape, st)
+                       : launch_as(mt, std::false_type{}, shape, st);
+    };
+    if (!op.has_vals) return with(TypeIs<void>{});
+    if (base.vals32) return with(TypeIs<float>{});
+    return with(TypeIs<double>{});
+  };
+  // The normalising iteration of a single graph, as wide as its sums' shares.
+  auto launch_one = [&] {
+    EgoGraph g1 = base;
+    g1.nk = n;
+    g1.ps = pers ? ps[0] : 1.0;
+    if (n < sums.split) {
+      ego_one<1><<<1, sums.threads, 0, s>>>(g1, prm, sums, iters, status, changes);
+    } else {
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = EGO_SHARES;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(EGO_SHARES);
+      cfg.blockDim = dim3(sums.threads);
+      cfg.stream = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      KNB_CUDA(cudaLaunchKernelEx(&cfg, ego_one<EGO_SHARES>, g1, prm, sums, iters, status,
+                                  changes));
+    }
+    KNB_LAUNCH("ego_one");
   };
   if (!P.t0) {
     KNB_CUDA(cudaEventCreate(&P.t0));
@@ -831,13 +1096,21 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     own.resize(meta);
     back = own.data();
   }
-  KNB_CUDA(cudaMemcpyAsync(back, together ? scores : changes, together ? all : meta,
-                           cudaMemcpyDeviceToHost, s));
-  KNB_CUDA(cudaStreamSynchronize(s));
+  auto fetch = [&] {
+    KNB_CUDA(cudaMemcpyAsync(back, together ? scores : changes, together ? all : meta,
+                             cudaMemcpyDeviceToHost, s));
+    KNB_CUDA(cudaStreamSynchronize(s));
+  };
+  fetch();
   const double* hscores = reinterpret_cast<const double*>(back);
   const double* hchange = together ? hscores + n : hscores;
   const int32_t* hit = reinterpret_cast<const int32_t*>(hchange + count);
   const int32_t* hst = hit + count;
+  if (count == 1 && hst[0] == 2) {
+    launch_one();
+    KNB_CUDA(cudaEventRecord(P.t1, s));
+    fetch();
+  }
   float ms = 0;
   KNB_CUDA(cudaEventElapsedTime(&ms, P.t0, P.t1));
   for (uint32_t k = 0; k < count; ++k)
