@@ -4,8 +4,9 @@
 // One sweep is two kernels: the sparse product with the PageRank update
 // fused into its epilogue (by default the sliced sweep slice_spmv, else a
 // merge-path kernel, with PagerankEpi) and the split-row / reduction kernel
-// (split_rows), whose last CTA also computes the exact L1 change when the
-// fused estimate is too close to the tolerance.
+// (split_rows). Where the fused L1 change is too close to the tolerance the
+// iteration is held, and a kernel over the whole grid computes the exact change
+// (run_phase).
 //
 // Normalisation is folded into the next sweep. The device stores the
 // unnormalised iterate y_k and z_k = y_k / out (0 for dangling nodes); with
@@ -33,6 +34,7 @@
 #include <mutex>
 #include <chrono>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -46,7 +48,6 @@ template <class VT, bool PV, bool JU, bool EXACT>
 struct PagerankEpi {
   static constexpr int NACC = 3;
   static constexpr bool SUMS = true;  // total, dangling mass, change
-  static constexpr bool DECIDES = EXACT;
   const VT* y_old;
   VT* y_new;
   VT* z_new;
@@ -54,7 +55,6 @@ struct PagerankEpi {
   const double* p;  // personalization (rescaled), when PV
   double d;
   double pu;        // 1 / n
-  uint32_t n;
   VT c_it = 0, c_dt = 0;
 
   __device__ __forceinline__ void prepare(const IterState* st) {
@@ -90,11 +90,6 @@ struct PagerankEpi {
     row_in(g, s, fetch(g), a);
   }
 
-  // |x_new - x_old| of node i once the total T is known (y_new comes from
-  // other CTAs, past L1)
-  __device__ __forceinline__ double exact_change(uint32_t i, double T, double ip) const {
-    return fabs((double)__ldcg(y_new + i) / T - (double)y_old[i] * ip);
-  }
   __device__ void finish(IterState* st, const double* tot) const {
     const double T = tot[0], D = tot[1], ch = tot[2];
     st->prev_inv_total = st->inv_total;
@@ -110,7 +105,7 @@ struct PagerankEpi {
       st->slack = slack;
       amb = fabs(ch - st->tol) <= slack;
     }
-    if (amb) st->ambiguous = 1;
+    if (amb) st->stopped = HELD;
     else if (ch <= st->tol) st->converged = 1;
     else if (st->iter >= st->max_iter) st->stopped = 1;
   }
@@ -130,7 +125,6 @@ template <class VT, bool ANCHOR, bool PV, bool JU, bool EXACT>
 struct RefineEpi {
   static constexpr int NACC = 3;
   static constexpr bool SUMS = true;
-  static constexpr bool DECIDES = EXACT;
   const double* y_ref;
   double* s_ref;        // written by the anchor sweep, read by refinement sweeps
   const float* e_old;   // refinement sweeps: e of the input iterate
@@ -140,7 +134,6 @@ struct RefineEpi {
   const double* p;
   double d;
   double pu;
-  uint32_t n;
   double c_it = 0, c_dt = 0;
 
   __device__ __forceinline__ void prepare(const IterState* st) {
@@ -192,11 +185,6 @@ struct RefineEpi {
     row_in(g, s_in, fetch(g), a);
   }
 
-  __device__ __forceinline__ double exact_change(uint32_t i, double T, double ip) const {
-    const double yr = y_ref[i];
-    const double yo = ANCHOR ? yr : yr + (double)e_old[i];
-    return fabs((yr + (double)__ldcg(e_new + i)) / T - yo * ip);
-  }
   __device__ void finish(IterState* st, const double* tot) const {
     PagerankEpi<double, PV, JU, EXACT> base;
     base.finish(st, tot);
@@ -257,6 +245,40 @@ __global__ void pr_init(VT* __restrict__ y, VT* __restrict__ z, const VT* __rest
     st->dterm = r[1];
     st->total = r[0];
     st->prev_inv_total = 1.0;
+    st->ticket = 0;
+  }
+}
+
+// Exact L1 change sum |y_new / T - y_old * prev_inv_total| of a held iteration,
+// which goes on or ends by it. The iterates are y, or with y_ref (refinement
+// sweeps) y_ref + y (y_old null: y_ref itself, the anchor sweep's input). Bound
+// by the two or three vectors it streams. A solve of 2^23 nodes that meets one
+// open change takes 20.9 ms against 20.7 of one that meets none (2^17 nodes 0.84
+// against 0.73, the host's wait); with one CTA, the last of split_rows, adding
+// alone it took 39.8.
+template <class VT>
+__global__ void pr_exact_change(const double* __restrict__ y_ref, const VT* y_old,
+                                const VT* y_new, uint32_t n, double* __restrict__ part,
+                                IterState* st) {
+  chain_wait();
+  if (st->stopped != HELD) return;
+  __shared__ double sh[VT_THREADS / 32];
+  const double T = st->total, ip = st->prev_inv_total;
+  double a = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double yr = y_ref ? y_ref[i] : 0.0;
+    const double yo = y_old ? yr + (double)y_old[i] : yr;
+    a += fabs((yr + (double)y_new[i]) / T - yo * ip);
+  }
+  a = block_sum(a, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = a;
+  if (!last_block(&st->ticket)) return;
+  double r[1];
+  reduce_parts<1>(part, gridDim.x, r, sh);
+  if (threadIdx.x == 0) {
+    st->change = r[0];
+    st->converged = r[0] <= st->tol ? 1 : 0;
+    st->stopped = r[0] > st->tol && st->iter >= st->max_iter ? 1 : 0;
     st->ticket = 0;
   }
 }
@@ -744,7 +766,6 @@ static void launch_sweep(const Operator& op, const Partition& P, const SweepBuff
   e.p = B.p;
   e.d = d;
   e.pu = 1.0 / (double)op.n;
-  e.n = op.n;
   OpView<MT> v;
   if constexpr (sizeof(MT) == 8) v = B.v64; else v = B.v32;
   launch_spmv<VT, MT, Epi, VAR, IPT>(op, P, v, (const VT*)B.z[buf], e, (VT*)B.carry,
@@ -814,7 +835,6 @@ static void launch_refine(const Operator& op, const Partition& P, const SweepBuf
   e.p = B.p;
   e.d = d;
   e.pu = 1.0 / (double)op.n;
-  e.n = op.n;
   launch_spmv<float, float, Epi, VAR, IPT>(op, P, B.v32, (const float*)B.z[buf], e,
                                            (float*)B.carry, (float*)B.head, B.part1, B.part2,
                                            B.st, s, ev0, ev1, B.so);
@@ -838,7 +858,6 @@ static void launch_anchor(const Operator& op, const Partition& P, const SweepBuf
   e.p = B.p;
   e.d = d;
   e.pu = 1.0 / (double)op.n;
-  e.n = op.n;
   OpView<MT> v;
   if constexpr (sizeof(MT) == 8) v = B.v64; else v = B.v32;
   launch_spmv<double, MT, Epi, VAR, IPT>(op, P, v, z_ref, e, carry64, head64, B.part1, B.part2,
@@ -948,38 +967,67 @@ struct PhaseResult {
   int launches = 0;
 };
 
+// Computes the exact change of sweep `iter` (counted from 1), if it is held.
+using ExactFn = std::function<void(int32_t iter)>;
+
 // Runs sweeps until the phase's state converges or stops. The host keeps
 // one batch of `U` sweeps in flight ahead of the state it inspects, so the
 // GPU never waits for the host; sweeps after convergence exit at once.
+// Sweeps after one whose change is left open exit as well: the host sees it,
+// has the exact change computed, and goes on from there with a kernel for it
+// behind every sweep, which does nothing unless that sweep is held. How often
+// that happens depends on the tolerance: a solve meets an open change with a
+// probability of about 4 |1 - T| / (0.16 tol), T the sum of the iterate
+// (|1 - T| about 1e-15: a few in a hundred solves at 1e-12, most sweeps near
+// 1e-15), so the kernel runs only in solves that met one (it took 2 us of every
+// sweep).
 static PhaseResult run_phase(SweepFn fn, const Operator& op, const Partition& P,
                              const SweepBuffers& B, double d, cudaStream_t s,
                              PrWorkspace& ws, IterState* h_state /* pinned, 2 slots */,
-                             double* timing_ms, int64_t* timing_n, int32_t iter0 = 0) {
+                             double* timing_ms, int64_t* timing_n, int32_t iter0 = 0,
+                             const ExactFn& exact = nullptr) {
   const int U = 8;
   PhaseResult r;
   int batch = 0;
   size_t nev = 0;
-  bool finished = false;
+  std::vector<size_t> timed;  // the first event of each sweep
+  int32_t at = iter0;         // sweeps enqueued, but for those behind a held one
+  bool follow = false;
   auto enqueue = [&](int b) {
     for (int k = 0; k < U; ++k) {
       cudaEvent_t e0 = nullptr, e1 = nullptr;
       if (g_timing_on) {
+        timed.push_back(nev);
         e0 = ws.timing_event(nev++);
         e1 = ws.timing_event(nev++);
       }
-      fn(op, P, B, k & 1, d, s, e0, e1);
+      fn(op, P, B, (at - iter0) & 1, d, s, e0, e1);
       r.launches += 2;
+      ++at;
+      if (follow) {
+        exact(at);
+        ++r.launches;
+      }
     }
     KNB_CUDA(cudaMemcpyAsync(&h_state[b & 1], B.st, sizeof(IterState), cudaMemcpyDeviceToHost, s));
     KNB_CUDA(cudaEventRecord(ws.done[b & 1], s));
   };
   enqueue(batch);
-  while (!finished) {
+  for (;;) {
     enqueue(batch + 1);
     KNB_CUDA(cudaEventSynchronize(ws.done[batch & 1]));
-    const IterState& hs = h_state[batch & 1];
-    if (hs.converged || hs.stopped) finished = true;
+    const IterState hs = h_state[batch & 1];
     ++batch;
+    if (hs.converged || hs.stopped == 1) break;
+    if (hs.stopped != HELD) continue;
+    // everything enqueued behind sweep hs.iter has done nothing
+    KNB_CUDA(cudaEventSynchronize(ws.done[batch & 1]));
+    follow = true;
+    at = hs.iter;
+    timed.resize(std::min(timed.size(), (size_t)(at - iter0)));
+    exact(at);
+    ++r.launches;
+    enqueue(batch);
   }
   KNB_CUDA(cudaMemcpyAsync(&h_state[0], B.st, sizeof(IterState), cudaMemcpyDeviceToHost, s));
   KNB_CUDA(cudaStreamSynchronize(s));
@@ -990,15 +1038,11 @@ static PhaseResult run_phase(SweepFn fn, const Operator& op, const Partition& P,
   r.stopped = fin.stopped;
   r.change = fin.change;
   // Only sweeps that did work count for the timing (later ones exit at once).
-  if (g_timing_on) {
-    for (size_t k = 0; k + 1 < nev; k += 2) {
-      if ((int64_t)(k / 2) < fin.iter - iter0) {
-        float ms = 0;
-        KNB_CUDA(cudaEventElapsedTime(&ms, ws.pool[k], ws.pool[k + 1]));
-        *timing_ms += ms;
-        *timing_n += 1;
-      }
-    }
+  for (size_t k = 0; k < timed.size() && (int64_t)k < fin.iter - iter0; ++k) {
+    float ms = 0;
+    KNB_CUDA(cudaEventElapsedTime(&ms, ws.pool[timed[k]], ws.pool[timed[k] + 1]));
+    *timing_ms += ms;
+    *timing_n += 1;
   }
   return r;
 }
@@ -1365,7 +1409,13 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
          g_timing_on ? ws.a0 : nullptr, g_timing_on ? ws.a1 : nullptr);
       launches += 2;
       SweepFn fr = pick_refine(var_r, ipt_r, pv, ju);
-      r64 = run_phase(fr, op, *PR, R, prm.damping, s, ws, hstate, &tmsr, &tnr, 1);
+      // sweep 1 is the anchor, which writes the first of the two buffers of e
+      auto exact = [&](int32_t iter) {
+        launch_chained(pr_exact_change<float>, gv, VT_THREADS, 0, s, R.y_ref,
+                       iter == 1 ? nullptr : (const float*)R.y[iter & 1],
+                       (const float*)R.y[(iter & 1) ^ 1], n, ws.part3.get(), st + 1);
+      };
+      r64 = run_phase(fr, op, *PR, R, prm.damping, s, ws, hstate, &tmsr, &tnr, 1, exact);
       if (g_timing_on) {
         float ms = 0;
         KNB_CUDA(cudaEventElapsedTime(&ms, ws.a0, ws.a1));
@@ -1379,7 +1429,12 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
       B.so = SO;
       SweepFn fn = use32 ? pick_kernel<double, float, true>(var64, ipt64, pv, ju)
                          : pick_kernel<double, double, true>(var64, ipt64, pv, ju);
-      r64 = run_phase(fn, op, *P64, B, prm.damping, s, ws, hstate, &tms64, &tn64);
+      auto exact = [&](int32_t iter) {
+        launch_chained(pr_exact_change<double>, gv, VT_THREADS, 0, s, nullptr,
+                       (const double*)B.y[(iter & 1) ^ 1], (const double*)B.y[iter & 1], n,
+                       ws.part3.get(), st + 1);
+      };
+      r64 = run_phase(fn, op, *P64, B, prm.damping, s, ws, hstate, &tms64, &tn64, 0, exact);
     }
     launches += r64.launches;
     if (!r64.converged)

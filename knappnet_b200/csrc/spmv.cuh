@@ -73,12 +73,15 @@ struct IterState {
   int32_t iter;           // sweeps done
   int32_t max_iter;       // sweep cap
   int32_t converged;      // 1 once change <= tol
-  int32_t stopped;        // 1 when the cap is reached without convergence
-  int32_t ambiguous;      // 1 when the exact change must decide
+  int32_t stopped;        // 1 when the cap is reached without convergence, or HELD
+  int32_t ambiguous;      // 1 once the adjoint has extrapolated
   uint32_t ticket;        // CTA counter of the last-CTA reductions
   uint32_t ticket2;
   int32_t fault;          // 1 when a sweep gave up waiting for its staged copies
 };
+
+// IterState::stopped of an iteration that waits for its exact change.
+constexpr int32_t HELD = 2;
 
 __device__ __forceinline__ bool iteration_done(const IterState* st) {
   return st->converged != 0 || st->stopped != 0;
@@ -637,11 +640,6 @@ constexpr size_t tile_smem_bytes() {
 // Epi::finish. Every
 // sum has a fixed association, so results do not change from run to run.
 // Partials written by other CTAs are read with ld.global.cg (L2, not L1).
-// Epilogues that may leave the decision open (st->ambiguous) declare DECIDES
-// and give the exact change of node i: the last CTA sums it alone (about one
-// solve in a thousand, when the fused change is within rounding of the
-// tolerance; a kernel of its own for that, launched after every sweep, took 2
-// us and a launch's gap each time).
 //
 // Bound by latency: the bytes are few, but each row is a chain of loads (the
 // row, its partials, its node's inputs). So all that does not depend on the
@@ -688,15 +686,6 @@ __device__ __forceinline__ VT add_carries(VT sum, const VT* __restrict__ carry, 
   }
   return sum;
 }
-
-template <class E, class = void>
-struct EpiDecides {
-  static constexpr bool value = false;
-};
-template <class E>
-struct EpiDecides<E, std::void_t<decltype(E::DECIDES)>> {
-  static constexpr bool value = E::DECIDES;
-};
 
 // CTAs of split_rows: what its rows and partials need, at most SPLIT_CTAS
 // (four per SM; a sweep of 3.6M arcs spent 9 us in 296 that it did not need).
@@ -830,20 +819,6 @@ split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort,
   if (tid == 0) {
     epi.finish(st, tot);
     st->ticket = 0;
-  }
-  if constexpr (EpiDecides<Epi>::value) {
-    __syncthreads();
-    if (st->ambiguous == 0) return;
-    const double T2 = st->total, ip = st->prev_inv_total;
-    double ch = 0;
-    for (uint32_t i = tid; i < epi.n; i += T) ch += epi.exact_change(i, T2, ip);
-    ch = block_sum(ch, red[0]);
-    if (tid == 0) {
-      st->change = ch;
-      st->ambiguous = 0;
-      if (ch <= st->tol) st->converged = 1;
-      else if (st->iter >= st->max_iter) st->stopped = 1;
-    }
   }
 }
 
