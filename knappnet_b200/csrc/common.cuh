@@ -44,9 +44,14 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
   return p;
 }
 
-// Read-only loads with an L2 policy (ld.global.nc.L2::cache_hint). They are
-// not `volatile`, so the compiler may batch independent loads ahead of their
-// uses (a volatile asm would keep every gather in program order).
+// Loads with an L2 policy (L2::cache_hint). ld_stream is for arrays that are
+// laid out once and read-only while a kernel lives (ld.global.nc, not volatile:
+// the compiler may move them). ld_keep and ld_keep_na gather the iterate, which
+// the kernel before may still be writing when a chained kernel starts: ordinary
+// loads, which no volatile asm, chain_wait's among them, is moved across. Sweeps
+// take the same time either way (FP64 Katz on 2^24 arcs 7.8 to 7.9 ms a call,
+// R-MAT with 2^28 arcs 23.8; a pointer made to depend on the wait instead costs
+// its registers, Katz 8.1).
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t* p, uint64_t pol) {
   uint32_t v;
   asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u32 %0, [%1], %2;"
@@ -67,12 +72,12 @@ __device__ __forceinline__ double ld_stream(const double* p, uint64_t pol) {
 }
 __device__ __forceinline__ float ld_keep(const float* p, uint64_t pol) {
   float v;
-  asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ double ld_keep(const double* p, uint64_t pol) {
   double v;
-  asm("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 
@@ -96,12 +101,12 @@ __device__ __forceinline__ void ld_stream4(const double* p, uint64_t pol, double
 // Gathers that skip L1 allocation (the L2 policy still applies).
 __device__ __forceinline__ float ld_keep_na(const float* p, uint64_t pol) {
   float v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ double ld_keep_na(const double* p, uint64_t pol) {
   double v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 
@@ -204,7 +209,10 @@ inline void set_func_attr(const void* fn, cudaFuncAttribute attr, int value) {
 // for that one's end before it touches memory; every kernel launched this way
 // calls chain_wait first. It hides most of the 3 to 4 us that a kernel boundary
 // costs between sweeps of a few microseconds. Launched the ordinary way,
-// chain_wait returns at once.
+// chain_wait returns at once. What the kernel before writes (iterates, partials,
+// the state) is not read-only while a chained kernel lives: it takes no
+// `const __restrict__` pointer to it, which would let the compiler read it
+// through the non-coherent path or before the wait.
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

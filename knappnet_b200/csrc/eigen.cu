@@ -783,8 +783,8 @@ inline unsigned project_groups(int k, int mode) {
 // once; every dot product is summed per thread in row order, then per warp and
 // CTA and over the row blocks in fixed order, as in a one-dimensional sweep.
 __global__ void __launch_bounds__(VB_T)
-lz_project(const double* __restrict__ V, size_t dim, int lo, int hi, const double* __restrict__ w,
-           int mode, double* __restrict__ part, LzState* st, const IterState* ist) {
+lz_project(const double* V, size_t dim, int lo, int hi, const double* w, int mode,
+           double* __restrict__ part, LzState* st, const IterState* ist) {
   chain_wait();
   if (ist && iteration_done(ist)) return;
   if (mode == 2 && !st->need2) return;
@@ -848,7 +848,7 @@ lz_project(const double* __restrict__ V, size_t dim, int lo, int hi, const doubl
 // Each thread keeps its 16 values of w in registers and subtracts one basis
 // vector at a time from all of them, in basis order.
 __global__ void __launch_bounds__(VB_T)
-lz_subtract(const double* __restrict__ V, size_t dim, int lo, int hi, double* __restrict__ w,
+lz_subtract(const double* V, size_t dim, int lo, int hi, double* __restrict__ w,
             int mode, double* __restrict__ part, LzState* st, const IterState* ist) {
   chain_wait();
   if (ist && iteration_done(ist)) return;
@@ -948,7 +948,7 @@ __global__ void lz_end(LzState* st, IterState* ist, double* hm, int m, int j) {
 }
 
 // v = w / beta into basis column `col` (and its FP32 copy); hm(col, col-1).
-__global__ void lz_next(double* __restrict__ V, size_t dim, int col, const double* __restrict__ w,
+__global__ void lz_next(double* __restrict__ V, size_t dim, int col, const double* w,
                         float* __restrict__ v32, double* hm, int m, const LzState* st,
                         const IterState* ist, int set_hm) {
   chain_wait();

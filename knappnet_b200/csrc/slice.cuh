@@ -80,8 +80,8 @@ __device__ __forceinline__ VT slice_fma(const MT* vals, MT w, VT x, VT s) {
 // 32-arc boundary at or below lo (so each load instruction touches one
 // 128-byte line); U arcs per lane in flight; warp butterfly at the end.
 template <class VT, class MT, int U, int GNA>
-__device__ __forceinline__ VT slice_long_sum(const SliceView<MT>& op, const VT* __restrict__ xg,
-                                             uint32_t lo, uint32_t hi, int lane, uint32_t l1_hot,
+__device__ __forceinline__ VT slice_long_sum(const SliceView<MT>& op, const VT* xg, uint32_t lo,
+                                             uint32_t hi, int lane, uint32_t l1_hot,
                                              uint64_t pol_stream, uint64_t pol_keep,
                                              const VT* smem, uint32_t smem_n) {
   VT s = VT(0);
@@ -116,9 +116,9 @@ __device__ __forceinline__ VT slice_long_sum(const SliceView<MT>& op, const VT* 
 // those columns read it there instead of sending a request to L1 and L2.
 template <class VT, class MT, class Epi, int U, int WPB, int MINB, int GNA>
 __global__ void __launch_bounds__(WPB * 32, MINB)
-slice_spmv(SliceView<MT> op, const VT* __restrict__ xg, Epi epi_in, VT* __restrict__ carry,
-           VT* __restrict__ head, double* __restrict__ part, const IterState* __restrict__ st,
-           uint32_t l1_hot, uint32_t smem_n) {
+slice_spmv(SliceView<MT> op, const VT* xg, Epi epi_in, VT* __restrict__ carry,
+           VT* __restrict__ head, double* __restrict__ part, const IterState* st, uint32_t l1_hot,
+           uint32_t smem_n) {
   chain_wait();
   if (st && iteration_done(st)) return;
   extern __shared__ __align__(16) unsigned char slice_smem[];
@@ -127,7 +127,7 @@ slice_spmv(SliceView<MT> op, const VT* __restrict__ xg, Epi epi_in, VT* __restri
     const uint4* src = reinterpret_cast<const uint4*>(xg);
     uint4* dst = reinterpret_cast<uint4*>(slice_smem);
     const uint32_t nvec = smem_n * (uint32_t)sizeof(VT) / 16u;
-    for (uint32_t i = threadIdx.x; i < nvec; i += WPB * 32) dst[i] = __ldg(src + i);
+    for (uint32_t i = threadIdx.x; i < nvec; i += WPB * 32) dst[i] = src[i];
     __syncthreads();
     hot = reinterpret_cast<const VT*>(slice_smem);
   }

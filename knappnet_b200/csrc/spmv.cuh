@@ -407,10 +407,9 @@ constexpr int warp_min_blocks() {
 // gathers pass through.
 template <class VT, class MT, class Epi, int IPT, int WPB, int GNA = 0>
 __global__ void __launch_bounds__(WPB * 32, (warp_min_blocks<VT, IPT, WPB>()))
-warp_spmv(OpView<MT> op, const VT* __restrict__ xg, Epi epi_in,
-          const TileCoord* __restrict__ coords, uint32_t ntiles, VT* __restrict__ carry,
-          VT* __restrict__ head, double* __restrict__ part, const IterState* __restrict__ st,
-          uint32_t l1_hot) {
+warp_spmv(OpView<MT> op, const VT* xg, Epi epi_in, const TileCoord* __restrict__ coords,
+          uint32_t ntiles, VT* __restrict__ carry, VT* __restrict__ head,
+          double* __restrict__ part, const IterState* st, uint32_t l1_hot) {
   using S = WarpSmem<VT, IPT>;
   chain_wait();
   if (st && iteration_done(st)) return;
@@ -674,8 +673,7 @@ struct EpiFetch<E, std::void_t<typename E::In>> {
 // sum + carry[q], carry[q + STEP], ... below `last`, added in that order with
 // U of them in flight.
 template <int U, int STEP, class VT>
-__device__ __forceinline__ VT add_carries(VT sum, const VT* __restrict__ carry, uint32_t q,
-                                          uint32_t last) {
+__device__ __forceinline__ VT add_carries(VT sum, const VT* carry, uint32_t q, uint32_t last) {
   for (; q < last; q += U * STEP) {
     VT c[U];
 #pragma unroll
@@ -698,10 +696,9 @@ inline unsigned split_grid(uint32_t nsplit, uint32_t nshort, uint32_t npart) {
 
 template <class VT, class Epi>
 __global__ void __launch_bounds__(SPMV_THREADS)
-split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort,
-           const VT* __restrict__ carry,
-           const VT* __restrict__ head, Epi epi_in, const double* __restrict__ part1,
-           uint32_t npart, double* __restrict__ part2, IterState* st) {
+split_rows(const SplitRow* __restrict__ sr, uint32_t nsr, uint32_t nshort, const VT* carry,
+           const VT* head, Epi epi_in, const double* part1, uint32_t npart,
+           double* __restrict__ part2, IterState* st) {
   constexpr int T = SPMV_THREADS;
   constexpr int NA = Epi::NACC;
   chain_wait();
