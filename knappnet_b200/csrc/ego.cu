@@ -767,6 +767,7 @@ struct EgoPlan : Workspace {
   bool tuned = false;          // this batch's shape is chosen
   EgoShape pick;
   EgoShape shape;              // of the instantiated launch
+  int64_t pin_big = 0;         // the large-graph threshold it was pinned to
   uint32_t nbig = 0;           // graphs it gives to clusters
   DevBuf<uint32_t> doff, dorder;
   DevBuf<double> dpers, y, z;
@@ -906,8 +907,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   // nodes (by default max(4096, n / CTAs of the grid), so no graph holds
   // much more than a CTA's share of the batch) are each split over a
   // cluster; the others go one per CTA. Returns the graphs given to clusters.
+  const int64_t pin_big = g_ego_big.load();
   auto big_count = [&](uint64_t ctas) {
-    const int64_t pin_big = g_ego_big.load();
     const uint64_t big =
         pin_big > 0 ? (uint64_t)pin_big
         : count == 1 ? 1  // the shape chosen for it says whether it is split
@@ -1068,7 +1069,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   EgoShape shape = P.pick;
   if (pin_t) shape.threads = pin_t;
   if (pin_c) shape.cluster = pin_c;
-  if (!P.exec || !(P.shape == shape) || P.pers != pers || !same_params(P.prm, prm)) {
+  if (!P.exec || !(P.shape == shape) || P.pin_big != pin_big || P.pers != pers ||
+      !same_params(P.prm, prm)) {
     P.drop_graph();
     cudaStream_t cs;
     KNB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -1079,6 +1081,7 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     KNB_CUDA(cudaGraphInstantiate(&P.exec, P.graph, 0));
     KNB_CUDA(cudaStreamDestroy(cs));
     P.shape = shape;
+    P.pin_big = pin_big;
     P.pers = pers;
     P.prm = prm;
     ++P.instantiations;

@@ -1,0 +1,31 @@
+"""The kept launch of a packed batch follows what it depends on: the tuning keys
+and the teleport vector of the call, not those of an earlier one."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import knappnet_b200 as K
+
+pytestmark = pytest.mark.gpu
+
+
+def packed(sizes, degree, seed):
+    rng = np.random.default_rng(seed)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    which = np.repeat(np.arange(len(sizes)), np.maximum(1, np.asarray(sizes) * degree // 2))
+    a, b = (off[which] + (rng.random(len(which)) * np.asarray(sizes)[which]).astype(np.int64)
+            for _ in range(2))
+    return K.Graph(int(off[-1]), a, b, None, False), off
+
+
+def test_the_large_graph_threshold_of_the_call():
+    sizes = [6000, 3000, 1500, 700, 300]
+    g, off = packed(sizes, 8, 1)
+    try:
+        for big, split in ((0, 1), (1000, 3), (500, 4), (0, 1)):
+            K.set_tuning(K.TUNE_EGO_BIG_NODES, big)
+            _, _, info = g.pagerank_graphs(off)
+            assert info.iterations_fp32 == split  # graphs split over a cluster
+    finally:
+        K.set_tuning(K.TUNE_EGO_BIG_NODES, 0)
