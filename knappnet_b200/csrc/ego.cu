@@ -764,7 +764,8 @@ struct EgoPlan : Workspace {
   bool pers = false;
   EgoParams prm{};
   std::vector<uint32_t> sizes;  // node counts of the graphs, largest first
-  bool tuned = false;          // this batch's shape is chosen
+  bool tuned = false;          // this batch's shape is chosen, with these pinned:
+  int pin_t = 0, pin_c = 0;
   EgoShape pick;
   EgoShape shape;              // of the instantiated launch
   int64_t pin_big = 0;         // the large-graph threshold it was pinned to
@@ -1031,7 +1032,7 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   //   enough to be split (100 graphs up to 20,000 nodes: 390 us against 626
   //   with 256 threads), else 256 threads.
   const int pin_t = g_ego_threads.load(), pin_c = g_ego_cluster.load();
-  if (!P.tuned) {
+  if (!P.tuned || P.pin_t != pin_t || P.pin_c != pin_c) {
     EgoShape pick;
     const uint32_t most = ego_most_smem();
     if (count == 1) {
@@ -1049,6 +1050,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
         float best = 1e30f;
         for (EgoShape c : {EgoShape{256, 8, EGO_BATCH_SMEM}, EgoShape{256, 16, EGO_BATCH_SMEM},
                            EgoShape{512, 16, EGO_BATCH_SMEM}, EgoShape{1024, 16, EGO_BATCH_SMEM}}) {
+          if (pin_t) c.threads = pin_t;
+          if (pin_c) c.cluster = pin_c;
           if (c.cluster == 16 && c.threads == 256 && !split) continue;
           KNB_CUDA(cudaEventRecord(P.t0, s));
           launch(c, s);
@@ -1065,6 +1068,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     }
     P.pick = pick;
     P.tuned = true;
+    P.pin_t = pin_t;
+    P.pin_c = pin_c;
   }
   EgoShape shape = P.pick;
   if (pin_t) shape.threads = pin_t;

@@ -29,3 +29,25 @@ def test_the_large_graph_threshold_of_the_call():
             assert info.iterations_fp32 == split  # graphs split over a cluster
     finally:
         K.set_tuning(K.TUNE_EGO_BIG_NODES, 0)
+
+
+def test_a_pinned_shape_does_not_outlive_its_pins():
+    rng = np.random.default_rng(2)
+    sizes = np.concatenate([[30_000], rng.integers(50, 400, 1500)])
+    fresh = set()
+    for _ in range(3):  # timed on the batch itself
+        g, off = packed(sizes, 12, 3)
+        _, _, info = g.pagerank_graphs(off)
+        fresh.add((info.sweep_kernel, info.hot_columns))
+    g, off = packed(sizes, 12, 3)
+    try:
+        for threads, cluster in ((128, 4), (128, 0), (0, 4)):
+            K.set_tuning(K.TUNE_EGO_THREADS, threads)
+            K.set_tuning(K.TUNE_EGO_CLUSTER, cluster)
+            _, _, info = g.pagerank_graphs(off)
+            assert threads in (0, info.sweep_kernel) and cluster in (0, info.hot_columns)
+    finally:
+        K.set_tuning(K.TUNE_EGO_THREADS, 0)
+        K.set_tuning(K.TUNE_EGO_CLUSTER, 0)
+    _, _, info = g.pagerank_graphs(off)
+    assert (info.sweep_kernel, info.hot_columns) in fresh
