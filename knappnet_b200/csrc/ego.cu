@@ -1032,7 +1032,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   //   enough to be split (100 graphs up to 20,000 nodes: 390 us against 626
   //   with 256 threads), else 256 threads.
   const int pin_t = g_ego_threads.load(), pin_c = g_ego_cluster.load();
-  if (!P.tuned || P.pin_t != pin_t || P.pin_c != pin_c) {
+  // (a single graph's depends on whether it has a teleport vector to hold)
+  if (!P.tuned || count == 1 || P.pin_t != pin_t || P.pin_c != pin_c) {
     EgoShape pick;
     const uint32_t most = ego_most_smem();
     if (count == 1) {

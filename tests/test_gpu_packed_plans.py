@@ -51,3 +51,14 @@ def test_a_pinned_shape_does_not_outlive_its_pins():
         K.set_tuning(K.TUNE_EGO_CLUSTER, 0)
     _, _, info = g.pagerank_graphs(off)
     assert (info.sweep_kernel, info.hot_columns) in fresh
+
+
+# 10,000 nodes and arcs fit a cluster of 8 without a teleport vector only
+def test_a_single_graphs_shape_follows_its_own_teleport():
+    n = 10_000
+    rng = np.random.default_rng(4)
+    g = K.Graph(n, rng.integers(0, n, n), rng.integers(0, n, n), None, True)
+    pers = rng.random(n)
+    for p, cluster in ((pers, 16), (None, 8), (pers, 16), (None, 8)):
+        _, _, info = g.pagerank_graphs([0, n], personalization=p)
+        assert info.hot_columns == cluster
