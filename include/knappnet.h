@@ -536,8 +536,9 @@ NET_API int32_t net_measure_gather(int32_t source, int64_t words, double *gather
                                    char *err, size_t err_len);
 
 /* Waits for the device; reports an asynchronous CUDA error if one occurred.
- * Also gives back to the driver the device memory the library keeps for its
- * next allocations (at most 512 MiB per device between calls). */
+ * Also gives back to the driver the memory the library keeps between calls for
+ * the next ones: device memory (at most 512 MiB per device) and page-locked
+ * host memory (at most 4 MiB). */
 NET_API int32_t net_device_sync(char *err, size_t err_len);
 
 #ifdef __cplusplus

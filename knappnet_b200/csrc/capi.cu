@@ -1565,6 +1565,7 @@ int32_t net_device_sync(char* err, size_t err_len) {
   return guard(err, err_len, [&] {
     KNB_CUDA(cudaDeviceSynchronize());
     knb::device_pool_trim();
+    knb::host_staging_trim();
   });
 }
 

@@ -272,18 +272,21 @@ struct PlainMemory {
   PlainMemory(const PlainMemory&) = delete;
 };
 
-// Page-locked host memory of the calling thread for small copies (a copy from
-// or to pageable memory costs about 10 us and waits; freed with the thread).
-// The lower half is for copies to the device, the upper for copies back, and
-// whoever uses it waits for its copies before returning.
+// Page-locked host memory for a call's small copies (a copy from or to pageable
+// memory costs about 10 us and waits). The lower half is for copies to the
+// device, the upper for copies back, and whoever holds it waits for its copies
+// before it lets go. Blocks are shared by all threads: there are as many as calls
+// have held at once, of which STAGING_KEEP stay for the next ones until
+// host_staging_trim.
 constexpr size_t STAGING_HALF = size_t(512) << 10;
+constexpr size_t STAGING_KEEP = 4;
 struct HostStaging {
   unsigned char* p = nullptr;  // null where none could be had
   HostStaging();
   ~HostStaging();
   HostStaging(const HostStaging&) = delete;
 };
-HostStaging& host_staging();
+void host_staging_trim();
 
 // Device memory owned by RAII.
 template <class T>

@@ -884,7 +884,8 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
   double* const changes = scores + n;
   int32_t* const iters = reinterpret_cast<int32_t*>(changes + count);
   int32_t* const status = iters + count;
-  unsigned char* const stage = host_staging().p;
+  const HostStaging staging;
+  unsigned char* const stage = staging.p;
   if (pers) {  // the vectors, then their sums
     if (!P.dpers.get()) P.dpers.alloc((size_t)n + count);
     if (stage && ((size_t)n + count) * 8 <= STAGING_HALF) {

@@ -101,17 +101,43 @@ void device_free(const DeviceBlock& b) noexcept {
   }
 }
 
+static std::mutex g_staging_mu;
+static unsigned char* g_staging[STAGING_KEEP];  // idle blocks
+static size_t g_staging_n = 0;
+
 HostStaging::HostStaging() {
+  {
+    std::lock_guard<std::mutex> lock(g_staging_mu);
+    if (g_staging_n) p = g_staging[--g_staging_n];
+  }
   void* q = nullptr;
-  if (cudaMallocHost(&q, 2 * STAGING_HALF) == cudaSuccess) p = static_cast<unsigned char*>(q);
-  else cudaGetLastError();
+  if (p) return;
+  if (cudaHostAlloc(&q, 2 * STAGING_HALF, cudaHostAllocPortable) == cudaSuccess)
+    p = static_cast<unsigned char*>(q);
+  else
+    cudaGetLastError();
 }
 HostStaging::~HostStaging() {
-  if (p) cudaFreeHost(p);
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lock(g_staging_mu);
+    if (g_staging_n < STAGING_KEEP) {
+      g_staging[g_staging_n++] = p;
+      return;
+    }
+  }
+  cudaFreeHost(p);
 }
-HostStaging& host_staging() {
-  thread_local HostStaging s;
-  return s;
+void host_staging_trim() {
+  for (;;) {
+    unsigned char* q = nullptr;
+    {
+      std::lock_guard<std::mutex> lock(g_staging_mu);
+      if (!g_staging_n) return;
+      q = g_staging[--g_staging_n];
+    }
+    cudaFreeHost(q);
+  }
 }
 
 void device_pool_trim() {
