@@ -853,7 +853,8 @@ int32_t net_components(const GraphHandle* h, int32_t kind, int32_t* membership, 
     const knb::DevComps c = kind == 1 && g.directed
                                 ? knb::strong_components_device(g, nullptr, false, nullptr, s)
                                 : knb::weak_components_device(g, s);
-    if (c.count > (uint32_t)INT32_MAX)
+    // labels 0 to count - 1 have to fit
+    if (c.count - 1 > (uint32_t)INT32_MAX)
       throw Error("component count " + std::to_string(c.count - 1) + " is too large");
     KNB_CUDA(cudaMemcpyAsync(membership, c.label.get(), (size_t)g.n * 4, cudaMemcpyDeviceToHost, s));
     KNB_CUDA(cudaStreamSynchronize(s));
