@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import knappnet_b200 as K
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +63,25 @@ def test_a_single_graphs_shape_follows_its_own_teleport():
     for p, cluster in ((pers, 16), (None, 8), (pers, 16), (None, 8)):
         _, _, info = g.pagerank_graphs([0, n], personalization=p)
         assert info.hot_columns == cluster
+
+
+# On both sides of what a cluster of 8 holds (about 9,600 nodes of 10 arcs without
+# values), and a row whose CTA cannot hold its arcs (its graph's vectors stay in
+# shared memory, the arcs do not): scores of the oracle, and the cluster that says
+# which side a graph is on.
+@pytest.mark.parametrize("n,m,hub,weighted,cluster",
+                         [(9000, 90_000, 0, False, 8), (10_000, 100_000, 0, False, 16),
+                          (3000, 90_000, 45_000, True, 8)])
+def test_scores_on_both_sides_of_the_shared_memory(n, m, hub, weighted, cluster):
+    rng = np.random.default_rng(n)
+    src, tgt = rng.integers(0, n, m), rng.integers(0, n, m)
+    tgt[:hub] = 17
+    w = rng.lognormal(size=m) if weighted else None
+    g, o = K.Graph(n, src, tgt, w, True), O.Graph(n, src, tgt, w, True)
+    for pers in (None, rng.random(n)):
+        x, its, info = g.pagerank_graphs([0, n], weighted=weighted, personalization=pers,
+                                         tol=1e-12)
+        if pers is None:
+            assert info.hot_columns == cluster
+        y = o.pagerank(weighted=weighted, personalization=pers, tol=1e-12)
+        assert np.abs(x - y).sum() <= 1e-12 + abs(1.0 - y.sum())
