@@ -259,7 +259,9 @@ NET_API int32_t net_pagerank_batch_device(const GraphHandle *h, double damping,
  * graphs side by side (graph k on nodes node_offsets[k] ..
  * node_offsets[k + 1] - 1, no edge between graphs, e.g. ego networks built
  * into one handle), and out receives, for every graph, what net_pagerank on
- * that graph alone returns. One persistent CUDA launch solves all graphs.
+ * that graph alone returns, up to rounding; a change within rounding of the
+ * tolerance may end it a sweep apart. One persistent CUDA launch solves all
+ * graphs.
  * personalization is NULL (uniform per graph) or n values (rescaled per
  * graph); iterations (NULL or count values) receives each graph's
  * iteration count. */

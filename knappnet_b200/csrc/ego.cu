@@ -25,9 +25,10 @@
 // fit keep those in global memory, graphs whose vectors do not fit keep
 // everything there.
 // With the graph in global memory and two reductions an iteration of a graph
-// of 500 nodes took 8.0 us, now 1.8 us; 10,000 nodes and 100,000 arcs on a
-// cluster of 8 13.6 us, now 7.5 us; R-MAT graphs of 30,000 nodes, whose hub rows
-// each waited for one thread, 235 us and 25 us.
+// of 500 nodes took 8.0 us, now 1.8 us; 10,000 nodes and 100,000 arcs, on a
+// cluster of 8 then, of 16 and still in global memory now, 13.6 us and 6.5 us;
+// R-MAT graphs of 30,000 nodes, whose hub rows each waited for one thread, 235 us
+// and 25 us.
 #include <algorithm>
 #include <atomic>
 #include <cfloat>

@@ -452,36 +452,36 @@ __global__ void fill_value(double* x, uint32_t n, double v) {
 // carries into the next. The results are lane 0's.
 __device__ __forceinline__ void run_sums(const OpView<double>& op, uint32_t b, uint32_t e,
                                          int lane, double* sum, double* square) {
-      const unsigned F = 0xffffffffu;
+  const unsigned F = 0xffffffffu;
   double s = 0.0, q = 0.0, cacc = 0.0;
-      uint32_t ccol = 0xFFFFFFFFu;  // column of the run open at the previous chunk's end
-      for (uint32_t base = b; base < e; base += 32) {
-        const uint32_t k = base + lane;
-        const bool valid = k < e;
-        const uint32_t j = valid ? op.cols[k] : 0xFFFFFFFEu;
-        const double w = valid ? (op.vals ? op.vals[k] : 1.0) : 0.0;
-        s += w;
-        uint32_t pj = __shfl_up_sync(F, j, 1);
-        if (lane == 0) pj = ccol;
-        const bool start = j != pj;
-        const uint32_t starts = __ballot_sync(F, start);
-        // the run carried from the previous chunk ends where this chunk starts anew
-        if (lane == 0 && (starts & 1u) && ccol != 0xFFFFFFFFu) q += cacc * cacc;
-        const uint32_t upto = starts & (0xffffffffu >> (31 - lane));
-        const int seg0 = upto ? 31 - __clz(upto) : -1;  // -1: the run continues from ccol
-        double r = w;
-  #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double rr = __shfl_up_sync(F, r, o);
-          if (lane - o >= (seg0 < 0 ? 0 : seg0)) r += rr;
-        }
-        if (seg0 < 0) r += cacc;
-        const bool next_start = __shfl_down_sync(F, start, 1);
-        if (valid && lane < 31 && k + 1 < e && next_start) q += r * r;
-        const int last = (int)min(31u, e - 1 - base);
-        cacc = __shfl_sync(F, r, last);
-        ccol = __shfl_sync(F, j, last);
-      }
+  uint32_t ccol = 0xFFFFFFFFu;  // column of the run open at the previous chunk's end
+  for (uint32_t base = b; base < e; base += 32) {
+    const uint32_t k = base + lane;
+    const bool valid = k < e;
+    const uint32_t j = valid ? op.cols[k] : 0xFFFFFFFEu;
+    const double w = valid ? (op.vals ? op.vals[k] : 1.0) : 0.0;
+    s += w;
+    uint32_t pj = __shfl_up_sync(F, j, 1);
+    if (lane == 0) pj = ccol;
+    const bool start = j != pj;
+    const uint32_t starts = __ballot_sync(F, start);
+    // the run carried from the previous chunk ends where this chunk starts anew
+    if (lane == 0 && (starts & 1u) && ccol != 0xFFFFFFFFu) q += cacc * cacc;
+    const uint32_t upto = starts & (0xffffffffu >> (31 - lane));
+    const int seg0 = upto ? 31 - __clz(upto) : -1;  // -1: the run continues from ccol
+    double r = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double rr = __shfl_up_sync(F, r, o);
+      if (lane - o >= (seg0 < 0 ? 0 : seg0)) r += rr;
+    }
+    if (seg0 < 0) r += cacc;
+    const bool next_start = __shfl_down_sync(F, start, 1);
+    if (valid && lane < 31 && k + 1 < e && next_start) q += r * r;
+    const int last = (int)min(31u, e - 1 - base);
+    cacc = __shfl_sync(F, r, last);
+    ccol = __shfl_sync(F, j, last);
+  }
   q = warp_sum(q);
   s = warp_sum(s);
   if (e > b) q += cacc * cacc;

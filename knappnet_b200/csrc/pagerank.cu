@@ -486,7 +486,6 @@ struct SweepBuffers {
   void* head;
   double* part1;
   double* part2;
-  double* part3;
   IterState* st;
   const double* y_ref = nullptr;  // refinement sweeps: the anchor iterate (FP64)
   double* s_ref = nullptr;        //   and its row sums
@@ -1117,7 +1116,6 @@ static double time_candidate(Operator& op, const SweepPick& c, int cls, bool use
   B.v32 = sl ? OpView<float>{} : op.rview32();
   B.part1 = ws.part1.get();
   B.part2 = ws.part2.get();
-  B.part3 = ws.part3.get();
   B.st = st;
   B.so = SO;
   if (cls == 0) {
@@ -1369,7 +1367,7 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
     ++launches;
     SweepBuffers B{v64, v32, {ws.y32[0].get(), ws.y32[1].get()},
                    {ws.z32[0].get(), ws.z32[1].get()}, inv32, pdev, ws.carry32.get(),
-                   ws.head32.get(), ws.part1.get(), ws.part2.get(), ws.part3.get(), st};
+                   ws.head32.get(), ws.part1.get(), ws.part2.get(), st};
     B.so = SO;
     SweepFn fn = pick_kernel<float, float, false>(var32, ipt32, pv, ju);
     r32 = run_phase(fn, op, *P32, B, prm.damping, s, ws, hstate, &tms32, &tn32);
@@ -1401,7 +1399,7 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
       // the FP32 iterate buffers, free once pr_switch has read them.
       SweepBuffers R{v64, v32, {ws.y32[0].get(), ws.y32[1].get()},
                      {ws.z32[0].get(), ws.z32[1].get()}, inv32, pdev, ws.carry32.get(),
-                     ws.head32.get(), ws.part1.get(), ws.part2.get(), ws.part3.get(), st + 1,
+                     ws.head32.get(), ws.part1.get(), ws.part2.get(), st + 1,
                      ws.y64[0].get(), ws.z64[1].get(), SO};
       AnchorFn af = use32 ? pick_anchor<float>(var64, ipt64, pv, ju)
                           : pick_anchor<double>(var64, ipt64, pv, ju);
@@ -1425,7 +1423,7 @@ void pagerank_op(Operator& op, const PagerankParams& prm_in, double* out, bool o
     } else {
       SweepBuffers B{v64, v32, {ws.y64[0].get(), ws.y64[1].get()},
                      {ws.z64[0].get(), ws.z64[1].get()}, inv64, pdev, ws.carry64.get(),
-                     ws.head64.get(), ws.part1.get(), ws.part2.get(), ws.part3.get(), st + 1};
+                     ws.head64.get(), ws.part1.get(), ws.part2.get(), st + 1};
       B.so = SO;
       SweepFn fn = use32 ? pick_kernel<double, float, true>(var64, ipt64, pv, ju)
                          : pick_kernel<double, double, true>(var64, ipt64, pv, ju);

@@ -634,10 +634,10 @@ constexpr size_t tile_smem_bytes() {
 // tile order); long rows (hubs) take one warp: lane l adds tiles first+l,
 // first+l+32, ... in order, then a fixed butterfly joins the lanes. Each CTA
 // also reduces a fixed slice of the sweep's `npart` partials (one per tile
-// from tile_spmv, one per warp from the warp-tile kernels); the last CTA to
-// finish adds the per-CTA results in CTA order and hands them to
-// Epi::finish. Every
-// sum has a fixed association, so results do not change from run to run.
+// from tile_spmv, one per CTA from warp_spmv and slice_spmv, one per warp from
+// the hot-node and bulk-staged kernels); the last CTA to finish adds the per-CTA
+// results in a fixed order and hands them to Epi::finish. Every sum has a fixed
+// association, so results do not change from run to run.
 // Partials written by other CTAs are read with ld.global.cg (L2, not L1).
 //
 // Bound by latency: the bytes are few, but each row is a chain of loads (the
@@ -645,9 +645,9 @@ constexpr size_t tile_smem_bytes() {
 // sums is loaded first (the next row, the node's inputs, the head, the CTA's
 // partials), up to eight of a lane's partials are in flight at once and added
 // in the same order, and short and long rows go to different ends of the grid
-// (3.6M arcs, FP64: 1.78 -> 1.68 ms a solve; R-MAT with 2^24 arcs: HITS 7.5 ->
-// 7.0, a gradient 10.1 -> 9.7, Katz 8.0 -> 7.8 ms; level with 2^28 arcs, where
-// the next kernel's wait hides it).
+// (3.6M arcs, FP64: 1.78 -> 1.68 ms a solve; R-MAT with 2^24 arcs: a gradient
+// 10.1 -> 9.7, Katz 8.0 -> 7.8 ms; level with 2^28 arcs, where the next kernel's
+// wait hides it).
 constexpr int SPLIT_CTAS = 592;
 
 template <class E, class = void>
