@@ -353,8 +353,9 @@ __device__ __forceinline__ bool ego_iterate(const EgoGraph& g, const EgoParams& 
 // K sums over the rows [g.g_lo, g_hi) of a graph in the order `o` states:
 // row(i, a) adds row i's terms to a[0, K). The CTAs of a cluster take the
 // shares by turns, each in the launch's own threads, and every CTA adds the
-// shares' sums in order (slots: 2 turns x EGO_SHARES x 2). The barrier in it
-// publishes everything written before it.
+// shares' sums in order (slots: 2 turns x EGO_SHARES x 2; sh: 2 turns x 2 x 32).
+// The barrier in it publishes everything written before it. Warps of `o` that
+// have no rows add nothing: for 60 nodes two warps' sums are joined, not 32.
 template <int C, int K, class F>
 __device__ __forceinline__ void ego_ordered_sums(const EgoGraph& g, uint32_t g_hi,
                                                  const EgoOrder& o, double (&out)[K], double* sh,
@@ -363,11 +364,13 @@ __device__ __forceinline__ void ego_ordered_sums(const EgoGraph& g, uint32_t g_h
   const uint32_t per = (g.nk + shares - 1) / shares;
   const uint32_t lane = threadIdx.x & 31;
   double* mine = slots + (turn & 1) * EGO_SHARES * 2;
+  sh += (turn & 1) * 64;
   unsigned rank = 0;
   if constexpr (C > 1) rank = cg::this_cluster().block_rank();
   for (uint32_t r = rank; r < shares; r += C) {
     const uint32_t lo = min(g_hi, g.g_lo + r * per), hi = min(g_hi, lo + per);
-    for (uint32_t t = threadIdx.x; t < o.threads; t += blockDim.x) {
+    const uint32_t used = min(o.threads, (hi - lo + 31u) & ~31u);
+    for (uint32_t t = threadIdx.x; t < used; t += blockDim.x) {
       double a[K];
 #pragma unroll
       for (int j = 0; j < K; ++j) a[j] = 0.0;
@@ -379,9 +382,20 @@ __device__ __forceinline__ void ego_ordered_sums(const EgoGraph& g, uint32_t g_h
       }
     }
     __syncthreads();
+    if (C == 1 && shares == 1) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        double t = 0.0;
+#pragma unroll 4
+        for (uint32_t k = 0; k < used / 32; ++k) t += sh[32 * j + k];
+        out[j] = t;
+      }
+      return;
+    }
     if (threadIdx.x < K) {
       double t = 0.0;
-      for (uint32_t k = 0; k < o.threads / 32; ++k) t += sh[32 * threadIdx.x + k];
+#pragma unroll 4
+      for (uint32_t k = 0; k < used / 32; ++k) t += sh[32 * threadIdx.x + k];
       if constexpr (C == 1) {
         mine[r * 2 + threadIdx.x] = t;
       } else {
@@ -403,30 +417,46 @@ __device__ __forceinline__ void ego_ordered_sums(const EgoGraph& g, uint32_t g_h
 
 // The reference's iteration step by step (z = x / out with the dangling mass,
 // A z, the update, the division by the total, the L1 change), with two
-// reductions an iteration and every row's sum in CSR order. It runs, in global
-// memory, for a graph whose other iteration comes so near to the tolerance that
-// rounding would decide the sweep it stops on: about one in a hundred at 1e-12
-// (2,000 graphs: 2.01 ms a call without it, 2.12 with). In batches of 300 and
-// 2,000 graphs at 60 tolerances each, 25 of 1.7 million solves stopped a sweep
-// earlier or later than here without it.
+// reductions an iteration and every row's sum in CSR order. It runs, with its
+// three vectors in shared memory where one CTA's holds them, for a graph whose
+// other iteration comes so near to the tolerance that rounding would decide the
+// sweep it stops on: about one in a hundred at 1e-12. 2,000 graphs take 2.04 ms a
+// call without it and 2.06 with; a small batch whose longest graph is such a one
+// up to twice as long (60 graphs of up to 1,000 nodes 0.27 and 0.53 ms, one batch
+// of sixteen). In batches of 300 and 2,000 graphs at 60 tolerances each, 25 of 1.7
+// million solves stopped a sweep earlier or later than here without it.
 struct EgoEnd {
   int32_t it, done;
   double change;
 };
 template <int C>
 __device__ __noinline__ EgoEnd ego_normalising(const EgoGraph g, const uint32_t g_hi,
-                                               const EgoParams prm, const EgoOrder o, double* sh,
+                                               const EgoParams prm, const EgoOrder o,
+                                               const uint32_t sm_bytes, double* sh,
                                                double* slots) {
+  extern __shared__ __align__(16) unsigned char ego_smem[];
   const double inv_n = 1.0 / (double)g.nk;
-  const OpView<double>& op = g.op;
+  // (copies: what a store might change would be loaded again after each)
+  const uint32_t* __restrict__ off = g.op.off;
+  const uint32_t* __restrict__ cols = g.op.cols;
+  const double* __restrict__ vals = g.op.vals;
+  const double* __restrict__ outstr = g.outstr;
+  const double* __restrict__ pers = g.pers;
+  const double d = prm.d, ps = g.ps;
+  const bool jump_uniform = prm.jump_uniform;
   double* x = g.y;
   double* y = g.y + g.n;
   double* z = g.z;
+  if (C == 1 && (size_t)24 * g.nk <= sm_bytes) {  // row i at its place in the graph
+    x = reinterpret_cast<double*>(ego_smem) - g.g_lo;
+    y = x + g.nk;
+    z = y + g.nk;
+  }
   int turn = 0;
   double st[1];
-  ego_ordered_sums<C, 1>(g, g_hi, o, st, sh, slots, turn++, [&](uint32_t i, double* a) {
+  ego_ordered_sums<C, 1>(g, g_hi, o, st, sh, slots, turn++, [=](uint32_t i, double* a) {
     x[i] = inv_n;
-    const double out = g.outstr[i];
+    const double out = outstr[i];
     if (out > 0.0) {
       z[i] = inv_n / out;
     } else {
@@ -439,40 +469,40 @@ __device__ __noinline__ EgoEnd ego_normalising(const EgoGraph g, const uint32_t 
   double change = 0.0;
   while (it < prm.max_iter) {
     double tot[1];
-    ego_ordered_sums<C, 1>(g, g_hi, o, tot, sh, slots, turn++, [&](uint32_t i, double* a) {
+    ego_ordered_sums<C, 1>(g, g_hi, o, tot, sh, slots, turn++, [=](uint32_t i, double* a) {
       // arcs in CSR order; four gathers in flight before their products
       // are added in that order
       double s = 0;
-      uint32_t k = op.off[i];
-      const uint32_t ke = op.off[i + 1];
+      uint32_t k = off[i];
+      const uint32_t ke = off[i + 1];
       for (; k + 4 <= ke; k += 4) {
         double zk[4], wk[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          zk[u] = z[op.cols[k + u]];
-          wk[u] = op.vals ? op.vals[k + u] : 1.0;
+          zk[u] = z[cols[k + u]];
+          wk[u] = vals ? vals[k + u] : 1.0;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) s += wk[u] * zk[u];
       }
       for (; k < ke; ++k) {
-        const double w = op.vals ? op.vals[k] : 1.0;
-        s += w * z[op.cols[k]];
+        const double w = vals ? vals[k] : 1.0;
+        s += w * z[cols[k]];
       }
-      const double p = g.pers ? g.pers[i] / g.ps : inv_n;
-      const double jmp = prm.jump_uniform ? inv_n : p;
-      const double v = prm.d * (s + stuck * jmp) + (1.0 - prm.d) * p;
+      const double p = pers ? pers[i] / ps : inv_n;
+      const double jmp = jump_uniform ? inv_n : p;
+      const double v = d * (s + stuck * jmp) + (1.0 - d) * p;
       y[i] = v;
       a[0] += v;
     });
     const double total = tot[0];
     // the division, the change, and the next z and dangling mass
     double cs[2];
-    ego_ordered_sums<C, 2>(g, g_hi, o, cs, sh, slots, turn++, [&](uint32_t i, double* a) {
+    ego_ordered_sums<C, 2>(g, g_hi, o, cs, sh, slots, turn++, [=](uint32_t i, double* a) {
       const double v = y[i] / total;
       y[i] = v;
       a[0] += fabs(v - x[i]);
-      const double out = g.outstr[i];
+      const double out = outstr[i];
       if (out > 0.0) {
         z[i] = v / out;
       } else {
@@ -492,8 +522,9 @@ __device__ __noinline__ EgoEnd ego_normalising(const EgoGraph g, const uint32_t 
     }
   }
   double none[1];
+  double* const out = g.out;
   ego_ordered_sums<C, 1>(g, g_hi, o, none, sh, slots, turn,
-                         [&](uint32_t i, double*) { g.out[i] = x[i]; });
+                         [=](uint32_t i, double*) { out[i] = x[i]; });
   return {it, done, change};
 }
 
@@ -555,7 +586,7 @@ __device__ __forceinline__ void ego_solve(EgoGraph g, uint32_t g_hi, const EgoPa
     // every CTA has read the last sums before their places are used anew
     if constexpr (C > 1) cg::this_cluster().sync();
     else __syncthreads();
-    const EgoEnd e = ego_normalising<C>(g, g_hi, prm, order, sh, slots);
+    const EgoEnd e = ego_normalising<C>(g, g_hi, prm, order, sm_bytes, sh, slots);
     *it = e.it;
     *done = e.done;
     *ch = e.change;
@@ -643,13 +674,13 @@ ego_pagerank(EgoGraph g, const uint32_t* __restrict__ node_off,
 // The normalising iteration of a single graph (nodes [0, g.nk)) on one cluster.
 template <int C>
 __global__ void __launch_bounds__(1024, 1)
-ego_one(EgoGraph g, EgoParams prm, EgoOrder sums, int32_t* __restrict__ iters,
+ego_one(EgoGraph g, EgoParams prm, EgoOrder sums, uint32_t sm_bytes, int32_t* __restrict__ iters,
         int32_t* __restrict__ status, double* __restrict__ changes) {
-  __shared__ double sh[2 * 32];
+  __shared__ double sh[2 * 2 * 32];
   __shared__ double slots[2 * EGO_SHARES * 2];
   // (the first sums write into every CTA's slots: all have to be there)
   if constexpr (C > 1) cg::this_cluster().sync();
-  const EgoEnd e = ego_normalising<C>(g, g.nk, prm, sums, sh, slots);
+  const EgoEnd e = ego_normalising<C>(g, g.nk, prm, sums, sm_bytes, sh, slots);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *iters = e.it;
     *status = ego_status(e.done);
@@ -1000,7 +1031,11 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
     g1.nk = n;
     g1.ps = pers ? ps[0] : 1.0;
     if (n < sums.split) {
-      ego_one<1><<<1, sums.threads, 0, s>>>(g1, prm, sums, iters, status, changes);
+      const uint32_t most = ego_most_smem();
+      set_func_attr((const void*)ego_one<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    (int)most);
+      const uint32_t smem = (size_t)24 * n <= most ? 24 * n : 0;
+      ego_one<1><<<1, sums.threads, smem, s>>>(g1, prm, sums, smem, iters, status, changes);
     } else {
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1013,7 +1048,7 @@ void pagerank_graphs(GraphHandleImpl& g, const EgoInput& in, double* out, EgoRes
       cfg.stream = s;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      KNB_CUDA(cudaLaunchKernelEx(&cfg, ego_one<EGO_SHARES>, g1, prm, sums, iters, status,
+      KNB_CUDA(cudaLaunchKernelEx(&cfg, ego_one<EGO_SHARES>, g1, prm, sums, 0u, iters, status,
                                   changes));
     }
     KNB_LAUNCH("ego_one");
